@@ -158,6 +158,11 @@ int nse2d_step_timed(nse2d_ctx* ctx, int nsteps, double* kernel_ms, cudaStream_t
 int nse2d_step_profiled(nse2d_ctx* ctx, double* step_ms, double* fft_ms, double* tridiag_ms, cudaStream_t s) {
     CHECK_CTX(ctx);
     Context* c = ctx->c;
+    struct Plain {
+        Context* c;
+        explicit Plain(Context* x) : c(x) { c->plain_step = true; }
+        ~Plain() { c->plain_step = false; }
+    } plain(c);                                 // the row-band launches hold a transform and a stage each
     const int nk = launches_per_step(c);
     std::vector<cudaEvent_t> ev((size_t)nk + 1);
     for (auto& e : ev) NSE_CUDA_TRY(cudaEventCreate(&e));

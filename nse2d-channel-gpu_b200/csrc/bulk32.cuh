@@ -245,9 +245,8 @@ static __global__ void __launch_bounds__(256) k_stage32(Stage32Params p) {
         const size_t id = (size_t)j * Nx + i;
         if (p.rhs_out) p.rhs_out[id] = rhs;
         float wnew;
-        if (p.stage == 1) wnew = fmaf(dt, rhs, wc);
-        else if (p.stage == 2) wnew = 0.75f * p.w_n[id] + 0.25f * fmaf(dt, rhs, wc);
-        else wnew = (1.0f / 3.0f) * p.w_n[id] + (2.0f / 3.0f) * fmaf(dt, rhs, wc);
+        wnew = fmaf(dt, rhs, wc);
+        if (p.stage > 1) wnew = rk_combine(p.stage, p.w_n[id], wnew);
         p.w_out[id] = wnew;
     }
 }
@@ -342,7 +341,7 @@ __device__ __forceinline__ void stage32_tile4(const Stage32Params& p, float dt, 
             const float nn[4] = {n4.x, n4.y, n4.z, n4.w};
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                wn[k] = (p.stage == 2) ? 0.75f * nn[k] + 0.25f * wn[k] : (1.0f / 3.0f) * nn[k] + (2.0f / 3.0f) * wn[k];
+                wn[k] = rk_combine(p.stage, nn[k], wn[k]);
         }
         *reinterpret_cast<float4*>(p.w_out + id) = make_float4(wn[0], wn[1], wn[2], wn[3]);
     }
@@ -412,6 +411,12 @@ static __global__ void __launch_bounds__(256, 2) k_stage32_tma(const __grid_cons
                       srow[b]);
         fence_proxy_async_smem();                        // reads of buffer b before its next TMA write
     }
+}
+
+// w'_wall from psi' at the first two interior rows; the multiply-adds are written out, so that every
+// kernel gives the same bits.
+__device__ __forceinline__ float thom32_value(float base, float A, float B, float p1, float p2) {
+    return base - fmaf(A, p1, B * p2);
 }
 
 // ---- FP32 row transforms, FP32 spectral buffer ----
@@ -605,7 +610,7 @@ static __global__ void __launch_bounds__(IP_NT, 5) k_ifft_thom32(Fft32Params p) 
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
                     const int i = i0 + c * IP_NT;
-                    if (i < Nx) wr[i] = p.free_slip ? base : base - (A * a1[c] + B * a2[c]);
+                    if (i < Nx) wr[i] = p.free_slip ? base : thom32_value(base, A, B, a1[c], a2[c]);
                 }
             }
         }

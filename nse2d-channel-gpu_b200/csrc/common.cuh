@@ -115,8 +115,13 @@ struct Context {
     double *w = nullptr, *w1 = nullptr, *w2 = nullptr, *psi = nullptr;
     // scratch used by diagnostics: rhs and J at one state, and the stage-3 rhs of the last step
     double *rhs = nullptr, *J = nullptr;
-    // spectral buffer [Ny][Hp] complex, FP64 (in place: omega-hat in, psi-hat out)
+    // spectral buffer [Ny][Hp] complex, FP64: omega-hat, and psi-hat in place where there is no hat2
     cpx<double>* hat = nullptr;
+    // psi-hat, where bands are used (they read halo rows of psi-hat while other CTAs write omega-hat);
+    // otherwise psi-hat takes the place of omega-hat
+    cpx<double>* hat2 = nullptr;
+    bool band = false;             // row transforms of band.cuh: rows of 64 to 2048 points
+    bool plain_step = false;       // a step of separate transforms and stages (nse2d_step_profiled times them apart)
     double* cp = nullptr;          // elimination table [Ni][Hp]
     cpx<double>* tw = nullptr;     // per-pass twiddle pairs of the Nx/2-point transform
     cpx<double>* wN = nullptr;     // M+1 twiddles e^{-2 pi i k/Nx}

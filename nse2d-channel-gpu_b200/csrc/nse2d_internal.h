@@ -36,6 +36,13 @@ int launch_thomas(Context* c, cudaStream_t s);
 int launch_thomas_maps(Context* c, cudaStream_t s, bool homog = false);
 int launch_thomas_apply(Context* c, cudaStream_t s, bool homog = false);
 int launch_thomas_cluster(Context* c, cudaStream_t s, bool homog = false);
+// row-band kernels (band64.cu)
+bool band_rows_ok(int M);
+bool band_stage_ok(int M);
+int band_stage(Context* c, int stage, bool inv, double* w_in, const double* w_n, double* w_out, double* rhs_out,
+               const double* closure, cudaStream_t s);
+int band_rows_fwd(Context* c, const double* src, int row0, int nrows, cudaStream_t s);
+int band_rows_inv(Context* c, double* psi, double* w, bool thom, bool advance, cudaStream_t s);
 // learned closure (closure.cu)
 struct Cnn;
 int cnn_forward(Cnn* n, const double* w, const double* psi, const double* u, const double* v, double* tau, cudaStream_t s);

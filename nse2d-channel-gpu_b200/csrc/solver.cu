@@ -114,7 +114,7 @@ static ThomasClusterKernel thomas_cluster_kernel(int L, bool f32 = false) {
 // homog: the FP32-bulk step's solve, for psi' (zero on the walls) in the FP32 spectral buffer
 static ThomasParams thomas_params(const Context* c, bool homog = false) {
     ThomasParams p{};
-    p.hat = c->hat; p.hat32 = c->hat32; p.cp = c->cp; p.asub = c->rt.asub; p.inv_csup = c->rt.inv_csup; p.csup = c->rt.csup;
+    p.hat = c->hat; p.hat32 = c->hat32; p.out = c->hat2 ? c->hat2 : c->hat; p.out32 = c->hat32; p.cp = c->cp; p.asub = c->rt.asub; p.inv_csup = c->rt.inv_csup; p.csup = c->rt.csup;
     p.tconst = c->tconst; p.tmaps = c->tmaps; p.tblk = c->tblk; p.tbcarry = c->tbcarry; p.tcount = c->tcount;
     p.Nx = c->Nx; p.Ny = c->Ny; p.Hp = c->Hp; p.H = c->H; p.Ni = c->Ni;
     p.nseg = c->thomas_nseg; p.nsb = c->thomas_nsb;
@@ -323,6 +323,8 @@ int context_create(const Config& cfg, Context** out) {
     if (dalloc(&c->hat, (size_t)Ny * c->Hp) || dalloc(&c->cp, (size_t)c->Ni * c->Hp) ||
         dalloc(&c->wN, (size_t)c->M + 1))
         return fail();
+    c->band = band_rows_ok(c->M);
+    if (c->band && cfg.precision == 64 && band_stage_ok(c->M) && dalloc(&c->hat2, (size_t)Ny * c->Hp)) return fail();
     c->thomas_nseg = (c->Ni + TS_ROWS - 1) / TS_ROWS;
     c->thomas_nsb = (c->thomas_nseg + TS_NW - 1) / TS_NW;
     if (dalloc(&c->tconst, (size_t)c->thomas_nseg * 3 * c->Hp) || dalloc(&c->tmaps, (size_t)c->thomas_nseg * 4 * c->Hp) ||
@@ -500,6 +502,7 @@ void context_destroy(Context* c) {
         if (p) cudaFree(p);
     if (c->closure_tau) cudaFree(c->closure_tau);
     if (c->hat) cudaFree(c->hat);
+    if (c->hat2) cudaFree(c->hat2);
     if (c->tconst) cudaFree(c->tconst);
     if (c->tmaps) cudaFree(c->tmaps);
     if (c->tblk) cudaFree(c->tblk);
@@ -539,20 +542,26 @@ static StageParams stage_params(Context* c) {
     return p;
 }
 
+// The learned closure's tau of the state before stage `stage` (the model runs just before the stage), or
+// nullptr without a model.
+static int closure_tau(Context* c, int stage, const double* w_in, const double** tau, cudaStream_t s) {
+    *tau = nullptr;
+    if (!c->closure_net) return 0;
+    if (stage == 1 || c->closure_every_stage) {
+        double* u = c->closure_tau + c->N;
+        double* v = c->closure_tau + 2 * c->N;
+        if (uv_from_psi(c, c->psi, u, v, s) || cnn_forward(c->closure_net, w_in, c->psi, u, v, c->closure_tau, s))
+            return -1;
+    }
+    *tau = c->closure_tau;
+    return 0;
+}
+
 int launch_stage(Context* c, int stage, const double* w_in, const double* w_n, double* w_out, cudaStream_t s,
                  double* rhs_out) {
     StageParams p = stage_params(c);
     p.w_in = w_in; p.w_n = w_n; p.w_out = w_out; p.rhs_out = rhs_out; p.stage = stage;
-    // the learned closure's tau of this stage's state (the model runs just before the stage)
-    if (c->closure_net) {
-        if (stage == 1 || c->closure_every_stage) {
-            double* u = c->closure_tau + c->N;
-            double* v = c->closure_tau + 2 * c->N;
-            if (uv_from_psi(c, c->psi, u, v, s) || cnn_forward(c->closure_net, w_in, c->psi, u, v, c->closure_tau, s))
-                return -1;
-        }
-        p.closure = c->closure_tau;
-    }
+    if (closure_tau(c, stage, w_in, &p.closure, s)) return -1;
     if (c->stage_tma) {
         if (stage > 1 && w_n != c->w) { set_error("launch_stage: omega^n is not the context's omega"); return -1; }
         StageMaps maps;
@@ -594,6 +603,7 @@ template <typename K> static int fft_wave(K kern, size_t smem, int nrows, int nu
 }
 
 template <int M> static int fft_fwd_t(Context* c, FftParams& p, cudaStream_t s) {
+    if constexpr (M >= 32 && M <= 1024) { set_error("rows of %d points use the row-band kernels", 2 * M); return -1; } else {
     if constexpr (M == 16 * IP_NT) if (c->rowfft_pf) {
         // the real rows prefetched into shared memory by bulk copies (k_fft_fwd_pf)
         const size_t sm = FftPf<M>::smem;
@@ -605,6 +615,7 @@ template <int M> static int fft_fwd_t(Context* c, FftParams& p, cudaStream_t s) 
     int grid = 0;
     if (fft_wave(k_fft_fwd<M>, sm, p.nrows, c->num_sms, &grid)) return -1;
     return launch_step_kernel(c, k_fft_fwd<M>, dim3(grid), dim3(IP_NT), sm, s, nullptr, p);
+    }
 }
 
 // Inverse transforms: one wave of CTAs over contiguous bands of floor or ceil(Ny / wave) rows
@@ -644,6 +655,7 @@ int launch_fft_fwd(Context* c, const double* src, cudaStream_t s) {
         set_error("omega must be 16-byte aligned for the row transform (got %p)", (const void*)src);
         return -1;
     }
+    if (c->band) return band_rows_fwd(c, src, 1, c->Ni, s);
     FftParams p = fft_params(c);
     p.src = src;
     p.row0 = 1;
@@ -657,6 +669,7 @@ int launch_fft_all_rows(Context* c, const double* src, cudaStream_t s) {
         set_error("the field must be 16-byte aligned for the row transform (got %p)", (const void*)src);
         return -1;
     }
+    if (c->band) return band_rows_fwd(c, src, 0, c->Ny, s);
     FftParams p = fft_params(c);
     p.src = src;
     p.row0 = 0;
@@ -666,7 +679,9 @@ int launch_fft_all_rows(Context* c, const double* src, cudaStream_t s) {
 
 int launch_ifft_thom(Context* c, double* psi, double* w, int stage, bool do_thom, bool closure, cudaStream_t s,
                      bool advance) {
+    if (c->band && !closure) return band_rows_inv(c, psi, w, do_thom, advance, s);
     FftParams p = fft_params(c);
+    if (c->hat2) p.hat = c->hat2;
     p.psi = psi; p.w = w; p.stage = stage; p.do_thom = do_thom ? 1 : 0; p.closure = closure ? 1 : 0;
     p.advance = advance ? 1 : 0;
     p.fuse_max = (advance && fused_max(c)) ? 1 : 0;
@@ -786,10 +801,44 @@ int poisson_solve(Context* c, const double* w, double* psi, cudaStream_t s) {
     return 0;
 }
 
+// The steps that the row-band kernels take: without the MMS forcing and the wall-update bookkeeping of
+// closure_diag (verification runs and diagnostics of their own), which the separate kernels have.
+static bool band_step(const Context* c) { return c->band && band_stage_ok(c->M) && !c->cfg.mms && !c->closure_diag && !c->plain_step; }
+
+// A stage of the band step begins with the inverse transform, except stage 1 (psi is the step's) and,
+// with a model that runs before every stage, stages 2 and 3 (the model needs psi of the stage).
+static bool band_split(const Context* c) { return c->closure_net && c->closure_every_stage; }
+
+// The same step by the row-band kernels: per stage one launch of rows and one tridiagonal solve.
+static int band_step_impl(Context* c, cudaStream_t s, bool store_rhs, cudaEvent_t* ev) {
+    int k = 0;
+    auto mark = [&]() -> int {
+        if (ev) NSE_CUDA_TRY(cudaEventRecord(ev[k++], s));
+        return 0;
+    };
+    if (mark()) return -1;
+    if (c->cfg.adapt && (launch_maxuv(c, c->psi, true, s) || mark())) return -1;
+    double* wst[3] = {c->w1, c->w2, c->w};
+    double* win[3] = {c->w, c->w1, c->w2};
+    const bool split = band_split(c);
+    for (int st = 1; st <= 3; ++st) {
+        const double* tau = nullptr;
+        if (closure_tau(c, st, win[st - 1], &tau, s)) return -1;
+        if (band_stage(c, st, st > 1 && !split, win[st - 1], c->w, wst[st - 1], (store_rhs && st == 3) ? c->rhs : nullptr, tau, s) ||
+            mark())
+            return -1;
+        for (int i = 0; i < thomas_launches(c); ++i)
+            if (launch_thomas_part(c, i, s, false) || mark()) return -1;
+        if ((split || st == 3) && (band_rows_inv(c, c->psi, wst[st - 1], true, st == 3, s) || mark())) return -1;
+    }
+    return 0;
+}
+
 // One SSPRK(3,3) step (src/main.cu:439-541) with dt from the control block. With ev != nullptr
 // an event is recorded before the step and after every kernel (for per-kernel timing).
 static int step_impl(Context* c, cudaStream_t s, bool store_rhs, cudaEvent_t* ev) {
     if (c->prec32) return step32_impl(c, s, store_rhs, ev);
+    if (band_step(c)) return band_step_impl(c, s, store_rhs, ev);
     int k = 0;
     auto mark = [&]() -> int {
         if (ev) NSE_CUDA_TRY(cudaEventRecord(ev[k++], s));
@@ -825,6 +874,19 @@ const char* step_kernel_name(const Context* c, int k) {
         if (k == 0) return "k_maxuv_dt";
         --k;
     }
+    if (band_step(c)) {
+        const int nt = thomas_launches(c);
+        for (int st = 1; st <= 3 && k >= 0; ++st) {
+            if (k == 0) return st > 1 && !band_split(c) ? "k_band_inv_stage_fwd" : "k_band_stage_fwd";
+            if (k <= nt) return thomas_kernel_name(c, k - 1);
+            k -= 1 + nt;
+            if (st == 3 || band_split(c)) {
+                if (k == 0) return "k_rows_inv";
+                --k;
+            }
+        }
+        return "";
+    }
     const int per = 3 + thomas_launches(c);
     if (k < 0 || k >= 3 * per) return "";
     const int i = k % per;
@@ -836,6 +898,7 @@ const char* step_kernel_name(const Context* c, int k) {
 
 int launches_per_step(const Context* c) {
     if (c->prec32) return (c->cfg.adapt ? 1 : 0) + 3 * (3 + thomas_launches(c));
+    if (band_step(c)) return (c->cfg.adapt ? 1 : 0) + 3 * (1 + thomas_launches(c)) + (band_split(c) ? 3 : 1);
     return (c->cfg.adapt && !fused_max(c) ? 1 : 0) + 3 * (3 + thomas_launches(c));
 }
 

@@ -107,6 +107,17 @@ __device__ __forceinline__ double point_rhs(const StageParams& p, int j, int i, 
 // (as fmax skips it), and an accumulator that starts at 0 never becomes NaN.
 __device__ __forceinline__ double nn_max(double a, double b) { return b > a ? b : a; }
 
+// The Shu-Osher combines of stages 2 and 3 (src/ops.cu:650,654): omega^n and omega^(s) + dt rhs. The
+// multiply-adds are written out, so that every stage kernel gives the same bits.
+__device__ __forceinline__ double rk_combine(int stage, double wn, double x) {
+    return stage == 2 ? fma(0.25, x, 0.75 * wn) : fma(2.0 / 3.0, x, (1.0 / 3.0) * wn);
+}
+__device__ __forceinline__ float rk_combine(int stage, float wn, float x) {
+    return stage == 2 ? fmaf(0.25f, x, 0.75f * wn) : fmaf(2.0f / 3.0f, x, (1.0f / 3.0f) * wn);
+}
+// Thom wall vorticity (src/ops.cu:121-149) from psi - psi_wall at the first two interior rows.
+__device__ __forceinline__ double thom_value(double A, double B, double e1, double e2) { return -fma(A, e1, B * e2); }
+
 // Programmatic dependent launch: a step kernel launched with the programmatic-serialisation
 // attribute may be launched while the kernel before it in the stream is still finishing (its
 // CTAs trigger the next launch as they exit). Every step kernel begins with pdl_begin: it waits
@@ -259,15 +270,8 @@ __device__ __forceinline__ void stage_tile(const StageParams& p, const StageTime
         const size_t id = (size_t)j * Nx + i;
         if (p.closure && j != 0 && j != Ny - 1) rhs -= __ldg(&p.closure[id]);
         if (p.rhs_out) p.rhs_out[id] = rhs;
-        double wnew;
-        const double dt = st.dt;
-        if (p.stage == 1) {
-            wnew = wc + dt * rhs;                                                          // ops.cu:646
-        } else {
-            const double wn = swn ? swn[ly * ST_TX + lx] : p.w_n[id];
-            if (p.stage == 2) wnew = 0.75 * wn + 0.25 * (wc + dt * rhs);                   // ops.cu:650
-            else wnew = (1.0 / 3.0) * wn + (2.0 / 3.0) * (wc + dt * rhs);                 // ops.cu:654
-        }
+        double wnew = fma(st.dt, rhs, wc);                                                 // ops.cu:646
+        if (p.stage > 1) wnew = rk_combine(p.stage, swn ? swn[ly * ST_TX + lx] : p.w_n[id], wnew);
         p.w_out[id] = wnew;
     }
 }
@@ -432,20 +436,11 @@ __device__ __forceinline__ void stage_tile2(const StageParams& p, const StageTim
             rb -= tau.y;
         }
         if (p.rhs_out) *reinterpret_cast<double2*>(p.rhs_out + id) = make_double2(ra, rb);
-        double na, nb;
-        const double dt = st.dt;
-        if (p.stage == 1) {
-            na = wa + dt * ra;                                                              // ops.cu:646
-            nb = wb + dt * rb;
-        } else {
+        double na = fma(st.dt, ra, wa), nb = fma(st.dt, rb, wb);                            // ops.cu:646
+        if (p.stage > 1) {
             const double2 wn = *reinterpret_cast<const double2*>(swn + ly * ST_TX + 2 * lp);
-            if (p.stage == 2) {
-                na = 0.75 * wn.x + 0.25 * (wa + dt * ra);                                   // ops.cu:650
-                nb = 0.75 * wn.y + 0.25 * (wb + dt * rb);
-            } else {
-                na = (1.0 / 3.0) * wn.x + (2.0 / 3.0) * (wa + dt * ra);                    // ops.cu:654
-                nb = (1.0 / 3.0) * wn.y + (2.0 / 3.0) * (wb + dt * rb);
-            }
+            na = rk_combine(p.stage, wn.x, na);
+            nb = rk_combine(p.stage, wn.y, nb);
         }
         *reinterpret_cast<double2*>(p.w_out + id) = make_double2(na, nb);
     }
@@ -755,7 +750,7 @@ __device__ __forceinline__ void thom_row(const FftParams& p, bool top) {
             const int i = i0 + c * NT;
             if (i < Nx) {
                 double nv = 0.0;
-                if (!p.free_slip) nv = -(A * (a1[c] - pw) + B * (a2[c] - pw));
+                if (!p.free_slip) nv = thom_value(A, B, a1[c] - pw, a2[c] - pw);
                 wr[i] = nv;
                 sb += wq * ov[c] * ov[c];
                 sa += wq * nv * nv;
@@ -860,7 +855,7 @@ static __global__ void __launch_bounds__(IP_NT, 5) k_ifft_thom(FftParams p) {
             const int t = b0 + (int)threadIdx.x;
             if (NB0 % IP_NT != 0 && t >= NB0) break;
             cpx<double> v[R0];
-            // W_{2M}^n for n = t + NB0 r is W_{2M}^t e^{-i pi r/16} (one table load per thread)
+            // W_{2M}^n for n = t + NB0 r is W_{2M}^t e^{-i pi r/R0} (one table load per thread)
             const cpx<double> wt = ldtw(p.wN, t);
 #pragma unroll
             for (int r = 0; r < R0; ++r) {
@@ -868,7 +863,7 @@ static __global__ void __launch_bounds__(IP_NT, 5) k_ifft_thom(FftParams p) {
                 const double2 av = __ldcs(X + n), bv = __ldcs(X + (M - n));
                 const cpx<double> sm = {av.x + bv.x, av.y - bv.y};
                 const cpx<double> df = {av.x - bv.x, av.y + bv.y};
-                const cpx<double> wn = (R0 == 16) ? (r == 0 ? wt : cmul(wt, w32<double>(r))) : ldtw(p.wN, n);
+                const cpx<double> wn = (R0 >= 4) ? (r == 0 ? wt : cmul(wt, w32<double>(r * (16 / R0)))) : ldtw(p.wN, n);
                 v[r] = cadd(sm, mul_pi(cmulc(df, wn)));
             }
             dftR<double, R0, true>(v);
@@ -1226,8 +1221,10 @@ static __global__ void __launch_bounds__(IP_NT, 3) k_ifft_thom_pf(FftParams p) {
 }
 
 struct ThomasParams {
-    cpx<double>* hat;        // [Ny][Hp], in place: omega-hat in, psi-hat out
-    cpx<float>* hat32;       // the same in FP32 (the FP32-bulk step; the arithmetic stays FP64)
+    const cpx<double>* hat;  // [Ny][Hp] omega-hat
+    const cpx<float>* hat32; // the same in FP32 (the FP32-bulk step; the arithmetic stays FP64)
+    cpx<double>* out;        // psi-hat: the omega-hat buffer, or another one (see band.cuh)
+    cpx<float>* out32;
     const double* cp;        // [Ni][Hp]
     const double* asub;      // [Ny]
     const double* inv_csup;  // [Ny]
@@ -1564,7 +1561,7 @@ static __global__ void __launch_bounds__(TS_NW * 32) k_thomas_apply(ThomasParams
         if (w == warp) cw = cs[w];
     thomas_forward(p, r0, n, kx0re, cw, tl);
     using ST = typename SpecT<F32>::T;
-    ST* hatw = F32 ? reinterpret_cast<ST*>(p.hat32) : reinterpret_cast<ST*>(p.hat);
+    ST* hatw = F32 ? reinterpret_cast<ST*>(p.out32) : reinterpret_cast<ST*>(p.out);
     const size_t rowstride = (size_t)p.Hp * 2;
 #pragma unroll 8
     for (int t = n - 1; t >= 0; --t) {
@@ -1899,7 +1896,7 @@ static __global__ void __launch_bounds__(TC_THREADS, (L <= 8 ? 2 : 1)) k_thomas_
         const double2 X = make_double2(fma(E2.P, Xb.x, E2.D.x), fma(E2.P, Xb.y, E2.D.y));
         // 3. carry term; psi-hat out
         using ST2 = typename SpecT<F32>::T2;
-        ST2* hatw = F32 ? reinterpret_cast<ST2*>(p.hat32) : reinterpret_cast<ST2*>(p.hat);
+        ST2* hatw = F32 ? reinterpret_cast<ST2*>(p.out32) : reinterpret_cast<ST2*>(p.out);
         double Qc = 1.0;
 #pragma unroll
         for (int i = L - 1; i >= 0; --i) {
@@ -1944,9 +1941,9 @@ static __global__ void __launch_bounds__(256) k_thom(ThomParams p) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < Nx; i += gridDim.x * blockDim.x) {
         if (p.free_slip) { p.w[i] = 0.0; wt[i] = 0.0; continue; }
         const double d1 = p.psi[(size_t)1 * Nx + i] - p.psi_bot, d2 = p.psi[(size_t)2 * Nx + i] - p.psi_bot;
-        p.w[i] = -(Ab * d1 + Bb * d2);
+        p.w[i] = thom_value(Ab, Bb, d1, d2);
         const double e1 = p.psi[(size_t)(Ny - 2) * Nx + i] - p.psi_top, e2 = p.psi[(size_t)(Ny - 3) * Nx + i] - p.psi_top;
-        wt[i] = -(At * e1 + Bt * e2);
+        wt[i] = thom_value(At, Bt, e1, e2);
     }
 }
 

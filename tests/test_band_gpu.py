@@ -1,0 +1,48 @@
+"""The row-band kernels (csrc/band.cuh) on a B200, where their splits can go wrong: the smallest rows, rows of
+one to several bands, bands of uneven length, the fewest rows of a grid (both walls in one band), and every
+row length with a transform plan of its own.
+
+A step by the row-band kernels evaluates the per-point and transform arithmetic of the step by separate
+kernels (the one that nse2d_step_profiled times): the same fields and the same stored rhs to the bit. The
+Poisson solve is compared with the oracle at the 1e-12 of the other solves."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from test_parity_gpu import laminar_perturbed, relerr
+
+pytestmark = pytest.mark.gpu
+
+GRIDS = [(64, 5), (64, 6), (64, 11), (64, 900), (128, 150), (128, 1333), (256, 151), (256, 300), (512, 9), (512, 597), (1024, 6),
+         (1024, 595), (1024, 745), (2048, 5), (2048, 61)]
+
+
+@pytest.mark.parametrize("Nx,Ny", GRIDS)
+def test_band_step_gives_the_plain_step_and_solve_the_oracle(nse, oracle, cuda, Nx, Ny):
+    torch = cuda
+    cfg = dict(Nx=Nx, Ny=Ny, Lx=2 * np.pi, stretch=1, beta=1.5, Ub=1.0, Reb=2000.0, F0=0.05, nforce=4, lin_drag=1e-3, adapt=1)
+    a, b = nse.Solver(**cfg), nse.Solver(**cfg)
+    w0 = laminar_perturbed(Nx, Ny, a.metric(0), seed=Nx + Ny, amp=2e-2)
+    a.set_omega(w0)
+    b.set_omega(w0)
+    ms = [ctypes.c_double() for _ in range(3)]
+    rhs = np.empty((2, Ny, Nx))
+    for _ in range(3):
+        a.step_store_rhs(1)
+        assert b.lib.nse2d_step_profiled(b.h, *[ctypes.byref(x) for x in ms], None) == 0
+        assert a.time() == b.time()
+        assert all(np.array_equal(x, y) for x, y in zip(a.fields(), b.fields()))
+        for s, out in zip((a, b), rhs):
+            assert s.lib.nse2d_get_field(s.h, 4, out.ctypes.data_as(ctypes.c_void_p), None) == 0
+        assert np.array_equal(rhs[0], rhs[1])
+    assert np.all(np.isfinite(a.fields()[0]))
+    m = oracle.metrics(Nx, Ny, 2 * np.pi, 1.0, 1, 1.5)
+    w = np.random.default_rng(Nx * Ny).standard_normal((Ny, Nx))
+    wd = torch.from_numpy(w).cuda()
+    pd = torch.zeros_like(wd)
+    a.poisson_solve(wd, pd)
+    torch.cuda.synchronize()
+    assert relerr(pd.cpu().numpy(), oracle.poisson_solve(w, 2 * np.pi, m, 0.0, 2.0)) < 1e-12
+    a.close()
+    b.close()
