@@ -10,18 +10,18 @@
 // which the coarse solver subtracts from its rhs on interior rows. A batch is B whole coarse
 // fields side by side; every field keeps its own periodic x and its own walls.
 //
-// Layout. A pixel p = b Nx Ny + j Nx + i; activations are BF16 [P_pad][C] (channels
-// contiguous), P_pad a multiple of 128. A convolution is im2col (A[p][k], k = tap C + c,
-// tap = 3 (dy + 1) + dx + 1, K padded to a multiple of 64) and the GEMM Z = A . W^T + b with
-// W [N_pad][K] (N_pad a multiple of 16); the GEMM's epilogue writes Z (FP32, kept for the
-// backward pass) and GELU(Z) in BF16, the next layer's input.
+// Layout. A pixel p = b Nx Ny + j Nx + i; activations are BF16 [P][C] (channels contiguous; the input's 5
+// channels padded to 8). A convolution is k_conv (conv_tc.cuh), Z = A . W^T + b with W [N_pad][K] (K = tap C +
+// c, tap = 3 (dy + 1) + dx + 1, padded to a multiple of 64; N_pad a multiple of 16), whose epilogue writes Z
+// (FP32, kept for the backward pass) and GELU(Z) in BF16, the next layer's input.
 //
 // Backward (loss = mean over interior pixels of (z - tau/tau_scale)^2):
-//   dW[n][k] = sum_p dZ[p][n] A[p][k] and db[n] = sum_p dZ[p][n] on the CUDA cores (per-block
-//   partials folded in a fixed order, so the gradients do not depend on scheduling);
-//   dA = dZ . W on the tensor cores (dZ in BF16, padded to 64 channels; W^T kept in BF16);
-//   col2im gathers dA back to the pixels of the layer input and multiplies by GELU'(z).
-// AdamW updates FP32 master weights and re-exports the BF16 W and W^T.
+//   dW[n][k] = sum_p dZ[p][n] A[p][k] with dZ in FP32 (k_wgrad; k_wgrad_out for the one output channel),
+//   db[n] = sum_p dZ[p][n]; per-block partials folded in a fixed order, so the gradients do not depend on
+//   scheduling;
+//   dZ of the layer below = GELU'(z) times the convolution of dZ (BF16) with the flipped taps (k_conv again;
+//   k_dgrad_out for the output layer).
+// AdamW updates FP32 master weights and re-exports the BF16 W and the flipped W.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -30,7 +30,7 @@
 
 #include "common.cuh"
 #include "nse2d_internal.h"
-#include "tc_gemm.cuh"
+#include "conv_tc.cuh"
 #include "../../include/nse2d.h"
 
 namespace nse2d {
@@ -41,10 +41,9 @@ namespace {
 
 constexpr int CN_LAYERS = 4;
 constexpr int CN_CIN = 5;                 // omega, psi, u, v, y
-constexpr int CN_KD = 64;                 // reduction width of the input-gradient GEMM (channels padded)
-constexpr int CN_WG_PB = 64;              // pixels per block of the weight-gradient reduction
+constexpr int CN_C0 = 8;                  // channels of the stored input (padded: 16 bytes a pixel)
 constexpr int CN_NT = 256;
-constexpr int CN_ACT = 2;                 // GELU
+constexpr int CN_OUT_PX = 1024;           // pixels per block of the output layer's weight gradient
 
 int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
@@ -63,14 +62,14 @@ struct Cnn {
     float* mb[CN_LAYERS] = {};
     float* vb[CN_LAYERS] = {};
     __nv_bfloat16* wbf[CN_LAYERS] = {};   // [npad][K]
-    __nv_bfloat16* wtbf[CN_LAYERS] = {};  // [K][64]: W^T, channels padded with zeros
-    __nv_bfloat16* h[CN_LAYERS] = {};     // layer input: h[0] [Ppad][5], h[l] [Ppad][npad[l-1]]
-    __nv_bfloat16* A = nullptr;           // im2col of the current layer [Ppad][Kmax]
-    float* z[CN_LAYERS] = {};             // pre-activations [Ppad][npad]
-    float* dz = nullptr;                  // [Ppad][64]
-    __nv_bfloat16* dzb = nullptr;         // [Ppad][64]
-    float* dA = nullptr;                  // [Ppad][Kmax]
-    float* part = nullptr;                // weight-gradient partials [nblk][npad K + npad]
+    __nv_bfloat16* wtbf[CN_LAYERS] = {};  // layers 1, 2: [cin][9 npad], tap-major, for the gradient of the input
+    __nv_bfloat16* h[CN_LAYERS] = {};     // layer input: h[0] [Ppad][8], h[l] [Ppad][npad[l-1]]
+    float* z[CN_LAYERS] = {};             // pre-activations [Ppad][npad]; the output layer's [Ppad]
+    float* dz[2] = {};                    // dZ of two layers [Ppad][hidden]
+    __nv_bfloat16* dzb[2] = {};           // the same in BF16
+    float* dz_out = nullptr;              // dZ of the output layer [Ppad]
+    int wg_blocks = 0;                    // blocks of the weight-gradient reductions
+    float* part = nullptr;                // their partials
     float* lpart = nullptr;               // loss partials [ceil(Ppad / CN_NT)]
     float* loss = nullptr;                // [1]
     double* y = nullptr;                  // [Ny] wall-normal coordinate (the fifth input)
@@ -104,80 +103,41 @@ struct PackSrc {
     double s0, s1, s2, s3;   // 1 / scale of omega, psi, u, v
 };
 
-// the 5 input channels of every pixel of the batch (zero on padding pixels)
-__global__ void k_pack_input(PackSrc q, __nv_bfloat16* h0, int nxy, int Nx, int P, int Ppad) {
+// The 5 input channels of every pixel of the batch, padded to 8. UV: u and v of the fields' psi (one field;
+// src/ops.cu:47-70) instead of given ones, as the solver's coupling needs them.
+struct PackUv {
+    const double* a_node;
+    double inv_dx, inv_deta;
+};
+template <bool UV>
+__global__ void k_pack_input(PackSrc q, PackUv g, __nv_bfloat16* h0, int nxy, int Nx, int Ny, int P) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= Ppad) return;
-    float v[CN_CIN] = {0.f, 0.f, 0.f, 0.f, 0.f};
-    if (p < P) {
-        const int b = p / nxy, r = p - b * nxy;
-        const size_t src = (size_t)q.idx[b] * nxy + r;
-        v[0] = (float)(q.w[src] * q.s0);
-        v[1] = (float)(q.psi[src] * q.s1);
-        v[2] = (float)(q.u[src] * q.s2);
-        v[3] = (float)(q.v[src] * q.s3);
-        v[4] = (float)q.y[r / Nx];
-    }
-#pragma unroll
-    for (int c = 0; c < CN_CIN; ++c) h0[(size_t)p * CN_CIN + c] = __float2bfloat16_rn(v[c]);
-}
-
-// A[p][k] for one 8-wide chunk of k per thread; taps outside the walls of the pixel's own field
-// read zero, x is periodic within the field.
-__global__ void k_im2col(const __nv_bfloat16* h, int C, int Nx, int Ny, int P, int Ppad, int K, __nv_bfloat16* A) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int nch = K / 8;
-    if (t >= (long long)Ppad * nch) return;
-    const int p = (int)(t / nch), k0 = (int)(t % nch) * 8;
-    const int nxy = Nx * Ny;
+    if (p >= P) return;
     const int b = p / nxy, r = p - b * nxy;
-    const int j = r / Nx, i = r - j * Nx;
-    const size_t base = (size_t)b * nxy;
-    __align__(16) __nv_bfloat16 v[8];
-    if ((C & 7) == 0 && k0 < 9 * C) {                    // the chunk is 8 channels of one tap
-        const int tap = k0 / C, c = k0 - tap * C;
-        const int jj = j + tap / 3 - 1, ii = i + tap % 3 - 1;
-        if (p < P && jj >= 0 && jj < Ny) {
-            const int iw = ii < 0 ? ii + Nx : (ii >= Nx ? ii - Nx : ii);
-            *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(h + (base + (size_t)jj * Nx + iw) * C + c);
-        } else {
-            *reinterpret_cast<uint4*>(v) = make_uint4(0, 0, 0, 0);
-        }
+    const size_t src = (size_t)q.idx[b] * nxy + r;
+    double u, v;
+    const int j = r / Nx;
+    if constexpr (UV) {
+        const int i = r - j * Nx, xm = i == 0 ? Nx - 1 : i - 1, xp = i == Nx - 1 ? 0 : i + 1;
+        const int ym = j == 0 ? 0 : j - 1, yp = j == Ny - 1 ? j : j + 1;
+        const double dpsideta = (q.psi[(size_t)yp * Nx + i] - q.psi[(size_t)ym * Nx + i]) * 0.5 * g.inv_deta;
+        const double dpsidx = (q.psi[(size_t)j * Nx + xp] - q.psi[(size_t)j * Nx + xm]) * 0.5 * g.inv_dx;
+        u = g.a_node[j] * dpsideta;
+        v = -dpsidx;
     } else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int k = k0 + e;
-            float x = 0.f;
-            if (p < P && k < 9 * C) {
-                const int tap = k / C, c = k - tap * C;
-                const int jj = j + tap / 3 - 1, ii = i + tap % 3 - 1;
-                if (jj >= 0 && jj < Ny) {
-                    const int iw = ii < 0 ? ii + Nx : (ii >= Nx ? ii - Nx : ii);
-                    x = __bfloat162float(h[(base + (size_t)jj * Nx + iw) * C + c]);
-                }
-            }
-            v[e] = __float2bfloat16_rn(x);
-        }
+        u = q.u[src];
+        v = q.v[src];
     }
-    *reinterpret_cast<uint4*>(A + (size_t)p * K + k0) = *reinterpret_cast<const uint4*>(v);
-}
-
-// tau = tau_scale z[p][0] away from the walls, 0 on the wall_rows rows next to each wall
-// (batch slot 0)
-__global__ void k_unpack_output(const float* z, int ldz, double* tau, int Nx, int Ny, double ts, int wall_rows) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= Nx * Ny) return;
-    const int j = p / Nx;
-    tau[p] = (j < wall_rows || j >= Ny - wall_rows) ? 0.0 : ts * (double)z[(size_t)p * ldz];
+    const float f[CN_CIN] = {(float)(q.w[src] * q.s0), (float)(q.psi[src] * q.s1), (float)(u * q.s2), (float)(v * q.s3), (float)q.y[j]};
+    *reinterpret_cast<uint4*>(h0 + (size_t)p * CN_C0) = make_uint4(cv_pack2(f[0], f[1]), cv_pack2(f[2], f[3]), cv_pack2(f[4], 0.f), 0u);
 }
 
 // the x-mean of tau on every row: one CTA per row
-__global__ void __launch_bounds__(CN_NT) k_unpack_row_mean(const float* z, int ldz, double* tau, int Nx, int Ny, double ts,
-                                                           int wall_rows) {
+__global__ void __launch_bounds__(CN_NT) k_unpack_row_mean(const float* z, double* tau, int Nx, int Ny, double ts, int wall_rows) {
     __shared__ double red[CN_NT];
     const int j = blockIdx.x;
     double sum = 0.0;
-    for (int i = threadIdx.x; i < Nx; i += CN_NT) sum += (double)z[((size_t)j * Nx + i) * ldz];
+    for (int i = threadIdx.x; i < Nx; i += CN_NT) sum += (double)z[(size_t)j * Nx + i];
     red[threadIdx.x] = sum;
     __syncthreads();
     for (int st = CN_NT / 2; st > 0; st >>= 1) {
@@ -189,27 +149,21 @@ __global__ void __launch_bounds__(CN_NT) k_unpack_row_mean(const float* z, int l
 }
 
 // loss partials and dZ of the output layer: d = z - tau / tau_scale on interior pixels
-__global__ void __launch_bounds__(CN_NT) k_loss(const float* z, int ldz, const double* tau, const int* idx, double inv_ts,
-                                                int Nx, int Ny, int P, int Ppad, int wall_rows, float inv_pint, float* dz,
-                                                __nv_bfloat16* dzb, float* lpart) {
+__global__ void __launch_bounds__(CN_NT) k_loss(const float* z, const double* tau, const int* idx, double inv_ts, int Nx, int Ny, int P,
+                                                int wall_rows, float inv_pint, float* dz, float* lpart) {
     __shared__ float red[CN_NT];
     const int p = blockIdx.x * CN_NT + threadIdx.x;
     const int nxy = Nx * Ny;
     float l = 0.f;
-    if (p < Ppad) {
+    if (p < P) {
         float g = 0.f;
-        if (p < P) {
-            const int b = p / nxy, r = p - b * nxy, j = r / Nx;
-            if (j >= wall_rows && j < Ny - wall_rows) {
-                const float d = z[(size_t)p * ldz] - (float)(tau[(size_t)idx[b] * nxy + r] * inv_ts);
-                l = d * d;
-                g = 2.f * d * inv_pint;
-            }
+        const int b = p / nxy, r = p - b * nxy, j = r / Nx;
+        if (j >= wall_rows && j < Ny - wall_rows) {
+            const float d = z[p] - (float)(tau[(size_t)idx[b] * nxy + r] * inv_ts);
+            l = d * d;
+            g = 2.f * d * inv_pint;
         }
-        for (int c = 0; c < CN_KD; ++c) {
-            dz[(size_t)p * CN_KD + c] = c == 0 ? g : 0.f;
-            dzb[(size_t)p * CN_KD + c] = __float2bfloat16_rn(c == 0 ? g : 0.f);
-        }
+        dz[p] = g;
     }
     red[threadIdx.x] = l;
     __syncthreads();
@@ -219,80 +173,146 @@ __global__ void __launch_bounds__(CN_NT) k_loss(const float* z, int ldz, const d
     }
     if (threadIdx.x == 0) lpart[blockIdx.x] = red[0];
 }
-
-__global__ void k_fold(const float* part, int nblk, int nout, float* out, float scale) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= nout) return;
+__global__ void __launch_bounds__(CN_NT) k_fold_loss(const float* lpart, int n, float scale, float* loss) {
+    __shared__ float red[CN_NT];
     float s = 0.f;
-    for (int b = 0; b < nblk; ++b) s += part[(size_t)b * nout + o];
-    out[o] = s * scale;
-}
-
-// Per-block partial sums of dW[n][k] = sum_p dz[p][n] A[p][k] (o < npad K) and db[n] (o >= npad K)
-// over CN_WG_PB pixels; dz has row stride CN_KD.
-__global__ void __launch_bounds__(CN_NT) k_wgrad(const float* dz, const __nv_bfloat16* A, int npad, int K, float* part) {
-    extern __shared__ __align__(16) unsigned char wg_smem[];
-    float* sdz = reinterpret_cast<float*>(wg_smem);                                  // [PB][npad]
-    __nv_bfloat16* sA = reinterpret_cast<__nv_bfloat16*>(sdz + CN_WG_PB * npad);      // [PB][K]
-    const int p0 = blockIdx.x * CN_WG_PB;
-    for (int e = threadIdx.x; e < CN_WG_PB * npad; e += CN_NT) {
-        const int r = e / npad, n = e - r * npad;
-        sdz[e] = dz[(size_t)(p0 + r) * CN_KD + n];
-    }
-    for (int e = threadIdx.x; e < CN_WG_PB * K / 8; e += CN_NT) {
-        const int r = e / (K / 8), c = e - r * (K / 8);
-        reinterpret_cast<uint4*>(sA)[e] = reinterpret_cast<const uint4*>(A + (size_t)(p0 + r) * K)[c];
-    }
+    for (int i = threadIdx.x; i < n; i += CN_NT) s += lpart[i];
+    red[threadIdx.x] = s;
     __syncthreads();
-    const int nout = npad * K + npad;
-    float* out = part + (size_t)blockIdx.x * nout;
-    for (int o = threadIdx.x; o < nout; o += CN_NT) {
-        float s = 0.f;
-        if (o < npad * K) {
-            const int n = o / K, k = o - n * K;
-            for (int r = 0; r < CN_WG_PB; ++r) s = fmaf(sdz[r * npad + n], __bfloat162float(sA[r * K + k]), s);
-        } else {
-            const int n = o - npad * K;
-            for (int r = 0; r < CN_WG_PB; ++r) s += sdz[r * npad + n];
-        }
-        out[o] = s;
+    for (int st = CN_NT / 2; st > 0; st >>= 1) {
+        if ((int)threadIdx.x < st) red[threadIdx.x] += red[threadIdx.x + st];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *loss = red[0] * scale;
+}
+
+// Weight-gradient partials [nblk][nk][nn] and bias partials [nblk][nn] (after them) -> gw[n][k] (row stride K)
+// and gb[n]. A block folds 32 outputs in eight slices of the partials' blocks; the order is fixed.
+__global__ void __launch_bounds__(256) k_fold_grads(const float* part, int nblk, int nk, int nn, int K, float* gw, float* gb) {
+    __shared__ float red[8][33];
+    const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
+    const int nout = (nk + 1) * nn, o = blockIdx.x * 32 + lane;
+    const bool bias = o >= nk * nn;
+    const float* src = bias ? part + (size_t)nblk * nk * nn + (o - nk * nn) : part + o;
+    const size_t stride = bias ? nn : (size_t)nk * nn;
+    float s = 0.f;
+    if (o < nout) {
+        const int b0 = (int)((long long)sl * nblk / 8), b1 = (int)((long long)(sl + 1) * nblk / 8);
+#pragma unroll 8
+        for (int b = b0; b < b1; ++b) s += src[(size_t)b * stride];
+    }
+    red[sl][lane] = s;
+    __syncthreads();
+    if (sl == 0 && o < nout) {
+#pragma unroll
+        for (int q = 1; q < 8; ++q) s += red[q][lane];
+        if (bias) gb[o - nk * nn] = s;
+        else gw[(size_t)(o % nn) * K + o / nn] = s;
     }
 }
 
-// dh[q][c] = sum over taps of dA[q - tap offset][tap C + c] (source rows inside the walls of the
-// same field), then the activation's derivative of the layer below: dz[q][c] = dh GELU'(z_prev);
-// channels >= C written as zero.
-__global__ void k_col2im_act(const float* dA, int K, int C, const float* zprev, int ldzp, int Nx, int Ny, int P, int Ppad,
-                             float* dz, __nv_bfloat16* dzb) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)Ppad * CN_KD) return;
-    const int q = (int)(t / CN_KD), c = (int)(t % CN_KD);
-    float g = 0.f;
-    if (q < P && c < C) {
-        const int nxy = Nx * Ny;
-        const int b = q / nxy, r = q - b * nxy;
-        const int j = r / Nx, i = r - j * Nx;
-        const size_t base = (size_t)b * nxy;
-        float s = 0.f;
+// dZ of the layer below the output layer: the one output channel's dZ (BF16) times the flipped taps of W, times
+// GELU'(z). A thread takes eight channels of a pixel. Products of two BF16 values are exact in FP32.
+__global__ void __launch_bounds__(CN_NT) k_dgrad_out(const float* dz, const __nv_bfloat16* w, int C, const float* zprev, int Nx, int Ny, int P,
+                                                     float* dzo, __nv_bfloat16* dzb) {
+    extern __shared__ __align__(16) float ws[];                    // [9][C]
+    for (int e = threadIdx.x; e < 9 * C; e += CN_NT) ws[e] = __bfloat162float(w[e]);
+    __syncthreads();
+    const int nq = C >> 3;
+    const long long t = (long long)blockIdx.x * CN_NT + threadIdx.x;
+    const int p = (int)(t / nq), c = (int)(t - (long long)p * nq) * 8;
+    if (p >= P) return;
+    const size_t o = (size_t)p * C + c;
+    const float4 z0 = __ldg(reinterpret_cast<const float4*>(zprev + o)), z1 = __ldg(reinterpret_cast<const float4*>(zprev + o) + 1);
+    const CvPix q = cv_pix(p, P, Nx, Ny);
+    float d[9], s[8] = {};
+#pragma unroll
+    for (int tap = 0; tap < 9; ++tap) {
+        int src;
+        d[tap] = cv_tap(q, 1 - tap / 3, 1 - tap % 3, Nx, Ny, src) ? __bfloat162float(__float2bfloat16_rn(__ldg(dz + src))) : 0.f;
+    }
+#pragma unroll
+    for (int tap = 0; tap < 9; ++tap) {
+        const float4 a = *reinterpret_cast<const float4*>(ws + tap * C + c), b = *reinterpret_cast<const float4*>(ws + tap * C + c + 4);
+        s[0] = fmaf(d[tap], a.x, s[0]); s[1] = fmaf(d[tap], a.y, s[1]); s[2] = fmaf(d[tap], a.z, s[2]); s[3] = fmaf(d[tap], a.w, s[3]);
+        s[4] = fmaf(d[tap], b.x, s[4]); s[5] = fmaf(d[tap], b.y, s[5]); s[6] = fmaf(d[tap], b.z, s[6]); s[7] = fmaf(d[tap], b.w, s[7]);
+    }
+    s[0] *= tg_gelu_grad(z0.x); s[1] *= tg_gelu_grad(z0.y); s[2] *= tg_gelu_grad(z0.z); s[3] *= tg_gelu_grad(z0.w);
+    s[4] *= tg_gelu_grad(z1.x); s[5] *= tg_gelu_grad(z1.y); s[6] *= tg_gelu_grad(z1.z); s[7] *= tg_gelu_grad(z1.w);
+    reinterpret_cast<float4*>(dzo + o)[0] = make_float4(s[0], s[1], s[2], s[3]);
+    reinterpret_cast<float4*>(dzo + o)[1] = make_float4(s[4], s[5], s[6], s[7]);
+    *reinterpret_cast<uint4*>(dzb + o) = make_uint4(cv_pack2(s[0], s[1]), cv_pack2(s[2], s[3]), cv_pack2(s[4], s[5]), cv_pack2(s[6], s[7]));
+}
+
+// The output layer's weight gradient: dW[tap C + c] = sum_q h[q][c] dZ[q - offset of the tap], db = sum dZ, as
+// partials [nblk][9 C] and [nblk]. A warp takes 32 pixels at a time: every lane gathers the nine dZ of its own
+// pixel into shared memory, then the lanes are the channels (one or two each) and walk over the 32 pixels, whose
+// dZ they read as broadcasts. Gathering per pixel by the whole warp took 95 us for 264192 pixels.
+__global__ void __launch_bounds__(CN_NT) k_wgrad_out(const __nv_bfloat16* h, const float* dz, int C, int Nx, int Ny, int P, float* part) {
+    __shared__ float red[8][9 * 64 + 1];
+    __shared__ __align__(16) float sd[8][32][12];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int p1 = min(P, ((int)blockIdx.x + 1) * CN_OUT_PX);
+    float a[2][9] = {}, sb = 0.f;
+    for (int p0 = blockIdx.x * CN_OUT_PX + warp * 32; p0 < p1; p0 += 8 * 32) {
+        const CvPix q = cv_pix(p0 + lane, p1, Nx, Ny);             // beyond p1: zeros
+        float d[9];
 #pragma unroll
         for (int tap = 0; tap < 9; ++tap) {
-            const int dy = tap / 3 - 1, dx = tap % 3 - 1;
-            const int jp = j - dy;
-            if (jp < 0 || jp >= Ny) continue;
-            int ip = i - dx;
-            ip = ip < 0 ? ip + Nx : (ip >= Nx ? ip - Nx : ip);
-            s += dA[(base + (size_t)jp * Nx + ip) * K + tap * C + c];
+            int src;
+            d[tap] = cv_tap(q, 1 - tap / 3, 1 - tap % 3, Nx, Ny, src) ? __ldg(dz + src) : 0.f;
         }
-        g = s * tg_gelu_grad(zprev[(size_t)q * ldzp + c]);
+        sb += d[4];
+        __syncwarp();
+        float4* w = reinterpret_cast<float4*>(sd[warp][lane]);
+        w[0] = make_float4(d[0], d[1], d[2], d[3]);
+        w[1] = make_float4(d[4], d[5], d[6], d[7]);
+        w[2] = make_float4(d[8], 0.f, 0.f, 0.f);
+        __syncwarp();
+        const int n = min(32, p1 - p0);
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            const int c = lane + 32 * g;
+            if (c >= C) continue;
+            const __nv_bfloat16* hp = h + (size_t)p0 * C + c;
+#pragma unroll 8
+            for (int k = 0; k < n; ++k) {
+                const float x = __bfloat162float(hp[(size_t)k * C]);
+                const float4* v = reinterpret_cast<const float4*>(sd[warp][k]);
+                const float4 u0 = v[0], u1 = v[1];
+                const float u8 = sd[warp][k][8];
+                a[g][0] = fmaf(u0.x, x, a[g][0]); a[g][1] = fmaf(u0.y, x, a[g][1]); a[g][2] = fmaf(u0.z, x, a[g][2]);
+                a[g][3] = fmaf(u0.w, x, a[g][3]); a[g][4] = fmaf(u1.x, x, a[g][4]); a[g][5] = fmaf(u1.y, x, a[g][5]);
+                a[g][6] = fmaf(u1.z, x, a[g][6]); a[g][7] = fmaf(u1.w, x, a[g][7]); a[g][8] = fmaf(u8, x, a[g][8]);
+            }
+        }
     }
-    dz[t] = g;
-    dzb[t] = __float2bfloat16_rn(g);
+#pragma unroll
+    for (int g = 0; g < 2; ++g)
+        if (lane + 32 * g < C)
+            for (int tap = 0; tap < 9; ++tap) red[warp][tap * C + lane + 32 * g] = a[g][tap];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sb += __shfl_down_sync(0xffffffffu, sb, o);
+    if (lane == 0) red[warp][9 * C] = sb;
+    __syncthreads();
+    for (int o = threadIdx.x; o <= 9 * C; o += CN_NT) {
+        float s = red[0][o];
+        for (int w = 1; w < 8; ++w) s += red[w][o];
+        if (o < 9 * C) part[(size_t)blockIdx.x * 9 * C + o] = s;
+        else part[(size_t)gridDim.x * 9 * C + blockIdx.x] = s;
+    }
 }
 
-__global__ void k_adamw(float* w, const float* g, float* m, float* v, int n, float lr, float b1, float b2, float eps,
-                        float wd, float bc1, float bc2) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n) return;
+// One layer's parameters (AdamW and the export of the BF16 copies).
+struct LayerParams {
+    float *w, *gw, *mw, *vw, *b, *gb, *mb, *vb;
+    __nv_bfloat16 *wbf, *wt;               // wt: [cin][9 npad] or null
+    int npad, K, cin;
+};
+struct AllLayers { LayerParams l[CN_LAYERS]; };
+
+__device__ __forceinline__ void adamw_one(float* w, const float* g, float* m, float* v, int e, float lr, float b1, float b2, float eps,
+                                          float wd, float bc1, float bc2) {
     const float gg = g[e];
     const float mm = b1 * m[e] + (1.f - b1) * gg;
     const float vv = b2 * v[e] + (1.f - b2) * gg * gg;
@@ -301,18 +321,29 @@ __global__ void k_adamw(float* w, const float* g, float* m, float* v, int n, flo
     const float mh = mm / bc1, vh = vv / bc2;
     w[e] -= lr * (mh / (sqrtf(vh) + eps) + wd * w[e]);
 }
-
-__global__ void k_export_w(const float* w, int npad, int K, __nv_bfloat16* wbf, __nv_bfloat16* wtbf) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= K * CN_KD) return;
-    const int k = e / CN_KD, n = e - k * CN_KD;
-    if (n < npad) {
-        const __nv_bfloat16 b = __float2bfloat16_rn(w[(size_t)n * K + k]);
-        wbf[(size_t)n * K + k] = b;
-        wtbf[e] = b;
-    } else {
-        wtbf[e] = __float2bfloat16_rn(0.f);
+// W (BF16), and the flipped-tap gradient's [cin][tap npad + n]
+__device__ __forceinline__ void export_one(const LayerParams& q, int e) {
+    const int n = e / q.K, k = e - n * q.K;
+    const __nv_bfloat16 b = __float2bfloat16_rn(q.w[e]);
+    q.wbf[e] = b;
+    if (q.wt && k < 9 * q.cin) {
+        const int tap = k / q.cin, c = k - tap * q.cin;
+        q.wt[(size_t)c * 9 * q.npad + tap * q.npad + n] = b;
     }
+}
+// grid: (blocks of the largest layer, layers)
+__global__ void __launch_bounds__(CN_NT) k_adamw(AllLayers all, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2) {
+    const LayerParams& q = all.l[blockIdx.y];
+    const int e = blockIdx.x * CN_NT + threadIdx.x;
+    if (e < q.npad * q.K) {
+        adamw_one(q.w, q.gw, q.mw, q.vw, e, lr, b1, b2, eps, wd, bc1, bc2);
+        export_one(q, e);
+    }
+    if (e < q.npad) adamw_one(q.b, q.gb, q.mb, q.vb, e, lr, b1, b2, eps, 0.f, bc1, bc2);
+}
+__global__ void __launch_bounds__(CN_NT) k_export_w(LayerParams q) {
+    const int e = blockIdx.x * CN_NT + threadIdx.x;
+    if (e < q.npad * q.K) export_one(q, e);
 }
 
 // Top-hat filter of a fine field onto a coarse grid whose nodes are every rx-th column and
@@ -343,19 +374,61 @@ __global__ void k_box_filter(const double* f, int Nxf, int Nyf, double* c, int N
 
 int grid_of(long long n, int nt = CN_NT) { return (int)((n + nt - 1) / nt); }
 
-int gemm(Cnn* n, const __nv_bfloat16* A, const __nv_bfloat16* B, const float* bias, float* Cf, __nv_bfloat16* Cb, int M,
-         int N, int K, int ldc, int act, cudaStream_t s) {
-    TcGemmParams p{};
-    p.A = A; p.B = B; p.bias = bias; p.Cf = Cf; p.Cb = Cb; p.err = n ? n->err : nullptr;
-    p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.act = act;
-    return tc_gemm_launch(p, s);
+LayerParams layer_params(const Cnn* n, int l) {
+    return LayerParams{n->w32[l], n->gw[l], n->mw[l], n->vw[l], n->b32[l], n->gb[l], n->mb[l], n->vb[l],
+                       n->wbf[l], n->wtbf[l], n->npad[l], n->K[l], n->cin[l]};
 }
 
 int export_layer(Cnn* n, int l, cudaStream_t s) {
-    k_export_w<<<grid_of((long long)n->K[l] * CN_KD), CN_NT, 0, s>>>(n->w32[l], n->npad[l], n->K[l], n->wbf[l], n->wtbf[l]);
+    k_export_w<<<grid_of((long long)n->npad[l] * n->K[l]), CN_NT, 0, s>>>(layer_params(n, l));
     NSE_CUDA_TRY(cudaGetLastError());
     return 0;
 }
+
+template <int C, int MODE> int conv_t(const ConvParams& p, bool setup, cudaStream_t s) {
+    if (setup) {
+        NSE_CUDA_TRY(cudaFuncSetAttribute(k_conv<C, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cv_smem_bytes<C>(64)));
+        return 0;
+    }
+    k_conv<C, MODE><<<(p.P + TG_BM - 1) / TG_BM, CV_NT, cv_smem_bytes<C>(p.N), s>>>(p);
+    NSE_CUDA_TRY(cudaGetLastError());
+    return 0;
+}
+// a convolution of C input channels (8: the input layer); setup: only the kernel's shared-memory limit
+template <int MODE> int conv(const ConvParams& p, int C, bool setup, cudaStream_t s) {
+    if constexpr (MODE == CV_FWD) if (C == CN_C0) return conv_t<CN_C0, MODE>(p, setup, s);
+    switch (C) {
+        case 16: return conv_t<16, MODE>(p, setup, s);
+        case 32: return conv_t<32, MODE>(p, setup, s);
+        case 48: return conv_t<48, MODE>(p, setup, s);
+        case 64: return conv_t<64, MODE>(p, setup, s);
+        default: set_error("no convolution of %d channels", C); return -1;
+    }
+}
+
+template <int C, int N, int TG> int wgrad_t(const WgradParams& p, int blocks, bool setup, cudaStream_t s) {
+    constexpr size_t sm = wg_smem_bytes<C, N, TG>();
+    if (setup) {
+        NSE_CUDA_TRY(cudaFuncSetAttribute(k_wgrad<C, N, TG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        return 0;
+    }
+    k_wgrad<C, N, TG><<<dim3(blocks, C == CN_C0 ? 1 : 9 / TG), WG_NT, sm, s>>>(p);
+    NSE_CUDA_TRY(cudaGetLastError());
+    return 0;
+}
+// weight gradient of the input layer (input = true) or of a hidden layer of H channels; all nine taps in a CTA
+// while its accumulators fit the registers
+int wgrad(const WgradParams& p, bool input, int H, int blocks, bool setup, cudaStream_t s) {
+    switch (H) {
+        case 16: return input ? wgrad_t<CN_C0, 16, 9>(p, blocks, setup, s) : wgrad_t<16, 16, 9>(p, blocks, setup, s);
+        case 32: return input ? wgrad_t<CN_C0, 32, 9>(p, blocks, setup, s) : wgrad_t<32, 32, 9>(p, blocks, setup, s);
+        case 48: return input ? wgrad_t<CN_C0, 48, 9>(p, blocks, setup, s) : wgrad_t<48, 48, 3>(p, blocks, setup, s);
+        case 64: return input ? wgrad_t<CN_C0, 64, 9>(p, blocks, setup, s) : wgrad_t<64, 64, 3>(p, blocks, setup, s);
+        default: set_error("no weight gradient of %d channels", H); return -1;
+    }
+}
+// blocks of a weight gradient over P pixels: tiles of 64 pixels strided over the resident CTAs
+int wgrad_blocks(const Cnn* n) { return std::max(1, std::min((n->P + WG_PX - 1) / WG_PX, n->wg_blocks)); }
 
 void set_batch(Cnn* n, int nb) {
     n->nb = nb;
@@ -394,18 +467,30 @@ int tc_gemm_setup() {
     return 0;
 }
 
-// Forward pass of the current batch from the packed sources.
-static int cnn_forward_batch(Cnn* n, const PackSrc& src, cudaStream_t s) {
-    k_pack_input<<<grid_of(n->Ppad), CN_NT, 0, s>>>(src, n->h[0], n->nxy, n->Nx, n->P, n->Ppad);
+// Forward pass of the current batch from the packed sources. keep: the pre-activations of every layer (for the
+// backward pass); else only the output layer's, and tau directly when it is given.
+static int cnn_forward_batch(Cnn* n, const PackSrc& src, const PackUv* uv, bool keep, double* tau, cudaStream_t s) {
+    if (uv)
+        k_pack_input<true><<<grid_of(n->P), CN_NT, 0, s>>>(src, *uv, n->h[0], n->nxy, n->Nx, n->Ny, n->P);
+    else
+        k_pack_input<false><<<grid_of(n->P), CN_NT, 0, s>>>(src, PackUv{}, n->h[0], n->nxy, n->Nx, n->Ny, n->P);
     NSE_CUDA_TRY(cudaGetLastError());
     for (int l = 0; l < CN_LAYERS; ++l) {
-        k_im2col<<<grid_of((long long)n->Ppad * (n->K[l] / 8)), CN_NT, 0, s>>>(n->h[l], n->cin[l], n->Nx, n->Ny, n->P, n->Ppad,
-                                                                              n->K[l], n->A);
-        NSE_CUDA_TRY(cudaGetLastError());
         const bool last = (l == CN_LAYERS - 1);
-        if (gemm(n, n->A, n->wbf[l], n->b32[l], n->z[l], last ? nullptr : n->h[l + 1], n->Ppad, n->npad[l], n->K[l],
-                 n->npad[l], CN_ACT, s))
-            return -1;
+        ConvParams p{};
+        p.h = n->h[l]; p.W = n->wbf[l]; p.bias = n->b32[l]; p.err = n->err;
+        p.Nx = n->Nx; p.Ny = n->Ny; p.P = n->P; p.N = n->npad[l]; p.ldw = n->K[l];
+        if (last) {
+            p.z = tau ? nullptr : n->z[l];
+            p.tau = tau;
+            p.wall_rows = n->wall_rows;
+            p.ts = n->out_tau * n->gain;
+            if (conv<CV_OUT>(p, n->cin[l], false, s)) return -1;
+        } else {
+            p.z = keep ? n->z[l] : nullptr;
+            p.hn = n->h[l + 1];
+            if (conv<CV_FWD>(p, l == 0 ? CN_C0 : n->cin[l], false, s)) return -1;
+        }
     }
     return 0;
 }
@@ -418,54 +503,59 @@ static PackSrc pack_src(const Cnn* n, const double* w, const double* psi, const 
 }
 
 // Inference on one field (slot 0 of the index table is always sample 0); graph-capturable.
-int cnn_forward(Cnn* n, const double* w, const double* psi, const double* u, const double* v, double* tau, cudaStream_t s) {
+static int cnn_forward_field(Cnn* n, const PackSrc& src, const PackUv* uv, double* tau, cudaStream_t s) {
     set_batch(n, 1);
-    if (cnn_forward_batch(n, pack_src(n, w, psi, u, v), s)) return -1;
-    if (n->row_mean)
-        k_unpack_row_mean<<<n->Ny, CN_NT, 0, s>>>(n->z[CN_LAYERS - 1], n->npad[CN_LAYERS - 1], tau, n->Nx, n->Ny,
-                                                  n->out_tau * n->gain, n->wall_rows);
-    else
-        k_unpack_output<<<grid_of(n->nxy), CN_NT, 0, s>>>(n->z[CN_LAYERS - 1], n->npad[CN_LAYERS - 1], tau, n->Nx, n->Ny,
-                                                          n->out_tau * n->gain, n->wall_rows);
-    NSE_CUDA_TRY(cudaGetLastError());
+    if (cnn_forward_batch(n, src, uv, false, n->row_mean ? nullptr : tau, s)) return -1;
+    if (n->row_mean) {
+        k_unpack_row_mean<<<n->Ny, CN_NT, 0, s>>>(n->z[CN_LAYERS - 1], tau, n->Nx, n->Ny, n->out_tau * n->gain, n->wall_rows);
+        NSE_CUDA_TRY(cudaGetLastError());
+    }
     return 0;
+}
+int cnn_forward(Cnn* n, const double* w, const double* psi, const double* u, const double* v, double* tau, cudaStream_t s) {
+    return cnn_forward_field(n, pack_src(n, w, psi, u, v), nullptr, tau, s);
+}
+// the same with u and v of psi
+int cnn_forward_psi(Cnn* n, const double* w, const double* psi, const double* a_node, double inv_dx, double inv_deta, double* tau,
+                    cudaStream_t s) {
+    const PackUv uv{a_node, inv_dx, inv_deta};
+    return cnn_forward_field(n, pack_src(n, w, psi, nullptr, nullptr), &uv, tau, s);
 }
 
 // Loss against tau (samples idx of the batch) and the gradients of every layer (after the forward pass).
 static int cnn_backward(Cnn* n, const double* tau, cudaStream_t s) {
-    const int nlb = (n->Ppad + CN_NT - 1) / CN_NT;
+    constexpr int L = CN_LAYERS - 1;
+    const int nlb = grid_of(n->P), H = n->npad[0];
     const int pint = n->nb * n->Nx * (n->Ny - 2 * n->wall_rows);
-    k_loss<<<nlb, CN_NT, 0, s>>>(n->z[CN_LAYERS - 1], n->npad[CN_LAYERS - 1], tau, n->idx, 1.0 / n->out_tau, n->Nx, n->Ny, n->P,
-                                 n->Ppad, n->wall_rows, 1.f / (float)pint, n->dz, n->dzb, n->lpart);
+    k_loss<<<nlb, CN_NT, 0, s>>>(n->z[L], tau, n->idx, 1.0 / n->out_tau, n->Nx, n->Ny, n->P, n->wall_rows, 1.f / (float)pint, n->dz_out,
+                                 n->lpart);
+    k_fold_loss<<<1, CN_NT, 0, s>>>(n->lpart, nlb, 1.f / (float)pint, n->loss);
     NSE_CUDA_TRY(cudaGetLastError());
-    k_fold<<<1, 32, 0, s>>>(n->lpart, nlb, 1, n->loss, 1.f / (float)pint);
+    auto fold = [&](int l, int nblk, int nk, int nn) {
+        k_fold_grads<<<((nk + 1) * nn + 31) / 32, 256, 0, s>>>(n->part, nblk, nk, nn, n->K[l], n->gw[l], n->gb[l]);
+        return cudaGetLastError();
+    };
+    // the output layer: its one channel on the CUDA cores
+    const int nob = (n->P + CN_OUT_PX - 1) / CN_OUT_PX;
+    k_wgrad_out<<<nob, CN_NT, 0, s>>>(n->h[L], n->dz_out, n->cin[L], n->Nx, n->Ny, n->P, n->part);
     NSE_CUDA_TRY(cudaGetLastError());
-    for (int l = CN_LAYERS - 1; l >= 0; --l) {
-        // the layer's im2col again (one A buffer is kept)
-        k_im2col<<<grid_of((long long)n->Ppad * (n->K[l] / 8)), CN_NT, 0, s>>>(n->h[l], n->cin[l], n->Nx, n->Ny, n->P, n->Ppad,
-                                                                              n->K[l], n->A);
-        NSE_CUDA_TRY(cudaGetLastError());
-        const int nblk = n->Ppad / CN_WG_PB, nout = n->npad[l] * n->K[l] + n->npad[l];
-        const size_t sm = (size_t)CN_WG_PB * n->npad[l] * 4 + (size_t)CN_WG_PB * n->K[l] * 2;
-        k_wgrad<<<nblk, CN_NT, sm, s>>>(n->dz, n->A, n->npad[l], n->K[l], n->part);
-        NSE_CUDA_TRY(cudaGetLastError());
-        // fold into the scratch dA (weights then biases), then copy out
-        k_fold<<<grid_of(nout), CN_NT, 0, s>>>(n->part, nblk, nout, n->dA, 1.f);
-        NSE_CUDA_TRY(cudaGetLastError());
-        NSE_CUDA_TRY(cudaMemcpyAsync(n->gw[l], n->dA, sizeof(float) * n->npad[l] * n->K[l], cudaMemcpyDeviceToDevice, s));
-        NSE_CUDA_TRY(cudaMemcpyAsync(n->gb[l], n->dA + (size_t)n->npad[l] * n->K[l], sizeof(float) * n->npad[l],
-                                     cudaMemcpyDeviceToDevice, s));
+    NSE_CUDA_TRY(fold(L, nob, 9 * n->cin[L], 1));
+    int cur = 0;
+    k_dgrad_out<<<grid_of((long long)n->P * (H / 8)), CN_NT, 9 * H * sizeof(float), s>>>(n->dz_out, n->wbf[L], H, n->z[L - 1], n->Nx, n->Ny,
+                                                                                      n->P, n->dz[cur], n->dzb[cur]);
+    NSE_CUDA_TRY(cudaGetLastError());
+    const int nwb = wgrad_blocks(n);
+    for (int l = L - 1; l >= 0; --l) {
+        const int nk = l == 0 ? 48 : 9 * n->cin[l];
+        WgradParams wp{n->h[l], n->dz[cur], n->part, n->Nx, n->Ny, n->P, nk};
+        if (wgrad(wp, l == 0, H, nwb, false, s)) return -1;
+        NSE_CUDA_TRY(fold(l, nwb, nk, H));
         if (l == 0) break;
-        // dA = dZ . W: N tiles of at most 256 columns of K
-        for (int c0 = 0; c0 < n->K[l]; c0 += 256) {
-            const int nc = std::min(256, n->K[l] - c0);
-            if (gemm(n, n->dzb, n->wtbf[l] + (size_t)c0 * CN_KD, nullptr, n->dA + c0, nullptr, n->Ppad, nc, CN_KD, n->K[l], 0, s))
-                return -1;
-        }
-        k_col2im_act<<<grid_of((long long)n->Ppad * CN_KD), CN_NT, 0, s>>>(n->dA, n->K[l], n->cin[l], n->z[l - 1],
-                                                                            n->npad[l - 1], n->Nx, n->Ny, n->P, n->Ppad, n->dz,
-                                                                            n->dzb);
-        NSE_CUDA_TRY(cudaGetLastError());
+        ConvParams p{};
+        p.h = n->dzb[cur]; p.W = n->wtbf[l]; p.zprev = n->z[l - 1]; p.z = n->dz[cur ^ 1]; p.hn = n->dzb[cur ^ 1]; p.err = n->err;
+        p.Nx = n->Nx; p.Ny = n->Ny; p.P = n->P; p.N = n->cin[l]; p.ldw = 9 * n->npad[l];
+        if (conv<CV_DGRAD>(p, n->npad[l], false, s)) return -1;
+        cur ^= 1;
     }
     return 0;
 }
@@ -474,13 +564,14 @@ static int cnn_adamw(Cnn* n, float lr, float wd, cudaStream_t s) {
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     n->step += 1;
     const float bc1 = 1.f - powf(b1, (float)n->step), bc2 = 1.f - powf(b2, (float)n->step);
+    AllLayers all;
+    int most = 0;
     for (int l = 0; l < CN_LAYERS; ++l) {
-        const int nw = n->npad[l] * n->K[l];
-        k_adamw<<<grid_of(nw), CN_NT, 0, s>>>(n->w32[l], n->gw[l], n->mw[l], n->vw[l], nw, lr, b1, b2, eps, wd, bc1, bc2);
-        k_adamw<<<1, CN_NT, 0, s>>>(n->b32[l], n->gb[l], n->mb[l], n->vb[l], n->npad[l], lr, b1, b2, eps, 0.f, bc1, bc2);
-        NSE_CUDA_TRY(cudaGetLastError());
-        if (export_layer(n, l, s)) return -1;
+        all.l[l] = layer_params(n, l);
+        most = std::max(most, n->npad[l] * n->K[l]);
     }
+    k_adamw<<<dim3(grid_of(most), CN_LAYERS), CN_NT, 0, s>>>(all, lr, b1, b2, eps, wd, bc1, bc2);
+    NSE_CUDA_TRY(cudaGetLastError());
     return 0;
 }
 
@@ -493,7 +584,8 @@ void cnn_free(Cnn* n) {
         cudaFree(n->mw[l]); cudaFree(n->vw[l]); cudaFree(n->mb[l]); cudaFree(n->vb[l]);
         cudaFree(n->wbf[l]); cudaFree(n->wtbf[l]); cudaFree(n->h[l]); cudaFree(n->z[l]);
     }
-    cudaFree(n->A); cudaFree(n->dz); cudaFree(n->dzb); cudaFree(n->dA); cudaFree(n->part); cudaFree(n->lpart);
+    for (int k = 0; k < 2; ++k) { cudaFree(n->dz[k]); cudaFree(n->dzb[k]); }
+    cudaFree(n->dz_out); cudaFree(n->part); cudaFree(n->lpart);
     cudaFree(n->loss); cudaFree(n->y); cudaFree(n->idx); cudaFree(n->err);
     delete n;
 }
@@ -511,40 +603,47 @@ static int cnn_create(int Nx, int Ny, int hidden, int max_batch, const double* y
     set_batch(n, max_batch);
     const int Pmax = n->Ppad;
     const int ch[CN_LAYERS + 1] = {CN_CIN, hidden, hidden, hidden, 1};
-    int kmax = 0, nmax = 0;
     for (int l = 0; l < CN_LAYERS; ++l) {
         n->cin[l] = (l == 0) ? CN_CIN : round_up(ch[l], 16);
         n->cout[l] = ch[l + 1];
         n->npad[l] = round_up(ch[l + 1], 16);
         n->K[l] = round_up(9 * n->cin[l], 64);
-        kmax = std::max(kmax, n->K[l]);
-        nmax = std::max(nmax, n->npad[l] * n->K[l] + n->npad[l]);
     }
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int H = n->npad[0];
+    n->wg_blocks = 2 * (sms > 0 ? sms : 148);                       // resident CTAs of k_wgrad
     auto fail = [&]() { cnn_free(n); return -1; };
     for (int l = 0; l < CN_LAYERS; ++l) {
         const size_t nw = (size_t)n->npad[l] * n->K[l];
         if (cn_alloc(&n->w32[l], nw) || cn_alloc(&n->b32[l], n->npad[l]) || cn_alloc(&n->gw[l], nw) ||
             cn_alloc(&n->gb[l], n->npad[l]) || cn_alloc(&n->mw[l], nw) || cn_alloc(&n->vw[l], nw) ||
             cn_alloc(&n->mb[l], n->npad[l]) || cn_alloc(&n->vb[l], n->npad[l]) || cn_alloc(&n->wbf[l], nw) ||
-            cn_alloc(&n->wtbf[l], (size_t)n->K[l] * CN_KD) || cn_alloc(&n->h[l], (size_t)Pmax * n->cin[l]) ||
-            cn_alloc(&n->z[l], (size_t)Pmax * n->npad[l]))
+            cn_alloc(&n->h[l], (size_t)Pmax * (l == 0 ? CN_C0 : n->cin[l])) ||
+            cn_alloc(&n->z[l], (size_t)Pmax * (l == CN_LAYERS - 1 ? 1 : n->npad[l])))
             return fail();
+        if (l >= 1 && l < CN_LAYERS - 1 && cn_alloc(&n->wtbf[l], (size_t)n->cin[l] * 9 * n->npad[l])) return fail();
     }
-    if (cn_alloc(&n->A, (size_t)Pmax * kmax) || cn_alloc(&n->dz, (size_t)Pmax * CN_KD) ||
-        cn_alloc(&n->dzb, (size_t)Pmax * CN_KD) || cn_alloc(&n->dA, std::max((size_t)Pmax * kmax, (size_t)nmax)) ||
-        cn_alloc(&n->part, (size_t)(Pmax / CN_WG_PB) * nmax) || cn_alloc(&n->lpart, (size_t)(Pmax + CN_NT - 1) / CN_NT) ||
+    for (int k = 0; k < 2; ++k)
+        if (cn_alloc(&n->dz[k], (size_t)Pmax * H) || cn_alloc(&n->dzb[k], (size_t)Pmax * H)) return fail();
+    const size_t npart = std::max((size_t)wgrad_blocks(n) * (9 * H + 1) * H, (size_t)((Pmax + CN_OUT_PX - 1) / CN_OUT_PX) * (9 * H + 1));
+    if (cn_alloc(&n->dz_out, Pmax) || cn_alloc(&n->part, npart) || cn_alloc(&n->lpart, (size_t)(Pmax + CN_NT - 1) / CN_NT) ||
         cn_alloc(&n->loss, 1) || cn_alloc(&n->y, Ny) || cn_alloc(&n->idx, max_batch) || cn_alloc(&n->err, 1))
         return fail();
     if (cudaMemcpy(n->y, y_host, sizeof(double) * Ny, cudaMemcpyHostToDevice) != cudaSuccess) {
         set_error("nse2d_cnn_create: y upload");
         return fail();
     }
-    size_t wg_max = 0;
-    for (int l = 0; l < CN_LAYERS; ++l)
-        wg_max = std::max(wg_max, (size_t)CN_WG_PB * n->npad[l] * 4 + (size_t)CN_WG_PB * n->K[l] * 2);
-    if (cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wg_max) != cudaSuccess) {
-        set_error("nse2d_cnn_create: %s", cudaGetErrorString(cudaGetLastError()));
-        return fail();
+    {
+        ConvParams p{};
+        bool bad = false;
+        p.N = H;
+        bad |= conv<CV_FWD>(p, CN_C0, true, 0) || conv<CV_FWD>(p, H, true, 0) || conv<CV_DGRAD>(p, H, true, 0);
+        p.N = n->npad[CN_LAYERS - 1];
+        bad |= conv<CV_OUT>(p, H, true, 0) != 0;
+        bad |= wgrad(WgradParams{}, true, H, 0, true, 0) || wgrad(WgradParams{}, false, H, 0, true, 0);
+        if (bad) return fail();
     }
     set_batch(n, 1);
     *out = n;
@@ -696,8 +795,8 @@ int nse2d_set_closure(nse2d_ctx* ctx, nse2d_cnn* net, int every_stage) {
     }
     if (c->prec32) { set_error("nse2d_set_closure: the closure runs with precision 64"); return -1; }
     if (!c->closure_tau) {
-        NSE_CUDA_TRY(cudaMalloc((void**)&c->closure_tau, 3 * c->N * sizeof(double)));
-        NSE_CUDA_TRY(cudaMemset(c->closure_tau, 0, 3 * c->N * sizeof(double)));
+        NSE_CUDA_TRY(cudaMalloc((void**)&c->closure_tau, c->N * sizeof(double)));
+        NSE_CUDA_TRY(cudaMemset(c->closure_tau, 0, c->N * sizeof(double)));
     }
     c->closure_net = net->n;
     c->closure_every_stage = every_stage != 0;
@@ -724,7 +823,7 @@ int nse2d_cnn_gradients(nse2d_cnn* c, const double* w, const double* psi, const 
     if (!c || !w || !psi || !u || !v || !tau) { set_error("nse2d_cnn_gradients: null argument"); return -1; }
     Cnn* n = c->n;
     if (batch_setup(n, idx, nb, s)) return -1;
-    const int rc = (cnn_forward_batch(n, pack_src(n, w, psi, u, v), s) || cnn_backward(n, tau, s)) ? -1 : 0;
+    const int rc = (cnn_forward_batch(n, pack_src(n, w, psi, u, v), nullptr, true, nullptr, s) || cnn_backward(n, tau, s)) ? -1 : 0;
     // slot 0 back to sample 0 for inference
     const int zero = 0;
     NSE_CUDA_TRY(cudaMemcpyAsync(n->idx, &zero, sizeof(int), cudaMemcpyHostToDevice, s));

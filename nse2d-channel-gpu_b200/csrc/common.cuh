@@ -158,7 +158,7 @@ struct Context {
     int maxuv_ctas = 0;            // resident CTAs of k_maxuv_dt (occupancy x SMs)
     // learned closure: the model evaluated before every stage and its output tau [Ny][Nx]
     struct Cnn* closure_net = nullptr;
-    double* closure_tau = nullptr;       // tau, then the u, v scratch of the model's inputs
+    double* closure_tau = nullptr;       // tau [Ny][Nx]
     bool closure_every_stage = true;     // false: tau of the step's first stage for all three
     // FP32-bulk variant (precision 32): base profiles (FP64) and FP32 fluctuations
     bool prec32 = false;

@@ -45,7 +45,8 @@ int band_rows_fwd(Context* c, const double* src, int row0, int nrows, cudaStream
 int band_rows_inv(Context* c, double* psi, double* w, bool thom, bool advance, cudaStream_t s);
 // learned closure (closure.cu)
 struct Cnn;
-int cnn_forward(Cnn* n, const double* w, const double* psi, const double* u, const double* v, double* tau, cudaStream_t s);
+int cnn_forward_psi(Cnn* n, const double* w, const double* psi, const double* a_node, double inv_dx, double inv_deta, double* tau,
+                    cudaStream_t s);
 bool cnn_matches(const Cnn* n, int Nx, int Ny);
 int thomas_launches(const Context* c);
 const char* thomas_kernel_name(const Context* c, int i);

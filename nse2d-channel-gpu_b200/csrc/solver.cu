@@ -548,10 +548,7 @@ static int closure_tau(Context* c, int stage, const double* w_in, const double**
     *tau = nullptr;
     if (!c->closure_net) return 0;
     if (stage == 1 || c->closure_every_stage) {
-        double* u = c->closure_tau + c->N;
-        double* v = c->closure_tau + 2 * c->N;
-        if (uv_from_psi(c, c->psi, u, v, s) || cnn_forward(c->closure_net, w_in, c->psi, u, v, c->closure_tau, s))
-            return -1;
+        if (cnn_forward_psi(c->closure_net, w_in, c->psi, c->rt.a_node, c->inv_dx, c->inv_deta, c->closure_tau, s)) return -1;
     }
     *tau = c->closure_tau;
     return 0;

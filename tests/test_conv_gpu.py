@@ -1,0 +1,35 @@
+"""The closure model's convolutions and weight gradients (csrc/conv_tc.cuh) at their edges, on a B200, against
+the CPU oracle: every width of the hidden layers, batches, pixel counts that are not multiples of the 128 and
+64 pixels of a tile (fewer pixels than one tile too), rows that are not powers of two, and fields of few rows,
+where most taps meet a wall. Bars as in test_closure_gpu.py: the output within 1e-2 of its largest magnitude,
+every gradient within 3e-2 in the relative L2 norm, the loss within 1e-3 (a hidden activation next to a BF16
+rounding boundary can round the other way)."""
+import numpy as np
+import pytest
+
+from conftest import load_oracle_module
+from test_closure_gpu import SCALES, _dev, _net, _rel, _sample
+
+pytestmark = pytest.mark.gpu
+
+co = load_oracle_module("closure_oracle")
+
+
+@pytest.mark.parametrize("Nx,Ny,H,idx", [(4, 5, 16, (0,)), (20, 9, 16, (1, 0)), (12, 7, 48, (2, 0, 3)), (34, 11, 48, (0,)),
+                                         (64, 33, 64, (3, 1)), (128, 5, 32, (0, 1, 2, 3)), (96, 40, 32, (2,))])
+def test_edges_match_the_oracle(nse, cuda, Nx, Ny, H, idx):
+    torch = cuda
+    net, y = _net(nse, Nx, Ny, H, 7, max_batch=len(idx) + 1)
+    S = [_sample(Ny, Nx, 30 + s) for s in range(4)]
+    out = torch.full((Ny, Nx), 7.0, dtype=torch.float64, device="cuda")
+    net.forward(*[_dev(torch, f) for f in S[1][:4]], out)
+    ref = co.predict(net.params(), *S[1][:4], y, SCALES, bf=True)
+    assert np.abs(out.cpu().numpy() - ref).max() <= 1e-2 * np.abs(ref).max()
+    stack = [_dev(torch, np.stack([smp[f] for smp in S])) for f in range(5)]
+    loss = net.gradients(*stack, idx=idx)
+    ref_loss, ref_grads = co.loss_and_grads(net.params(), [S[i] for i in idx], y, SCALES, bf=True)
+    assert abs(loss - ref_loss) <= 1e-3 * ref_loss, (loss, ref_loss)
+    for layer in range(4):
+        gw, gb = net.get_grads(layer)
+        assert _rel(gw, ref_grads[layer][0]) < 3e-2, (layer, _rel(gw, ref_grads[layer][0]))
+        assert _rel(gb, ref_grads[layer][1]) < 3e-2, (layer, _rel(gb, ref_grads[layer][1]))
