@@ -87,6 +87,7 @@ struct RowTables {
     double* w_node;     // trapezoid weights
     double* wt_node;    // deta / a_node on interior rows, 0 at walls
     double* frow;       // vorticity forcing f(y_j)
+    double* fx;         // its body force F0 sin(n pi (y_j + h) / (2 h))
     double* st_cj;      // stage stencil: a_j inv_dx inv_deta / 12 (the Arakawa factor a / (4 dx deta) / 3)
     double* st_ap;      // stage stencil: nu a_j a_{j+1/2} / deta^2
     double* st_am;      // stage stencil: nu a_j a_{j-1/2} / deta^2

@@ -29,13 +29,16 @@ struct DiagParams {
     RowTables rt;
     double* rows;            // [Ny][NSUM]
     int Nx, Ny;
-    double inv_dx, inv_deta, h, F0;
-    int nforce;
+    double inv_dx, inv_deta;
 };
 
+// One CTA per row. The 21 sums of a row are folded through shared memory, one thread per sum and warp adding
+// 32 lanes in the order of a shuffle tree (lane l + 16, + 8, ..): shuffling every sum across every warp was
+// 2500 warp instructions a row, more than the points of a row of 1024. That, and sin and cos of the forcing in
+// every thread, took 27 us at 1024x513.
 __global__ void __launch_bounds__(256) k_diag_rows(DiagParams p) {
     const int Nx = p.Nx, Ny = p.Ny;
-    __shared__ double red[NSUM][8];
+    __shared__ double red[NSUM * 8][33];                  // [sum, warp][lane]
     const double inv_dx2 = p.inv_dx * p.inv_dx, inv_deta2 = p.inv_deta * p.inv_deta;
     for (int j = blockIdx.x; j < Ny; j += gridDim.x) {
         double s[NSUM];
@@ -43,10 +46,7 @@ __global__ void __launch_bounds__(256) k_diag_rows(DiagParams p) {
         for (int q = 0; q < NSUM; ++q) s[q] = 0.0;
         const double wq = p.rt.w_node[j], a = p.rt.a_node[j], wt = p.rt.wt_node[j];
         const int ym = (j == 0 ? 0 : j - 1), yp = (j == Ny - 1 ? Ny - 1 : j + 1);
-        const double yy = p.rt.y[j];
-        const double argF = (double)p.nforce * kPiD * ((yy + p.h) / (2.0 * p.h));
-        const double Fx = p.F0 * sin(argF);                                          // diag.cu:359
-        const double fom = -p.F0 * ((double)p.nforce * kPiD / (2.0 * p.h)) * cos(argF);  // diag.cu:392-393
+        const double Fx = p.rt.fx[j], fom = p.rt.frow[j];                            // diag.cu:359,392-393
         const double* w = p.w;
         const double* psi = p.psi;
         for (int i = threadIdx.x; i < Nx; i += blockDim.x) {
@@ -111,57 +111,62 @@ __global__ void __launch_bounds__(256) k_diag_rows(DiagParams p) {
             if (j == Ny - 1) s[S_T2_PHI] += wc * p.rt.a_edge[Ny - 2] * (wc - w[(size_t)(Ny - 2) * Nx + i]) * p.inv_deta;
             if (p.rhs && !interior) s[S_WALL_WRHS] += wq * wc * p.rhs[c];           // main.cu:290-296
         }
-        // warp tree, then the 8 warps in order
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-        for (int q = 0; q < NSUM; ++q) {
-            double v = s[q];
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if (lane == 0) red[q][warp] = v;
+        for (int q = 0; q < NSUM; ++q) red[q * 8 + warp][lane] = s[q];
+        __syncthreads();
+        if (threadIdx.x < NSUM * 8) {
+            double v[32];
+            double* r = red[threadIdx.x];
+#pragma unroll
+            for (int l = 0; l < 32; ++l) v[l] = r[l];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int l = 0; l < o; ++l) v[l] += v[l + o];
+            r[0] = v[0];
         }
         __syncthreads();
-        if (threadIdx.x < NSUM) {
+        if (threadIdx.x < NSUM) {                          // the 8 warps in order
             double v = 0.0;
-            for (int k = 0; k < 8; ++k) v += red[threadIdx.x][k];
+            for (int k = 0; k < 8; ++k) v += red[threadIdx.x * 8 + k][0];
             p.rows[(size_t)j * NSUM + threadIdx.x] = v;
         }
         __syncthreads();
     }
 }
 
-// Sum the rows of each quantity in row order, compensated; one warp per quantity.
-__global__ void k_diag_final(const double* rows, int Ny, double* out) {
-    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (q >= NSUM) return;
+// Sum the rows of each quantity, compensated: a CTA per quantity, a thread per 64th row, then the threads in order.
+constexpr int DIAG_FT = 64;
+__global__ void __launch_bounds__(DIAG_FT) k_diag_final(const double* rows, int Ny, double* out) {
+    __shared__ double part[2][DIAG_FT];
+    const int q = blockIdx.x, t = threadIdx.x;
     double s = 0.0, cmp = 0.0;
-    for (int j = lane; j < Ny; j += 32) {
-        const double x = rows[(size_t)j * NSUM + q];
-        const double t = s + x;
-        cmp += (fabs(s) >= fabs(x)) ? (s - t) + x : (x - t) + s;
-        s = t;
+    auto add = [&](double x) {
+        const double u = s + x;
+        cmp += (fabs(s) >= fabs(x)) ? (s - u) + x : (x - u) + s;
+        s = u;
+    };
+#pragma unroll 4
+    for (int j = t; j < Ny; j += DIAG_FT) add(rows[(size_t)j * NSUM + q]);
+    part[0][t] = s;
+    part[1][t] = cmp;
+    __syncthreads();
+    if (t != 0) return;
+    for (int k = 1; k < DIAG_FT; ++k) {
+        add(part[0][k]);
+        cmp += part[1][k];
     }
-    __shared__ double part[NSUM][32];
-    part[q][lane] = s + cmp;
-    __syncwarp();
-    if (lane == 0) {
-        double S = 0.0, C = 0.0;
-        for (int k = 0; k < 32; ++k) {
-            const double x = part[q][k];
-            const double t = S + x;
-            C += (fabs(S) >= fabs(x)) ? (S - t) + x : (x - t) + S;
-            S = t;
-        }
-        out[q] = S + C;
-    }
+    out[q] = s + cmp;
 }
 
 int rhs_at_state(Context* c, const double* w, const double* psi, double* J, double* rhs, double tm, cudaStream_t s);
 
-static int diag_sums(Context* c, const double* rhs, const double* J, double* host_out, cudaStream_t s) {
+// The sums of the current state with its stored rhs, to the host (synchronous).
+static int read_sums(Context* c, const double* J, double* host_out, cudaStream_t s) {
     DiagParams p{};
-    p.psi = c->psi; p.w = c->w; p.rhs = rhs; p.J = J; p.rt = c->rt; p.rows = c->red_blocks;
-    p.Nx = c->Nx; p.Ny = c->Ny; p.inv_dx = c->inv_dx; p.inv_deta = c->inv_deta; p.h = c->cfg.h;
-    p.F0 = c->cfg.F0; p.nforce = c->cfg.nforce;
+    p.psi = c->psi; p.w = c->w; p.rhs = c->rhs; p.J = J; p.rt = c->rt; p.rows = c->red_blocks;
+    p.Nx = c->Nx; p.Ny = c->Ny; p.inv_dx = c->inv_dx; p.inv_deta = c->inv_deta;
     if ((size_t)c->Ny * NSUM > c->red_capacity) {
         set_error("diagnostics: reduction buffer too small (%zu < %zu)", c->red_capacity, (size_t)c->Ny * NSUM);
         return -1;
@@ -169,7 +174,7 @@ static int diag_sums(Context* c, const double* rhs, const double* J, double* hos
     const int grid = std::min(c->Ny, 8 * c->num_sms);
     k_diag_rows<<<grid, 256, 0, s>>>(p);
     NSE_CUDA_TRY(cudaGetLastError());
-    k_diag_final<<<1, 32 * NSUM, 0, s>>>(c->red_blocks, c->Ny, c->red_out);
+    k_diag_final<<<NSUM, DIAG_FT, 0, s>>>(c->red_blocks, c->Ny, c->red_out);
     NSE_CUDA_TRY(cudaGetLastError());
     NSE_CUDA_TRY(cudaMemcpyAsync(host_out, c->red_out, NSUM * sizeof(double), cudaMemcpyDeviceToHost, s));
     NSE_CUDA_TRY(cudaStreamSynchronize(s));
@@ -183,11 +188,12 @@ int diagnostics_row(Context* c, int t0_row, double* o, cudaStream_t s) {
     const double nan = std::numeric_limits<double>::quiet_NaN();
     if (launch_maxuv(c, c->psi, false, s)) return -1;
     NSE_CUDA_TRY(cudaMemcpyAsync(c->h_ctl, c->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
-    NSE_CUDA_TRY(cudaStreamSynchronize(s));
-    const double t = c->h_ctl->t;
-    if (t0_row && rhs_at_state(c, c->w, c->psi, nullptr, c->rhs, t, s)) return -1;
+    if (t0_row) {                                                // the rhs at the state's time
+        NSE_CUDA_TRY(cudaStreamSynchronize(s));
+        if (rhs_at_state(c, c->w, c->psi, nullptr, c->rhs, c->h_ctl->t, s)) return -1;
+    }
     double S[NSUM];
-    if (diag_sums(c, c->rhs, nullptr, S, s)) return -1;
+    if (read_sums(c, nullptr, S, s)) return -1;
     const double nu = c->nu, iA = c->invA_full, h = c->cfg.h, Nx = (double)c->Nx;
     const double mwb = S[S_WWY_BOT] / Nx, mwt = S[S_WWY_TOP] / Nx;
     const double mOb = S[S_MOB] / Nx, mOt = S[S_MOT] / Nx;
@@ -216,9 +222,9 @@ int diagnostics_row(Context* c, int t0_row, double* o, cudaStream_t s) {
         o[16] = o[4]; o[20] = 0.0; o[21] = 0.0; o[22] = 0.0;
         return 0;
     }
-    if (rhs_at_state(c, c->w, c->psi, c->J, c->rhs, t, s)) return -1;
+    if (rhs_at_state(c, c->w, c->psi, c->J, c->rhs, c->h_ctl->t, s)) return -1;
     double C[NSUM];
-    if (diag_sums(c, c->rhs, c->J, C, s)) return -1;
+    if (read_sums(c, c->J, C, s)) return -1;
     const double same = C[S_WRHS] * iA;
     o[16] = same;
     o[17] = same - C[S_WALL_WRHS] * iA;
@@ -363,18 +369,26 @@ int stats_read(Context* c, double* out5, double* T, cudaStream_t s) {
 
 // ---- 1-D energy spectra in x (src/diag.cuh:123-191, src/diag.cu:868-898) ----
 // E(k) += w_k / (Nx^2 Ny) sum_j |f-hat_j(k)|^2 for k = 0..Nx/2, w_k = 2 inside the half
-// spectrum and 1 at k = 0 and Nx/2, summed over the rows in row order (one thread per k).
-static __global__ void k_spectra_reduce(const cpx<double>* __restrict__ hat, int Ny, int Hp, int H, double norm,
-                                        double* __restrict__ acc) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= H) return;
-    const double wx = (k > 0 && k < H - 1) ? 2.0 : 1.0;
+// spectrum and 1 at k = 0 and Nx/2. A CTA takes 8 k (a 128-byte line of every row) and 64 row slices, folded in a
+// fixed order; one thread per k walking down all rows left five CTAs and one load in flight (79 us at 1024x513).
+constexpr int SPEC_K = 8, SPEC_S = 64;
+static __global__ void __launch_bounds__(SPEC_K * SPEC_S) k_spectra_reduce(const cpx<double>* __restrict__ hat, int Ny, int Hp, int H,
+                                                                          double norm, double* __restrict__ acc) {
+    __shared__ double red[SPEC_S][SPEC_K + 1];
+    const int kk = threadIdx.x % SPEC_K, sl = threadIdx.x / SPEC_K, k = blockIdx.x * SPEC_K + kk;    // k < Hp, a multiple of 16
     double sum = 0.0;
-    for (int j = 0; j < Ny; ++j) {
+#pragma unroll 4
+    for (int j = sl; j < Ny; j += SPEC_S) {
         const cpx<double> z = hat[(size_t)j * Hp + k];
         sum += (z.x * z.x + z.y * z.y);
     }
-    acc[k] += norm * wx * sum;
+    red[sl][kk] = sum;
+    __syncthreads();
+    for (int st = SPEC_S / 2; st > 0; st >>= 1) {
+        if (sl < st) red[sl][kk] += red[sl + st][kk];
+        __syncthreads();
+    }
+    if (sl == 0 && k < H) acc[k] += norm * ((k > 0 && k < H - 1) ? 2.0 : 1.0) * red[0][kk];
 }
 
 // One sample of E_u, E_v from device u, v [Ny][Nx] (16-byte aligned): the row transforms of the
@@ -386,10 +400,10 @@ int spectra_accumulate_uv(Context* c, const double* u, const double* v, cudaStre
         c->spec_samples = 0;
     }
     const double norm = 1.0 / ((double)c->Nx * (double)c->Nx * (double)c->Ny);
-    const int tb = 128, gb = (c->H + tb - 1) / tb;
+    const int gb = (c->H + SPEC_K - 1) / SPEC_K;
     for (int q = 0; q < 2; ++q) {
         if (launch_fft_all_rows(c, q == 0 ? u : v, s)) return -1;
-        k_spectra_reduce<<<gb, tb, 0, s>>>(c->hat, c->Ny, c->Hp, c->H, norm, c->spec_acc + (size_t)q * c->Hp);
+        k_spectra_reduce<<<gb, SPEC_K * SPEC_S, 0, s>>>(c->hat, c->Ny, c->Hp, c->H, norm, c->spec_acc + (size_t)q * c->Hp);
         NSE_CUDA_TRY(cudaGetLastError());
     }
     c->spec_samples += 1;

@@ -172,13 +172,15 @@ __global__ void k_setup_rows(RowTables rt, int Ny, double inv_deta2, double deta
         rt.asub[j] = 0.0; rt.csup[j] = 0.0; rt.inv_csup[j] = 0.0; rt.wt_node[j] = 0.0;
         rt.st_cj[j] = 0.0; rt.st_ap[j] = 0.0; rt.st_am[j] = 0.0;
     }
-    double f = 0.0;
+    double f = 0.0, fx = 0.0;
     if (F0 != 0.0) {
         const double yy = rt.y[j];
         const double arg = (double)nforce * kPiD * ((yy + h) / (2.0 * h));
         f = -F0 * ((double)nforce * kPiD / (2.0 * h)) * cos(arg);
+        fx = F0 * sin(arg);
     }
     rt.frow[j] = f;
+    rt.fx[j] = fx;
     if (rt.mms_g) {
         const double theta = mms_c * (rt.y[j] + h);
         const double two_th = 2.0 * theta;
@@ -308,7 +310,7 @@ int context_create(const Config& cfg, Context** out) {
     auto fail = [&]() { context_destroy(c); return -1; };
     RowTables& rt = c->rt;
     if (dalloc(&rt.y, Ny) || dalloc(&rt.a_node, Ny) || dalloc(&rt.a_edge, Ny) || dalloc(&rt.dy_edge, Ny) ||
-        dalloc(&rt.w_node, Ny) || dalloc(&rt.wt_node, Ny) || dalloc(&rt.frow, Ny) || dalloc(&rt.st_cj, Ny) ||
+        dalloc(&rt.w_node, Ny) || dalloc(&rt.wt_node, Ny) || dalloc(&rt.frow, Ny) || dalloc(&rt.fx, Ny) || dalloc(&rt.st_cj, Ny) ||
         dalloc(&rt.st_ap, Ny) || dalloc(&rt.st_am, Ny) || dalloc(&rt.asub, Ny) ||
         dalloc(&rt.csup, Ny) || dalloc(&rt.inv_csup, Ny))
         return fail();
@@ -496,7 +498,7 @@ int context_create(const Config& cfg, Context** out) {
 void context_destroy(Context* c) {
     if (!c) return;
     RowTables& rt = c->rt;
-    for (double* p : {rt.y, rt.a_node, rt.a_edge, rt.dy_edge, rt.w_node, rt.wt_node, rt.frow, rt.st_cj, rt.st_ap, rt.st_am, rt.asub, rt.csup,
+    for (double* p : {rt.y, rt.a_node, rt.a_edge, rt.dy_edge, rt.w_node, rt.wt_node, rt.frow, rt.fx, rt.st_cj, rt.st_ap, rt.st_am, rt.asub, rt.csup,
                       rt.inv_csup, rt.mms_g, rt.mms_gpp, rt.mms_sin2, rt.mms_sk, rt.mms_s2k, c->w, c->w1, c->w2,
                       c->psi, c->rhs, c->J, c->cp, c->red_blocks, c->red_out})
         if (p) cudaFree(p);
