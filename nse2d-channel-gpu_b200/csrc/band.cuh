@@ -22,15 +22,16 @@
 //
 // psi-hat and omega-hat are different buffers, because a CTA reads halo rows of psi-hat while its
 // neighbours write omega-hat. The per-point arithmetic is the stage kernels' (stage_rhs_interior,
-// stage32_rhs_interior) and the transforms are the plan of fft_rows.cuh with written-out
-// multiply-adds: every split of the work gives the same bits.
+// stage32_rhs_interior) and the transforms (band_fft.cuh) write their multiply-adds out: every split of the
+// work gives the same bits.
 #pragma once
+#include "band_fft.cuh"
 #include "bulk32.cuh"
 
 namespace nse2d {
 
 template <int M> struct Band {
-    static constexpr int R0 = p16_plan<M>::R(0);
+    static constexpr int R0 = band_plan<M>::R(0);
     static constexpr int NB0 = M / R0;                       // pass-0 butterflies of a row
     static constexpr int TPR = M <= 128 ? 32 : 64;           // threads of a row group
     static constexpr int ROW = ip_size(M);                   // elements of a row buffer
@@ -41,7 +42,7 @@ template <int M> struct Band {
 };
 // Shared memory: the twiddles (pass tables, then W_2M^k, k <= M / 2), the row constants, the row buffers,
 // the omega rows, omega^n and omega^(s+1) of the band.
-template <int M> __host__ __device__ constexpr int band_ntw() { return p16_plan<M>::off(p16_plan<M>::P); }
+template <int M> __host__ __device__ constexpr int band_ntw() { return band_plan<M>::off(band_plan<M>::P); }
 template <int M> __host__ __device__ constexpr int band_ntab() { return band_ntw<M>() + M / 2 + 2; }
 constexpr int BAND_RC = 10;                                  // row constants kept per row (RC32_N in FP32)
 template <typename T, int M> __host__ __device__ constexpr size_t band_head_bytes(int R) {
@@ -86,6 +87,16 @@ template <int TPR> __device__ __forceinline__ void row_sync(int group) {
 __device__ __forceinline__ void cp_async_cpx(cpx<double>* d, const cpx<double>* g) { cp_async16(d, g); }
 __device__ __forceinline__ void cp_async_cpx(cpx<float>* d, const cpx<float>* g) { cp_async8(d, g); }
 
+// loads from L2, for what other CTAs of the same launch wrote
+__device__ __forceinline__ cpx<double> ldcg_cpx(const cpx<double>* q) {
+    const double2 v = __ldcg(reinterpret_cast<const double2*>(q));
+    return {v.x, v.y};
+}
+__device__ __forceinline__ cpx<float> ldcg_cpx(const cpx<float>* q) {
+    const float2 v = __ldcg(reinterpret_cast<const float2*>(q));
+    return {v.x, v.y};
+}
+
 // The twiddles to shared memory (no kernel writes them, so this may precede the wait for the previous
 // kernel): every pass of every row reads them, and a table read from global memory would wait on L2
 // once per pass and CTA.
@@ -97,14 +108,14 @@ template <typename T, int M> __device__ __forceinline__ void band_load_tables(cp
 // Passes Q .. P-1 by a row group; the last pass hands its outputs to out(position, value).
 template <typename T, int M, int Q, bool INV, typename Out>
 __device__ __forceinline__ void band_passes(cpx<T>* buf, const SmemTw<T>& tw, int t, int group, Out out) {
-    constexpr int TPR = Band<M>::TPR, R = p16_plan<M>::R(Q), LP = p16_plan<M>::LP(Q), NB = M / R;
+    constexpr int TPR = Band<M>::TPR, R = band_plan<M>::R(Q), LP = band_plan<M>::LP(Q), NB = M / R;
 #pragma unroll 1
     for (int b0 = 0; b0 < NB; b0 += TPR) {
         const int b = b0 + t;
         if (NB % TPR != 0 && b >= NB) break;
         cpx<T> v[R];
-        const int base = p16_bfly<T, M, Q, INV>(buf, tw, b, v);
-        if constexpr (Q == p16_plan<M>::P - 1) {
+        const int base = plan_bfly<T, band_plan<M>, Q, INV>(buf, tw, b, v);
+        if constexpr (Q == band_plan<M>::P - 1) {
 #pragma unroll
             for (int r = 0; r < R; ++r) out(base + r * LP, v[r]);
         } else {
@@ -113,7 +124,7 @@ __device__ __forceinline__ void band_passes(cpx<T>* buf, const SmemTw<T>& tw, in
         }
     }
     row_sync<TPR>(group);
-    if constexpr (Q < p16_plan<M>::P - 1) band_passes<T, M, Q + 1, INV>(buf, tw, t, group, out);
+    if constexpr (Q < band_plan<M>::P - 1) band_passes<T, M, Q + 1, INV>(buf, tw, t, group, out);
 }
 
 // Inverse transform of one spectral row X into out(n, z_n) (z_n = x_2n + i x_2n+1, times 2M), through buf:
@@ -122,13 +133,13 @@ __device__ __forceinline__ void band_passes(cpx<T>* buf, const SmemTw<T>& tw, in
 template <typename T, int M> struct BandSpec {
     static constexpr bool PRE = Band<M>::R0 <= 8;
     cpx<T> a[PRE ? Band<M>::R0 : 1], c[PRE ? Band<M>::R0 : 1];
-    __device__ __forceinline__ void load(const cpx<T>* __restrict__ X, int t) {
+    template <bool CG = false> __device__ __forceinline__ void load(const cpx<T>* X, int t) {
         if constexpr (PRE) {
             if (t < Band<M>::NB0) {
 #pragma unroll
                 for (int r = 0; r < Band<M>::R0; ++r) {
-                    a[r] = ldtw(X, t + Band<M>::NB0 * r);
-                    c[r] = ldtw(X, M - t - Band<M>::NB0 * r);
+                    a[r] = CG ? ldcg_cpx(X + t + Band<M>::NB0 * r) : ldtw(X, t + Band<M>::NB0 * r);
+                    c[r] = CG ? ldcg_cpx(X + M - t - Band<M>::NB0 * r) : ldtw(X, M - t - Band<M>::NB0 * r);
                 }
             }
         }
@@ -149,11 +160,11 @@ __device__ __forceinline__ void band_inverse(const BandSpec<T, M>& sp, const cpx
             else { a = ldtw(X, n); c = ldtw(X, M - n); }
             const cpx<T> sm = {a.x + c.x, a.y - c.y};
             const cpx<T> df = {a.x - c.x, a.y + c.y};
-            const cpx<T> wn = (r == 0) ? wt : cmul(wt, w32<T>(r * (16 / R0)));
-            v[r] = cadd(sm, mul_pi(cmulc(df, wn)));
+            const cpx<T> wn = (r == 0) ? wt : fmul_c(wt, w32<T>(r * (16 / R0)));
+            v[r] = cadd(sm, mul_pi(fmul_cc(df, wn)));
         }
-        dftR<T, R0, true>(v);
-        const int p0 = dit16_pos<M>(t);
+        fdftR<T, R0, true>(v);
+        const int p0 = dit_pos<band_plan<M>>(t);
 #pragma unroll
         for (int q = 0; q < R0; ++q) buf[ip_idx<M>(p0 + q)] = v[q];
     }
@@ -168,8 +179,8 @@ __device__ __forceinline__ void band_forward(cpx<T> (&v)[Band<M>::R0], cpx<T>* b
                                              cpx<T>* __restrict__ dst) {
     constexpr int NB0 = Band<M>::NB0, TPR = Band<M>::TPR, R0 = Band<M>::R0;
     if (NB0 >= TPR || t < NB0) {
-        dftR<T, R0, false>(v);
-        const int p0 = dit16_pos<M>(t);
+        fdftR<T, R0, false>(v);
+        const int p0 = dit_pos<band_plan<M>>(t);
 #pragma unroll
         for (int q = 0; q < R0; ++q) buf[ip_idx<M>(p0 + q)] = v[q];
     }
@@ -184,10 +195,10 @@ __device__ __forceinline__ void band_forward(cpx<T> (&v)[Band<M>::R0], cpx<T>* b
         const cpx<T> b = buf[ip_idx<M>(k == 0 ? 0 : M - k)];
         const cpx<T> sm = {(T)0.5 * (a.x + b.x), (T)0.5 * (a.y - b.y)};
         const cpx<T> df = {a.x - b.x, a.y + b.y};
-        dst[k] = cadd(sm, cmul(wk, mul_mi(df)));
+        dst[k] = cadd(sm, fmul_c(wk, mul_mi(df)));
         if (k < M / 2) {
             const cpx<T> wm = {-wk.x, wk.y};
-            dst[M - k] = cadd(cpx<T>{sm.x, -sm.y}, cmul(wm, cpx<T>{df.y, df.x}));
+            dst[M - k] = cadd(cpx<T>{sm.x, -sm.y}, fmul_c(wm, cpx<T>{df.y, df.x}));
         }
     }
 }
@@ -317,146 +328,190 @@ __device__ __forceinline__ cpx<T> band_pair(const BandParams<T>& p, const Row& k
     return {w[0], w[1]};
 }
 
-// The stage and the forward transform of a band of rows, with (INV) the inverse transform and the
-// wall closure before it. Grid: an even split of the interior rows; blockDim = (R + 2) TPR for bands
-// of at most R rows.
-template <typename T, int M, bool INV>
-static __global__ void __launch_bounds__(Band<M>::MAXT, 1) k_band(BandParams<T> p) {
+// A CTA's band of rows and its shared memory: the pieces below are the row work of one CTA, by all of its threads.
+template <typename T, int M> struct BandCta {
     using B = Band<M>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int G = (int)blockDim.x / B::TPR, R = G - 2;
-    cpx<T>* tab = reinterpret_cast<cpx<T>*>(smem_raw);
-    T* rc = reinterpret_cast<T*>(tab + band_ntab<M>());      // constants of rows j0 - 1 .. j1
-    cpx<T>* rows = reinterpret_cast<cpx<T>*>(smem_raw + band_head_bytes<T, M>(R));
-    const SmemTw<T> tw{tab}, wN{tab + band_ntw<M>()};
-    const int t = (int)threadIdx.x % B::TPR, group = (int)threadIdx.x / B::TPR;
-    const int Ni = p.Ny - 2;
-    const int j0 = 1 + (int)(((long long)blockIdx.x * Ni) / gridDim.x);
-    const int j1 = 1 + (int)(((long long)(blockIdx.x + 1) * Ni) / gridDim.x);
-    const int nr = j1 - j0;                                   // rows of the band; row buffers 0 .. nr + 1
-    cpx<T>* ws = rows + (size_t)G * B::ROW;                   // omega rows j0 - 1 .. j1,
-    cpx<T>* wns = ws + (size_t)G * M;                         // omega^n of the band's rows
-    cpx<T>* zs = wns + (size_t)R * M;                         // and their omega^(s+1)
-    const bool bot = (j0 == 1), top = (j1 == p.Ny - 1);
-    // tables first: they do not depend on the kernel before this one
-    band_load_tables<T, M>(tab, p);
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    band_load_rows(rc, p, j0 - 1, nr + 2);
-    pdl_begin();
-    const T dt = (T)p.ctl->dt;
-    const cpx<T>* w_in = reinterpret_cast<const cpx<T>*>(p.w_in);
-    const bool rowed = group < nr + 2;
-    const int jr = j0 - 1 + group;                            // the group's psi row
-    const bool wallrow = jr == 0 || jr == p.Ny - 1;
-    cpx<T>* buf = rows + (size_t)group * B::ROW;
-    BandSpec<T, M> sp;
-    if (INV && rowed && !wallrow) sp.load(p.hat_in + (size_t)jr * p.Hp, t);
-    if (rowed) {
-        // the rows that the stage reads, in flight while psi is transformed (with INV the wall rows of
-        // omega are set below)
-        if constexpr (!INV) {
-            const cpx<T>* src = reinterpret_cast<const cpx<T>*>(p.psi_in) + (size_t)jr * M;
-            for (int n = t; n < M; n += B::TPR) cp_async_cpx(buf + ip_idx<M>(n), src + n);
-        }
+    cpx<T> *tab, *rows, *ws, *wns, *zs;      // tables, psi rows j0 - 1 .. j1, omega rows, omega^n and omega^(s+1) of the band
+    T* rc;                                   // row constants of rows j0 - 1 .. j1
+    SmemTw<T> tw, wN;
+    int t, group, j0, nr;                    // thread of a row group; rows [j0, j0 + nr) of the band
+    bool bot, top;                           // the band lies at a wall
+
+    // R: most rows of a band (the row groups 0 .. R + 1 take the rows j0 - 1 .. j1)
+    __device__ __forceinline__ BandCta(const BandParams<T>& p, unsigned char* smem, int R) {
+        tab = reinterpret_cast<cpx<T>*>(smem);
+        rc = reinterpret_cast<T*>(tab + band_ntab<M>());
+        rows = reinterpret_cast<cpx<T>*>(smem + band_head_bytes<T, M>(R));
+        ws = rows + (size_t)(R + 2) * B::ROW;
+        wns = ws + (size_t)(R + 2) * M;
+        zs = wns + (size_t)R * M;
+        tw.p = tab;
+        wN.p = tab + band_ntw<M>();
+        t = (int)threadIdx.x % B::TPR;
+        group = (int)threadIdx.x / B::TPR;
+        const int Ni = p.Ny - 2;
+        j0 = 1 + (int)(((long long)blockIdx.x * Ni) / gridDim.x);
+        const int j1 = 1 + (int)(((long long)(blockIdx.x + 1) * Ni) / gridDim.x);
+        nr = j1 - j0;
+        bot = (j0 == 1);
+        top = (j1 == p.Ny - 1);
+    }
+    __device__ __forceinline__ bool rowed() const { return group < nr + 2; }
+    __device__ __forceinline__ int row() const { return j0 - 1 + group; }                // the group's psi row
+    __device__ __forceinline__ bool wallrow() const { return (bot && group == 0) || (top && group == nr + 1); }
+    __device__ __forceinline__ cpx<T>* buf() const { return rows + (size_t)group * B::ROW; }
+
+    // tables and row constants, which no step kernel writes (a commit group of its own)
+    __device__ __forceinline__ void load_consts(const BandParams<T>& p) {
+        band_load_tables<T, M>(tab, p);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        band_load_rows(rc, p, j0 - 1, nr + 2);
+    }
+    // psi rows j0 - 1 .. j1 (cp.async)
+    __device__ __forceinline__ void load_psi(const T* psi) {
+        if (!rowed()) return;
+        const cpx<T>* src = reinterpret_cast<const cpx<T>*>(psi) + (size_t)row() * M;
+        for (int n = t; n < M; n += B::TPR) cp_async_cpx(buf() + ip_idx<M>(n), src + n);
+    }
+    // omega rows j0 - 1 .. j1, without the wall rows when the closure sets them (cp.async)
+    __device__ __forceinline__ void load_omega(const T* w, bool walls) {
         constexpr int CH = M * (int)sizeof(cpx<T>) / 16, CE = 16 / (int)sizeof(cpx<T>);
-        if (!(INV && wallrow))
-            for (int c = t; c < CH; c += B::TPR) cp_async16(ws + (size_t)group * M + CE * c, w_in + (size_t)jr * M + CE * c);
-        if (p.stage > 1 && group >= 1 && group <= nr) {
-            const cpx<T>* src = reinterpret_cast<const cpx<T>*>(p.w_n) + (size_t)jr * M;
-            for (int c = t; c < CH; c += B::TPR) cp_async16(wns + (size_t)(group - 1) * M + CE * c, src + CE * c);
-        }
+        if (!rowed() || (!walls && wallrow())) return;
+        const cpx<T>* src = reinterpret_cast<const cpx<T>*>(w) + (size_t)row() * M;
+        for (int c = t; c < CH; c += B::TPR) cp_async16(ws + (size_t)group * M + CE * c, src + CE * c);
     }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    if constexpr (INV) {
-        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-        __syncthreads();                                      // the tables
-        if (rowed && wallrow) {
-            const T v = (T)(jr == 0 ? p.psi_bot : p.psi_top);
-            for (int n = t; n < M; n += B::TPR) buf[ip_idx<M>(n)] = cpx<T>{v, v};
-        } else if (rowed) {
+    // omega^n of the band's rows (cp.async)
+    __device__ __forceinline__ void load_omega_n(const T* w) {
+        constexpr int CH = M * (int)sizeof(cpx<T>) / 16, CE = 16 / (int)sizeof(cpx<T>);
+        if (group < 1 || group > nr) return;
+        const cpx<T>* src = reinterpret_cast<const cpx<T>*>(w) + (size_t)row() * M;
+        for (int c = t; c < CH; c += B::TPR) cp_async16(wns + (size_t)(group - 1) * M + CE * c, src + CE * c);
+    }
+    // psi rows j0 - 1 .. j1 from psi-hat (sp: the group's loads in flight)
+    __device__ __forceinline__ void inverse(const BandParams<T>& p, const BandSpec<T, M>& sp) {
+        if (!rowed()) return;
+        cpx<T>* b = buf();
+        if (wallrow()) {
+            const T v = (T)(group == 0 ? p.psi_bot : p.psi_top);
+            for (int n = t; n < M; n += B::TPR) b[ip_idx<M>(n)] = cpx<T>{v, v};
+        } else {
             constexpr T scale = (T)0.5 / (T)M;                // the merge forms 2 Z_n
-            band_inverse<T, M>(sp, p.hat_in + (size_t)jr * p.Hp, buf, tw, wN, t, group,
-                               [&](int n, const cpx<T>& z) { buf[ip_idx<M>(n)] = cpx<T>{z.x * scale, z.y * scale}; });
+            band_inverse<T, M>(sp, p.hat_in + (size_t)row() * p.Hp, b, tw, wN, t, group,
+                               [&](int n, const cpx<T>& z) { b[ip_idx<M>(n)] = cpx<T>{z.x * scale, z.y * scale}; });
         }
     }
-    cp_async_wait_all();
-    __syncthreads();
-    if constexpr (INV) {
-        if (bot || top) {
-            if (bot) band_wall_row<T, M>(p, false, rows + B::ROW, rows + 2 * (size_t)B::ROW, p.w_in, ws);
-            if (top) band_wall_row<T, M>(p, true, rows + (size_t)nr * B::ROW, rows + (size_t)(nr - 1) * B::ROW, p.w_in,
-                                         ws + (size_t)(nr + 1) * M);
-            __syncthreads();
-        }
+    // wall rows of w (and of the omega rows) from the psi rows; between barriers
+    __device__ __forceinline__ void walls(const BandParams<T>& p, T* w) {
+        if (bot) band_wall_row<T, M>(p, false, rows + B::ROW, rows + 2 * (size_t)B::ROW, w, ws);
+        if (top) band_wall_row<T, M>(p, true, rows + (size_t)nr * B::ROW, rows + (size_t)(nr - 1) * B::ROW, w, ws + (size_t)(nr + 1) * M);
     }
-    if (p.rhs_out && (bot || top)) {
-        // the walls' rhs is f - r omega (their omega is the closure's)
-        for (int side = 0; side < 2; ++side) {
-            if (!(side ? top : bot)) continue;
-            const int j = side ? p.Ny - 1 : 0, q = side ? nr + 1 : 0;
-            const auto k = band_row(rc + q * BAND_RC);
-            for (int n = threadIdx.x; n < M; n += blockDim.x) {
-                const cpx<T> wc = ws[(size_t)q * M + n];
-                reinterpret_cast<cpx<T>*>(p.rhs_out)[(size_t)j * M + n] =
-                    cpx<T>{fma_t(-(T)p.lin_drag, wc.x, k.f), fma_t(-(T)p.lin_drag, wc.y, k.f)};
+    // omega^(s+1) of the band into zs and w_out. save_n: omega^(s) of the band's rows into wns (stage 1, whose
+    // omega^(s) is omega^n)
+    __device__ __forceinline__ void stage(const BandParams<T>& p, T dt, bool save_n) {
+        if (p.rhs_out && (bot || top)) {
+            // the walls' rhs is f - r omega (their omega is the closure's)
+            for (int side = 0; side < 2; ++side) {
+                if (!(side ? top : bot)) continue;
+                const int j = side ? p.Ny - 1 : 0, q = side ? nr + 1 : 0;
+                const auto k = band_row(rc + q * BAND_RC);
+                for (int n = threadIdx.x; n < M; n += blockDim.x) {
+                    const cpx<T> wc = ws[(size_t)q * M + n];
+                    reinterpret_cast<cpx<T>*>(p.rhs_out)[(size_t)j * M + n] =
+                        cpx<T>{fma_t(-(T)p.lin_drag, wc.x, k.f), fma_t(-(T)p.lin_drag, wc.y, k.f)};
+                }
             }
         }
-    }
-    // the stage: an item is a pair n and the rows [qa, qb) of the band (all of them, or half where that
-    // evens out the threads); a thread walks down its rows with j-1, j, j+1 of its window in registers
-    cpx<T>* w_out = reinterpret_cast<cpx<T>*>(p.w_out);
-    const T mdrag = -(T)p.lin_drag, nu_dx2 = (T)p.nu_dx2;
-    const int NT = (int)blockDim.x;
-    const int half = (nr + 1) / 2;
-    const bool split = ((2 * M + NT - 1) / NT) * half < ((M + NT - 1) / NT) * nr;
-    for (int item = threadIdx.x; item < (split ? 2 * M : M); item += NT) {
-        const int n = item & (M - 1);
-        const int qa = item < M ? 0 : half, qb = (split && item < M) ? half : nr;
-        const cpx<T>* pr = rows + (size_t)qa * B::ROW;
-        const cpx<T>* orow = ws + (size_t)qa * M;
-        const cpx<T>* w_n = wns + (size_t)qa * M + n;
-        BandWin<T> win[3];
-        band_window_row<T, M>(pr, orow, n, win[0]);
-        band_window_row<T, M>(pr + B::ROW, orow + M, n, win[1]);
-        band_window_row<T, M>(pr + 2 * B::ROW, orow + 2 * M, n, win[2]);
-        band_diffs(win[0]);
-        band_diffs(win[1]);
-        cpx<T> wn = {0, 0};
-        if (p.stage > 1) wn = *w_n;
-        // unrolled, so that the window rotates by name instead of by moves; the row after next and the next
-        // omega^n are loaded before this row's arithmetic
+        // an item is a pair n and the rows [qa, qb) of the band (all of them, or half where that evens out the
+        // threads); a thread walks down its rows with j-1, j, j+1 of its window in registers
+        cpx<T>* w_out = reinterpret_cast<cpx<T>*>(p.w_out);
+        const T mdrag = -(T)p.lin_drag, nu_dx2 = (T)p.nu_dx2;
+        const int NT = (int)blockDim.x;
+        const int half = (nr + 1) / 2;
+        const bool split = ((2 * M + NT - 1) / NT) * half < ((M + NT - 1) / NT) * nr;
+        for (int item = threadIdx.x; item < (split ? 2 * M : M); item += NT) {
+            const int n = item & (M - 1);
+            const int qa = item < M ? 0 : half, qb = (split && item < M) ? half : nr;
+            const cpx<T>* pr = rows + (size_t)qa * B::ROW;
+            const cpx<T>* orow = ws + (size_t)qa * M;
+            cpx<T>* w_n = wns + (size_t)qa * M + n;
+            BandWin<T> win[3];
+            band_window_row<T, M>(pr, orow, n, win[0]);
+            band_window_row<T, M>(pr + B::ROW, orow + M, n, win[1]);
+            band_window_row<T, M>(pr + 2 * B::ROW, orow + 2 * M, n, win[2]);
+            band_diffs(win[0]);
+            band_diffs(win[1]);
+            cpx<T> wn = {0, 0};
+            if (p.stage > 1) wn = *w_n;
+            // unrolled, so that the window rotates by name instead of by moves; the row after next and the next
+            // omega^n are loaded before this row's arithmetic
 #pragma unroll
-        for (int u = 0; u < B::RMAX; ++u) {
-            const int q = qa + u;
-            if (q >= qb) break;
-            BandWin<T>&wa = win[u % 3], &wb = win[(u + 1) % 3], &wc = win[(u + 2) % 3];
-            band_diffs(wc);
-            const cpx<T> wnq = wn;
-            BandWin<T> nx;
-            const bool more = q + 1 < qb;
-            if (more) {
-                band_window_row<T, M>(pr + (u + 3) * B::ROW, orow + (u + 3) * M, n, nx);
-                if (p.stage > 1) wn = w_n[(u + 1) * M];
+            for (int u = 0; u < B::RMAX; ++u) {
+                const int q = qa + u;
+                if (q >= qb) break;
+                BandWin<T>&wa = win[u % 3], &wb = win[(u + 1) % 3], &wc = win[(u + 2) % 3];
+                band_diffs(wc);
+                const cpx<T> wnq = wn;
+                BandWin<T> nx;
+                const bool more = q + 1 < qb;
+                if (more) {
+                    band_window_row<T, M>(pr + (u + 3) * B::ROW, orow + (u + 3) * M, n, nx);
+                    if (p.stage > 1) wn = w_n[(u + 1) * M];
+                }
+                const int j = j0 + q;
+                const cpx<T> z = band_pair<T, M>(p, band_row(rc + (q + 1) * BAND_RC), dt, mdrag, nu_dx2, j, n, wnq, wa, wb, wc);
+                w_out[j * M + n] = z;
+                zs[q * M + n] = z;
+                if (save_n) w_n[u * M] = cpx<T>{wb.o[1], wb.o[2]};
+                if (more) wa = nx;
             }
-            const int j = j0 + q;
-            const cpx<T> z = band_pair<T, M>(p, band_row(rc + (q + 1) * BAND_RC), dt, mdrag, nu_dx2, j, n, wnq, wa, wb, wc);
-            w_out[j * M + n] = z;
-            zs[q * M + n] = z;
-            if (more) wa = nx;
         }
     }
-    __syncthreads();                                          // every window is read: the row buffers are free
-    // group g transforms row j0 + g in row buffer g + 1
-    if (group < nr) {
-        const int j = j0 + group;
+    // forward transform of the band's omega^(s+1), after a barrier: group g transforms row j0 + g in row buffer
+    // g + 1, which ends the psi rows
+    __device__ __forceinline__ void forward(const BandParams<T>& p) {
+        if (group >= nr) return;
         const cpx<T>* src = zs + (size_t)group * M;
         cpx<T> z[B::R0];
         if (B::NB0 >= B::TPR || t < B::NB0) {
 #pragma unroll
             for (int r = 0; r < B::R0; ++r) z[r] = src[t + B::NB0 * r];
         }
-        band_forward<T, M>(z, buf + B::ROW, tw, wN, t, group, p.hat_out + (size_t)j * p.Hp);
+        band_forward<T, M>(z, buf() + B::ROW, tw, wN, t, group, p.hat_out + (size_t)(j0 + group) * p.Hp);
     }
+};
+
+// The stage and the forward transform of a band of rows, with (INV) the inverse transform and the
+// wall closure before it. Grid: an even split of the interior rows; blockDim = (R + 2) TPR for bands
+// of at most R rows.
+template <typename T, int M, bool INV>
+static __global__ void __launch_bounds__(Band<M>::MAXT, 1) k_band(BandParams<T> p) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    BandCta<T, M> c(p, smem_raw, (int)blockDim.x / Band<M>::TPR - 2);
+    c.load_consts(p);                                         // before the wait for the previous kernel
+    pdl_begin();
+    const T dt = (T)p.ctl->dt;
+    BandSpec<T, M> sp;
+    if (INV && c.rowed() && !c.wallrow()) sp.load(p.hat_in + (size_t)c.row() * p.Hp, c.t);
+    if constexpr (!INV) c.load_psi(p.psi_in);
+    c.load_omega(p.w_in, !INV);                               // in flight while psi is transformed
+    if (p.stage > 1) c.load_omega_n(p.w_n);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    if constexpr (INV) {
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        __syncthreads();                                      // the tables
+        c.inverse(p, sp);
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    if constexpr (INV) {
+        if (c.bot || c.top) {
+            c.walls(p, p.w_in);
+            __syncthreads();
+        }
+    }
+    c.stage(p, dt, false);
+    __syncthreads();
+    c.forward(p);
 }
 
 // Forward transforms of rows row0 .. row0 + nrows - 1, ROWS_G rows per CTA.

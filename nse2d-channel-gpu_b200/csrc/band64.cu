@@ -16,7 +16,7 @@ static int band_R(const Context* c, int rmax) { return std::max(1, std::min(rmax
 
 static BandParams<double> band_params(Context* c) {
     BandParams<double> p{};
-    p.hat_in = c->hat2 ? c->hat2 : c->hat; p.hat_out = c->hat; p.psi_in = c->psi; p.tw = c->tw; p.wN = c->wN; p.rt = c->rt; p.ctl = c->ctl;
+    p.hat_in = c->hat2 ? c->hat2 : c->hat; p.hat_out = c->hat; p.psi_in = c->psi; p.tw = c->tw_band; p.wN = c->wN; p.rt = c->rt; p.ctl = c->ctl;
     p.Nx = c->Nx; p.Ny = c->Ny; p.Hp = c->Hp; p.free_slip = c->cfg.free_slip;
     p.nu_dx2 = c->nu * c->inv_dx2; p.lin_drag = c->cfg.lin_drag;
     p.psi_bot = c->psi_bot; p.psi_top = c->psi_top;

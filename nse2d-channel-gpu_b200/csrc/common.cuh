@@ -125,6 +125,7 @@ struct Context {
     bool plain_step = false;       // a step of separate transforms and stages (nse2d_step_profiled times them apart)
     double* cp = nullptr;          // elimination table [Ni][Hp]
     cpx<double>* tw = nullptr;     // per-pass twiddle pairs of the Nx/2-point transform
+    cpx<double>* tw_band = nullptr;  // the same for the row-band kernels' plan
     cpx<double>* wN = nullptr;     // M+1 twiddles e^{-2 pi i k/Nx}
     // reductions
     double* red_blocks = nullptr;  // per-block partials (max and diagnostics)

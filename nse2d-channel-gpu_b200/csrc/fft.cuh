@@ -11,7 +11,6 @@
 // Every function here is __host__ __device__, so the same butterflies can be stepped on the
 // CPU to check index arithmetic and numerics before they run on a GPU.
 #pragma once
-#include <cmath>
 
 #ifdef __CUDACC__
 #define NSE_HD __host__ __device__ __forceinline__
@@ -25,11 +24,8 @@ namespace nse2d {
 // (FP32) access to shared or global memory.
 template <typename T> struct alignas(2 * sizeof(T)) cpx { T x, y; };
 
-// The multiply-adds are written out (and every other product here is exact or stands alone), so that
-// a transform gives the same bits in every kernel it is compiled into.
-template <typename T> NSE_HD T fmadd(T a, T b, T c) { return ::fma(a, b, c); }
-template <typename T> NSE_HD cpx<T> cmul(cpx<T> a, cpx<T> b) { return {fmadd(a.x, b.x, -(a.y * b.y)), fmadd(a.x, b.y, a.y * b.x)}; }
-template <typename T> NSE_HD cpx<T> cmulc(cpx<T> a, cpx<T> b) { return {fmadd(a.x, b.x, a.y * b.y), fmadd(a.y, b.x, -(a.x * b.y))}; }  // a * conj(b)
+template <typename T> NSE_HD cpx<T> cmul(cpx<T> a, cpx<T> b) { return {a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x}; }
+template <typename T> NSE_HD cpx<T> cmulc(cpx<T> a, cpx<T> b) { return {a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y}; }  // a * conj(b)
 template <typename T> NSE_HD cpx<T> cadd(cpx<T> a, cpx<T> b) { return {a.x + b.x, a.y + b.y}; }
 template <typename T> NSE_HD cpx<T> csub(cpx<T> a, cpx<T> b) { return {a.x - b.x, a.y - b.y}; }
 template <typename T> NSE_HD cpx<T> mul_mi(cpx<T> a) { return {a.y, -a.x}; }   // a * (-i)
@@ -53,17 +49,16 @@ template <typename T, bool INV> NSE_HD void dft8(cpx<T>* v) {
     cpx<T> e[4] = {v[0], v[2], v[4], v[6]};
     cpx<T> o[4] = {v[1], v[3], v[5], v[7]};
     dft4<T, INV>(e); dft4<T, INV>(o);
-    // o_k *= w^k, w = e^{-i pi/4} (forward) or e^{+i pi/4} (inverse); the factor s goes into the
-    // multiply-adds of the combine
-    const cpx<T> o1 = INV ? cpx<T>{o[1].x - o[1].y, o[1].x + o[1].y} : cpx<T>{o[1].x + o[1].y, o[1].y - o[1].x};
-    const cpx<T> o2 = INV ? mul_pi(o[2]) : mul_mi(o[2]);
-    const cpx<T> o3 = INV ? cpx<T>{-(o[3].x + o[3].y), o[3].x - o[3].y} : cpx<T>{o[3].y - o[3].x, -(o[3].x + o[3].y)};
+    // o_k *= w^k, w = e^{-i pi/4} (forward) or e^{+i pi/4} (inverse)
+    cpx<T> o1 = INV ? cpx<T>{(o[1].x - o[1].y) * s, (o[1].x + o[1].y) * s}
+                    : cpx<T>{(o[1].x + o[1].y) * s, (o[1].y - o[1].x) * s};
+    cpx<T> o2 = INV ? mul_pi(o[2]) : mul_mi(o[2]);
+    cpx<T> o3 = INV ? cpx<T>{-(o[3].x + o[3].y) * s, (o[3].x - o[3].y) * s}
+                    : cpx<T>{(o[3].y - o[3].x) * s, -(o[3].x + o[3].y) * s};
     v[0] = cadd(e[0], o[0]); v[4] = csub(e[0], o[0]);
-    v[1] = {fmadd(s, o1.x, e[1].x), fmadd(s, o1.y, e[1].y)};
-    v[5] = {fmadd(-s, o1.x, e[1].x), fmadd(-s, o1.y, e[1].y)};
+    v[1] = cadd(e[1], o1);   v[5] = csub(e[1], o1);
     v[2] = cadd(e[2], o2);   v[6] = csub(e[2], o2);
-    v[3] = {fmadd(s, o3.x, e[3].x), fmadd(s, o3.y, e[3].y)};
-    v[7] = {fmadd(-s, o3.x, e[3].x), fmadd(-s, o3.y, e[3].y)};
+    v[3] = cadd(e[3], o3);   v[7] = csub(e[3], o3);
 }
 
 // 16-point DFT as 4 x 4: four 4-point DFTs over x[4 n1 + n2] (n1), the twiddles W16^(n2 k1),
@@ -84,7 +79,7 @@ template <typename T> NSE_HD cpx<T> mul_w16(cpx<T> a, int j, bool inv) {
         default: wr = 1; wi = 0; break;                          // j = 0 (j = 4 is handled by the caller)
     }
     if (inv) wi = -wi;
-    return {fmadd(a.x, wr, -(a.y * wi)), fmadd(a.x, wi, a.y * wr)};
+    return {a.x * wr - a.y * wi, a.x * wi + a.y * wr};
 }
 // e^{-i pi r / 16}, r = 0..15, from cos and sin of pi/16, pi/8, 3 pi/16, pi/4 (the doubles
 // nearest the exact values): the factor W_{2M}^{(M/16) r} that relates the split/merge twiddles

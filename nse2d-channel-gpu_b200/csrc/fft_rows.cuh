@@ -21,10 +21,6 @@ __device__ __forceinline__ cpx<float> ldtw(const cpx<float>* tw, int i) {
     return {v.x, v.y};
 }
 
-// a twiddle table that a kernel has copied to shared memory
-template <typename T> struct SmemTw { const cpx<T>* p; };
-template <typename T> __device__ __forceinline__ cpx<T> ldtw(const SmemTw<T>& tw, int i) { return tw.p[i]; }
-
 // Shared-memory layout of a row of M points: ip_idx<M>(i) = i + (i >> A) + (i >> B) (in elements)
 // spreads the digit-reversed writes of the first pass, the strided accesses of the later passes
 // and the split step's descending reads over the banks. A and B are chosen per M by counting
@@ -42,44 +38,27 @@ __host__ __device__ constexpr int ip_size(int M) {
 }
 
 // ---------------------------------------------------------------------------------------
-// Plan of the row transforms (FP64 and FP32): in-place decimation-in-time passes of radix R(q), q < P.
+// Radix-16 plan of the row transforms (FP64 and FP32): in-place decimation-in-time passes of
+// radix 16, the last one of the remaining 1..4 bits.
 //
-// Pass 0 reads its R0 points straight into registers: with the digit-reversed layout, the butterfly
-// that starts at position dit16_pos(t) (t < M / R0) holds the points t + (M / R0) r, r < R0, so
-// thread t loads a coalesced column of the row and writes its outputs to positions dit16_pos(t) + s.
+// Pass 0 reads its 16 points straight from global memory into registers: with the
+// digit-reversed layout, the butterfly that starts at position dit16_pos(t) (t < M/16) holds
+// the points t + (M/16) r, r < 16, so thread t loads a coalesced column of the row and writes
+// its 16 outputs to positions dit16_pos(t) + s.
 //
-// Pass q >= 1 (radix R, sub-transform length LP before it, L = R LP), for every group g and m < LP:
-// x_r = buf[g L + m + r LP] times W_L^(r m), an R-point DFT, written back in place. The output is in
-// natural order. Its twiddles come from four tables of W^m, W^2m, W^4m and W^8m, m < LP (one after
-// the other, so that the lanes of a warp, which take consecutive m, read consecutive entries);
-// W^(r m) is applied as W^(a m) W^(4 b m) with r = a + 4 b, so that at most six twiddles are live at
-// a time.
-//
-// Radices: 16 from 1024 points on (fewest passes through shared memory, and one row fills two or more
-// warps); 8 at 512 and 4 below, where a row has 2 to 16 points per thread and the length of a thread's
-// own chain counts: a radix-16 pass of a 128-point row would run on 8 threads.
+// Pass q >= 1 (radix R, sub-transform length LP = 16^q before it, L = R LP), for every group g
+// and m < LP: x_r = buf[g L + m + r LP] times W_L^(r m), an R-point DFT, written back in place.
+// The output is in natural order. Its twiddles come from four tables of W^m, W^2m, W^4m and
+// W^8m, m < LP (one after the other, so that the lanes of a warp, which take consecutive m,
+// read consecutive entries); W^(r m) is applied as W^(a m) W^(4 b m) with r = a + 4 b, so that
+// at most six twiddles are live at a time.
 // ---------------------------------------------------------------------------------------
-__host__ __device__ constexpr int plan_log2(int M) {
-    int m = 0;
-    while ((1 << m) < M) ++m;
-    return m;
-}
-__host__ __device__ constexpr int plan_radix_bits(int M) { return M >= 1024 || M < 32 ? 4 : (M == 512 ? 3 : 2); }
-__host__ __device__ constexpr int plan_P(int M) {
-    // the last pass takes what is left: up to the radix, or one bit more than radix 4
-    const int m = plan_log2(M), rb = plan_radix_bits(M);
-    return rb == 2 ? m / 2 : (m + rb - 1) / rb;
-}
-__host__ __device__ constexpr int plan_bits(int M, int q) {
-    return q < plan_P(M) - 1 ? plan_radix_bits(M) : plan_log2(M) - plan_radix_bits(M) * (plan_P(M) - 1);
-}
 template <int M> struct p16_plan {
     static constexpr int m = ilog2<M>::v;
-    static constexpr int P = plan_P(M);
-    static constexpr int bits(int q) { return plan_bits(M, q); }
+    static constexpr int P = (m + 3) / 4;
+    static constexpr int bits(int q) { return (q < P - 1) ? 4 : m - 4 * (P - 1); }
     static constexpr int R(int q) { return 1 << bits(q); }
-    static constexpr int sh(int q) { return plan_radix_bits(M) * q; }      // log2 of LP(q)
-    static constexpr int LP(int q) { return 1 << sh(q); }
+    static constexpr int LP(int q) { return 1 << (4 * q); }
     static constexpr int off(int q) {           // first table entry of pass q >= 1
         int o = 0;
         for (int i = 1; i < q; ++i) o += 4 * LP(i);
@@ -93,7 +72,7 @@ template <int M> __host__ __device__ __forceinline__ int dit16_pos(int n) {
 #pragma unroll
     for (int q = P - 1; q >= 0; --q) {
         const int b = p16_plan<M>::bits(q);
-        p |= ((n >> sn) & ((1 << b) - 1)) << p16_plan<M>::sh(q);
+        p |= ((n >> sn) & ((1 << b) - 1)) << (4 * q);
         sn += b;
     }
     return p;
@@ -102,8 +81,11 @@ template <int M> __host__ __device__ __forceinline__ int dit16_pos(int n) {
 template <typename C>
 inline void p16_twiddle_table(int M, const C* tw, std::vector<C>& out) {
     out.clear();
-    for (int q = 1; q < plan_P(M); ++q) {
-        const int LP = 1 << (plan_radix_bits(M) * q), R = 1 << plan_bits(M, q), L = R * LP, step = M / L;
+    int m = 0;
+    while ((1 << m) < M) ++m;
+    const int P = (m + 3) / 4;
+    for (int q = 1; q < P; ++q) {
+        const int LP = 1 << (4 * q), R = 1 << ((q < P - 1) ? 4 : m - 4 * (P - 1)), L = R * LP, step = M / L;
         for (int e = 1; e <= 8; e *= 2)
             for (int k = 0; k < LP; ++k) out.push_back(tw[((long long)e * step * k) % M]);
     }
@@ -126,8 +108,8 @@ __device__ __forceinline__ void p16_pass(cpx<T>* __restrict__ buf, const cpx<T>*
 
 // Butterfly b of pass q >= 1: loads its R points from the buffer, applies the twiddles and the
 // R-point DFT; v[r] is then the output at position base + r LP (returned in base).
-template <typename T, int M, int Q, bool INV, typename TW>
-__device__ __forceinline__ int p16_bfly(const cpx<T>* __restrict__ buf, const TW& tw, int b,
+template <typename T, int M, int Q, bool INV>
+__device__ __forceinline__ int p16_bfly(const cpx<T>* __restrict__ buf, const cpx<T>* __restrict__ tw, int b,
                                         cpx<T> (&v)[p16_plan<M>::R(Q)]) {
     constexpr int R = p16_plan<M>::R(Q), LP = p16_plan<M>::LP(Q), OFF = p16_plan<M>::off(Q);
     const int mm = b & (LP - 1);

@@ -31,8 +31,8 @@ int context_create(const Config& cfg, Context** out);
 void context_destroy(Context* c);
 int launch_stage(Context* c, int stage, const double* w_in, const double* w_n, double* w_out, cudaStream_t s,
                  double* rhs_out = nullptr);
-int launch_fft_fwd(Context* c, const double* src, cudaStream_t s);
-int launch_thomas(Context* c, cudaStream_t s);
+int launch_fft_fwd(Context* c, const double* src, cudaStream_t s, bool general = false);
+int launch_thomas(Context* c, cudaStream_t s, bool general = false);
 int launch_thomas_maps(Context* c, cudaStream_t s, bool homog = false);
 int launch_thomas_apply(Context* c, cudaStream_t s, bool homog = false);
 int launch_thomas_cluster(Context* c, cudaStream_t s, bool homog = false);
@@ -69,10 +69,10 @@ int export32(Context* c, bool with_rhs, cudaStream_t s);
 int step32_impl(Context* c, cudaStream_t s, bool store_rhs, cudaEvent_t* ev);
 const char* step32_kernel_name(const Context* c, int k);
 int launch_ifft_thom(Context* c, double* psi, double* w, int stage, bool do_thom, bool closure, cudaStream_t s,
-                     bool advance = false);
+                     bool advance = false, bool general = false);
 int launch_thom(Context* c, double* w, const double* psi, cudaStream_t s);
 int launch_maxuv(Context* c, const double* psi, bool set_dt, cudaStream_t s, bool next_only = false);
-int poisson_solve(Context* c, const double* w, double* psi, cudaStream_t s);
+int poisson_solve(Context* c, const double* w, double* psi, cudaStream_t s, bool general = false);
 int enqueue_step(Context* c, cudaStream_t s, bool store_rhs);
 int launches_per_step(const Context* c);
 int enqueue_step_timed(Context* c, cudaStream_t s, cudaEvent_t* ev, bool store_rhs = false);

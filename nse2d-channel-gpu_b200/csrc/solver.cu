@@ -11,6 +11,8 @@
 
 #include "nse2d_internal.h"
 #include "step_kernels.cuh"
+#include "band_fft.cuh"
+#include "solve_cta.cuh"
 
 namespace nse2d {
 
@@ -354,11 +356,13 @@ int context_create(const Config& cfg, Context** out) {
         set_error("metric upload failed");
         return fail();
     }
-    std::vector<cpx<double>> tw_full, tw, wN;
+    std::vector<cpx<double>> tw_full, tw, tw_band, wN;
     twiddles(c->M, tw_full, wN);
     p16_twiddle_table(c->M, tw_full.data(), tw);
-    if (dalloc(&c->tw, tw.size())) return fail();
+    plan_twiddle_table(c->M, band_radix_bits(c->M), tw_full.data(), tw_band);
+    if (dalloc(&c->tw, tw.size()) || dalloc(&c->tw_band, tw_band.size())) return fail();
     if (cudaMemcpy(c->tw, tw.data(), tw.size() * sizeof(tw[0]), cudaMemcpyHostToDevice) ||
+        cudaMemcpy(c->tw_band, tw_band.data(), tw_band.size() * sizeof(tw[0]), cudaMemcpyHostToDevice) ||
         cudaMemcpy(c->wN, wN.data(), wN.size() * sizeof(wN[0]), cudaMemcpyHostToDevice)) {
         set_error("twiddle upload failed");
         return fail();
@@ -511,6 +515,7 @@ void context_destroy(Context* c) {
     if (c->tbcarry) cudaFree(c->tbcarry);
     if (c->tcount) cudaFree(c->tcount);
     if (c->tw) cudaFree(c->tw);
+    if (c->tw_band) cudaFree(c->tw_band);
     if (c->wN) cudaFree(c->wN);
     if (c->ctl) cudaFree(c->ctl);
     if (c->h_ctl) cudaFreeHost(c->h_ctl);
@@ -602,7 +607,6 @@ template <typename K> static int fft_wave(K kern, size_t smem, int nrows, int nu
 }
 
 template <int M> static int fft_fwd_t(Context* c, FftParams& p, cudaStream_t s) {
-    if constexpr (M >= 32 && M <= 1024) { set_error("rows of %d points use the row-band kernels", 2 * M); return -1; } else {
     if constexpr (M == 16 * IP_NT) if (c->rowfft_pf) {
         // the real rows prefetched into shared memory by bulk copies (k_fft_fwd_pf)
         const size_t sm = FftPf<M>::smem;
@@ -614,7 +618,6 @@ template <int M> static int fft_fwd_t(Context* c, FftParams& p, cudaStream_t s) 
     int grid = 0;
     if (fft_wave(k_fft_fwd<M>, sm, p.nrows, c->num_sms, &grid)) return -1;
     return launch_step_kernel(c, k_fft_fwd<M>, dim3(grid), dim3(IP_NT), sm, s, nullptr, p);
-    }
 }
 
 // Inverse transforms: one wave of CTAs over contiguous bands of floor or ceil(Ny / wave) rows
@@ -649,12 +652,12 @@ template <int M> static int fft_inv_t(Context* c, FftParams& p, cudaStream_t s) 
         default: set_error("no FFT kernel for M = %d", c->M); return -1;           \
     }
 
-int launch_fft_fwd(Context* c, const double* src, cudaStream_t s) {
+int launch_fft_fwd(Context* c, const double* src, cudaStream_t s, bool general) {
     if (reinterpret_cast<uintptr_t>(src) % 16 != 0) {
         set_error("omega must be 16-byte aligned for the row transform (got %p)", (const void*)src);
         return -1;
     }
-    if (c->band) return band_rows_fwd(c, src, 1, c->Ni, s);
+    if (c->band && !general) return band_rows_fwd(c, src, 1, c->Ni, s);
     FftParams p = fft_params(c);
     p.src = src;
     p.row0 = 1;
@@ -677,8 +680,8 @@ int launch_fft_all_rows(Context* c, const double* src, cudaStream_t s) {
 }
 
 int launch_ifft_thom(Context* c, double* psi, double* w, int stage, bool do_thom, bool closure, cudaStream_t s,
-                     bool advance) {
-    if (c->band && !closure) return band_rows_inv(c, psi, w, do_thom, advance, s);
+                     bool advance, bool general) {
+    if (c->band && !closure && !general) return band_rows_inv(c, psi, w, do_thom, advance, s);
     FftParams p = fft_params(c);
     if (c->hat2) p.hat = c->hat2;
     p.psi = psi; p.w = w; p.stage = stage; p.do_thom = do_thom ? 1 : 0; p.closure = closure ? 1 : 0;
@@ -754,17 +757,35 @@ int set_tridiag_form(Context* c, bool clusters) {
     return 0;
 }
 
-// Launches of one tridiagonal solve: 1 (cluster form) or 2 (maps, apply); part i of them.
-int thomas_launches(const Context* c) { return c->thomas_cluster ? 1 : 2; }
+// The one-CTA form, which replaces both others on short grids (see solve_cta.cuh).
+using ThomasCtaKernel = void (*)(ThomasParams);
+template <bool F32> static ThomasCtaKernel thomas_cta_kernel(int kx, int L) {
+    if (kx == 2) return L == 1 ? k_thomas_cta<2, 1, F32> : (L == 2 ? k_thomas_cta<2, 2, F32> : k_thomas_cta<2, 4, F32>);
+    return L == 1 ? k_thomas_cta<4, 1, F32> : (L == 2 ? k_thomas_cta<4, 2, F32> : (L == 4 ? k_thomas_cta<4, 4, F32> : k_thomas_cta<4, 8, F32>));
+}
+static bool thomas_cta(const Context* c) { return c->Ni <= SC_MAX_NI; }
+static int launch_thomas_cta(Context* c, cudaStream_t s, bool homog) {
+    const int kx = solve_kx(c->H, c->num_sms), L = solve_L(c->Ni, kx);
+    return launch_step_kernel(c, homog ? thomas_cta_kernel<true>(kx, L) : thomas_cta_kernel<false>(kx, L), dim3((c->H + kx - 1) / kx),
+                              dim3(SC_NT), 0, s, nullptr, thomas_params(c, homog));
+}
+
+// Launches of one tridiagonal solve: 1 (one-CTA or cluster form) or 2 (maps, apply); part i of them.
+int thomas_launches(const Context* c) { return thomas_cta(c) || c->thomas_cluster ? 1 : 2; }
 const char* thomas_kernel_name(const Context* c, int i) {
+    if (thomas_cta(c)) return "k_thomas_cta";
     if (c->thomas_cluster) return "k_thomas_cluster";
     return i == 0 ? "k_thomas_maps" : "k_thomas_apply";
 }
 int launch_thomas_part(Context* c, int i, cudaStream_t s, bool homog) {
+    if (thomas_cta(c)) return launch_thomas_cta(c, s, homog);
     if (c->thomas_cluster) return launch_thomas_cluster(c, s, homog);
     return i == 0 ? launch_thomas_maps(c, s, homog) : launch_thomas_apply(c, s, homog);
 }
-int launch_thomas(Context* c, cudaStream_t s) {
+int launch_thomas(Context* c, cudaStream_t s, bool general) {
+    // (where the one-CTA form stands for both others, the plan does not choose between them)
+    if (general && (thomas_cta(c) ? c->thomas_cluster_ok : c->thomas_cluster)) return launch_thomas_cluster(c, s, false);
+    if (general) return launch_thomas_maps(c, s) || launch_thomas_apply(c, s) ? -1 : 0;
     for (int i = 0; i < thomas_launches(c); ++i)
         if (launch_thomas_part(c, i, s, false)) return -1;
     return 0;
@@ -792,11 +813,12 @@ int launch_maxuv(Context* c, const double* psi, bool set_dt, cudaStream_t s, boo
     return launch_step_kernel(c, k_maxuv_dt<true>, dim3(grid), dim3(256), 0, s, nullptr, p);
 }
 
-// Poisson solve of the reference (src/poisson.cuh:83-118): omega -> psi.
-int poisson_solve(Context* c, const double* w, double* psi, cudaStream_t s) {
-    if (launch_fft_fwd(c, w, s)) return -1;
-    if (launch_thomas(c, s)) return -1;
-    if (launch_ifft_thom(c, psi, nullptr, 0, false, false, s)) return -1;
+// Poisson solve of the reference (src/poisson.cuh:83-118): omega -> psi. general: by the transforms and the solve
+// that every grid has, whatever this one uses in its steps.
+int poisson_solve(Context* c, const double* w, double* psi, cudaStream_t s, bool general) {
+    if (launch_fft_fwd(c, w, s, general)) return -1;
+    if (launch_thomas(c, s, general)) return -1;
+    if (launch_ifft_thom(c, psi, nullptr, 0, false, false, s, false, general)) return -1;
     return 0;
 }
 
@@ -989,7 +1011,8 @@ int run_until_halt(Context* c, cudaStream_t s) {
 
 // omega (device) -> initial solve + Thom, t = 0 (src/main.cu:197-215)
 int set_initial_omega(Context* c, cudaStream_t s) {
-    if (poisson_solve(c, c->w, c->psi, s)) return -1;
+    // by the general kernels: a start is set once, and stays to the bit what it was whatever forms the steps take
+    if (poisson_solve(c, c->w, c->psi, s, true)) return -1;
     if (launch_thom(c, c->w, c->psi, s)) return -1;
     if (c->prec32 && split32(c, s)) return -1;
     Ctl h{};

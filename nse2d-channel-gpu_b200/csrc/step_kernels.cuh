@@ -855,7 +855,7 @@ static __global__ void __launch_bounds__(IP_NT, 5) k_ifft_thom(FftParams p) {
             const int t = b0 + (int)threadIdx.x;
             if (NB0 % IP_NT != 0 && t >= NB0) break;
             cpx<double> v[R0];
-            // W_{2M}^n for n = t + NB0 r is W_{2M}^t e^{-i pi r/R0} (one table load per thread)
+            // W_{2M}^n for n = t + NB0 r is W_{2M}^t e^{-i pi r/16} (one table load per thread)
             const cpx<double> wt = ldtw(p.wN, t);
 #pragma unroll
             for (int r = 0; r < R0; ++r) {
@@ -863,7 +863,7 @@ static __global__ void __launch_bounds__(IP_NT, 5) k_ifft_thom(FftParams p) {
                 const double2 av = __ldcs(X + n), bv = __ldcs(X + (M - n));
                 const cpx<double> sm = {av.x + bv.x, av.y - bv.y};
                 const cpx<double> df = {av.x - bv.x, av.y + bv.y};
-                const cpx<double> wn = (R0 >= 4) ? (r == 0 ? wt : cmul(wt, w32<double>(r * (16 / R0)))) : ldtw(p.wN, n);
+                const cpx<double> wn = (R0 == 16) ? (r == 0 ? wt : cmul(wt, w32<double>(r))) : ldtw(p.wN, n);
                 v[r] = cadd(sm, mul_pi(cmulc(df, wn)));
             }
             dftR<double, R0, true>(v);
@@ -1941,9 +1941,9 @@ static __global__ void __launch_bounds__(256) k_thom(ThomParams p) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < Nx; i += gridDim.x * blockDim.x) {
         if (p.free_slip) { p.w[i] = 0.0; wt[i] = 0.0; continue; }
         const double d1 = p.psi[(size_t)1 * Nx + i] - p.psi_bot, d2 = p.psi[(size_t)2 * Nx + i] - p.psi_bot;
-        p.w[i] = thom_value(Ab, Bb, d1, d2);
+        p.w[i] = -(Ab * d1 + Bb * d2);
         const double e1 = p.psi[(size_t)(Ny - 2) * Nx + i] - p.psi_top, e2 = p.psi[(size_t)(Ny - 3) * Nx + i] - p.psi_top;
-        wt[i] = thom_value(At, Bt, e1, e2);
+        wt[i] = -(At * e1 + Bt * e2);
     }
 }
 
