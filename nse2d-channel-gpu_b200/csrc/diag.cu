@@ -136,28 +136,31 @@ __global__ void __launch_bounds__(256) k_diag_rows(DiagParams p) {
     }
 }
 
-// Sum the rows of each quantity, compensated: a CTA per quantity, a thread per 64th row, then the threads in order.
-constexpr int DIAG_FT = 64;
-__global__ void __launch_bounds__(DIAG_FT) k_diag_final(const double* rows, int Ny, double* out) {
-    __shared__ double part[2][DIAG_FT];
-    const int q = blockIdx.x, t = threadIdx.x;
+// Sum the rows of each quantity, compensated: a warp (a CTA of its own) per quantity, a lane per 32nd row, then the
+// lanes in order.
+__global__ void __launch_bounds__(32) k_diag_final(const double* rows, int Ny, double* out) {
+    __shared__ double part[32];
+    const int q = blockIdx.x, lane = threadIdx.x;
     double s = 0.0, cmp = 0.0;
-    auto add = [&](double x) {
-        const double u = s + x;
-        cmp += (fabs(s) >= fabs(x)) ? (s - u) + x : (x - u) + s;
-        s = u;
-    };
-#pragma unroll 4
-    for (int j = t; j < Ny; j += DIAG_FT) add(rows[(size_t)j * NSUM + q]);
-    part[0][t] = s;
-    part[1][t] = cmp;
-    __syncthreads();
-    if (t != 0) return;
-    for (int k = 1; k < DIAG_FT; ++k) {
-        add(part[0][k]);
-        cmp += part[1][k];
+#pragma unroll 8
+    for (int j = lane; j < Ny; j += 32) {
+        const double x = rows[(size_t)j * NSUM + q];
+        const double t = s + x;
+        cmp += (fabs(s) >= fabs(x)) ? (s - t) + x : (x - t) + s;
+        s = t;
     }
-    out[q] = s + cmp;
+    part[lane] = s + cmp;
+    __syncwarp();
+    if (lane == 0) {
+        double S = 0.0, C = 0.0;
+        for (int k = 0; k < 32; ++k) {
+            const double x = part[k];
+            const double t = S + x;
+            C += (fabs(S) >= fabs(x)) ? (S - t) + x : (x - t) + S;
+            S = t;
+        }
+        out[q] = S + C;
+    }
 }
 
 int rhs_at_state(Context* c, const double* w, const double* psi, double* J, double* rhs, double tm, cudaStream_t s);
@@ -174,7 +177,7 @@ static int read_sums(Context* c, const double* J, double* host_out, cudaStream_t
     const int grid = std::min(c->Ny, 8 * c->num_sms);
     k_diag_rows<<<grid, 256, 0, s>>>(p);
     NSE_CUDA_TRY(cudaGetLastError());
-    k_diag_final<<<NSUM, DIAG_FT, 0, s>>>(c->red_blocks, c->Ny, c->red_out);
+    k_diag_final<<<NSUM, 32, 0, s>>>(c->red_blocks, c->Ny, c->red_out);
     NSE_CUDA_TRY(cudaGetLastError());
     NSE_CUDA_TRY(cudaMemcpyAsync(host_out, c->red_out, NSUM * sizeof(double), cudaMemcpyDeviceToHost, s));
     NSE_CUDA_TRY(cudaStreamSynchronize(s));
