@@ -34,7 +34,7 @@ template <int M> struct Band {
     static constexpr int R0 = band_plan<M>::R(0);
     static constexpr int NB0 = M / R0;                       // pass-0 butterflies of a row
     static constexpr int TPR = M <= 128 ? 32 : 64;           // threads of a row group
-    static constexpr int ROW = ip_size(M);                   // elements of a row buffer
+    static constexpr int ROW = M + (M >> ip_shift_a(M)) + (M >> ip_shift_b(M)) + 1;   // elements of a row buffer: 0 .. M, padded
     static constexpr int RMAX = M <= 256 ? 6 : 4;            // rows of a band of k_band (M <= 512)
     static constexpr int MAXT = (RMAX + 2) * TPR;
     static constexpr int ROWS_G = 4;                         // row groups per CTA of the transforms alone
@@ -78,24 +78,18 @@ template <typename T> struct BandParams {
     double wall_bot, wall_top;   // FP32: the constant part of the wall vorticity
 };
 
+// filled by the launchers
+BandParams<double> band_params64(const Context* c);
+
 template <int TPR> __device__ __forceinline__ void row_sync(int group) {
     if constexpr (TPR == 32) __syncwarp();
     else asm volatile("bar.sync %0, %1;\n" ::"r"(group + 1), "n"(TPR) : "memory");
 }
 
-// element copy to shared memory (16 bytes in FP64, 8 in FP32)
+// element copy to shared memory (16 bytes in FP64, past L1; 8 in FP32, through it: after a barrier across the grid
+// L1 holds nothing stale)
 __device__ __forceinline__ void cp_async_cpx(cpx<double>* d, const cpx<double>* g) { cp_async16(d, g); }
 __device__ __forceinline__ void cp_async_cpx(cpx<float>* d, const cpx<float>* g) { cp_async8(d, g); }
-
-// loads from L2, for what other CTAs of the same launch wrote
-__device__ __forceinline__ cpx<double> ldcg_cpx(const cpx<double>* q) {
-    const double2 v = __ldcg(reinterpret_cast<const double2*>(q));
-    return {v.x, v.y};
-}
-__device__ __forceinline__ cpx<float> ldcg_cpx(const cpx<float>* q) {
-    const float2 v = __ldcg(reinterpret_cast<const float2*>(q));
-    return {v.x, v.y};
-}
 
 // The twiddles to shared memory (no kernel writes them, so this may precede the wait for the previous
 // kernel): every pass of every row reads them, and a table read from global memory would wait on L2
@@ -127,43 +121,33 @@ __device__ __forceinline__ void band_passes(cpx<T>* buf, const SmemTw<T>& tw, in
     if constexpr (Q < band_plan<M>::P - 1) band_passes<T, M, Q + 1, INV>(buf, tw, t, group, out);
 }
 
-// Inverse transform of one spectral row X into out(n, z_n) (z_n = x_2n + i x_2n+1, times 2M), through buf:
-// the merge of k_ifft_thom, then the passes. In two parts, so that the loads of short rows are in flight
-// before the tables are waited for (PRE; 16 points and their mirrors would be 128 registers).
-template <typename T, int M> struct BandSpec {
-    static constexpr bool PRE = Band<M>::R0 <= 8;
-    cpx<T> a[PRE ? Band<M>::R0 : 1], c[PRE ? Band<M>::R0 : 1];
-    template <bool CG = false> __device__ __forceinline__ void load(const cpx<T>* X, int t) {
-        if constexpr (PRE) {
-            if (t < Band<M>::NB0) {
-#pragma unroll
-                for (int r = 0; r < Band<M>::R0; ++r) {
-                    a[r] = CG ? ldcg_cpx(X + t + Band<M>::NB0 * r) : ldtw(X, t + Band<M>::NB0 * r);
-                    c[r] = CG ? ldcg_cpx(X + M - t - Band<M>::NB0 * r) : ldtw(X, M - t - Band<M>::NB0 * r);
-                }
-            }
-        }
-    }
-};
+// A spectral row X_0 .. X_M into buf (cp.async past L1; natural order, padded). Pass 0 needs X_n and X_{M-n}: from
+// shared memory they cost one read of the row, and none of the registers that two loads per point in flight do.
+template <typename T, int M> __device__ __forceinline__ void band_load_spec(const cpx<T>* X, cpx<T>* buf, int t) {
+    for (int n = t; n <= M; n += Band<M>::TPR) cp_async_cpx(buf + ip_idx<M>(n), X + n);
+}
+// Inverse transform of the spectral row in buf (all of it arrived, and a barrier of the group since) into
+// out(n, z_n), z_n = x_2n + i x_2n+1, times 2M: the merge of k_ifft_thom, then the passes.
 template <typename T, int M, typename Out>
-__device__ __forceinline__ void band_inverse(const BandSpec<T, M>& sp, const cpx<T>* __restrict__ X, cpx<T>* buf, const SmemTw<T>& tw,
-                                             const SmemTw<T>& wN, int t, int group, Out out) {
+__device__ __forceinline__ void band_inverse(cpx<T>* buf, const SmemTw<T>& tw, const SmemTw<T>& wN, int t, int group, Out out) {
     constexpr int NB0 = Band<M>::NB0, TPR = Band<M>::TPR, R0 = Band<M>::R0;
-    if (NB0 >= TPR || t < NB0) {
-        cpx<T> v[R0];
+    const bool on = NB0 >= TPR || t < NB0;
+    cpx<T> v[R0];
+    if (on) {
         const cpx<T> wt = ldtw(wN, t);
 #pragma unroll
         for (int r = 0; r < R0; ++r) {
             const int n = t + NB0 * r;
-            cpx<T> a, c;
-            if constexpr (BandSpec<T, M>::PRE) { a = sp.a[r]; c = sp.c[r]; }
-            else { a = ldtw(X, n); c = ldtw(X, M - n); }
+            const cpx<T> a = buf[ip_idx<M>(n)], c = buf[ip_idx<M>(M - n)];
             const cpx<T> sm = {a.x + c.x, a.y - c.y};
             const cpx<T> df = {a.x - c.x, a.y + c.y};
             const cpx<T> wn = (r == 0) ? wt : fmul_c(wt, w32<T>(r * (16 / R0)));
             v[r] = cadd(sm, mul_pi(fmul_cc(df, wn)));
         }
         fdftR<T, R0, true>(v);
+    }
+    row_sync<TPR>(group);                                     // the spectral row is read
+    if (on) {
         const int p0 = dit_pos<band_plan<M>>(t);
 #pragma unroll
         for (int q = 0; q < R0; ++q) buf[ip_idx<M>(p0 + q)] = v[q];
@@ -387,8 +371,12 @@ template <typename T, int M> struct BandCta {
         const cpx<T>* src = reinterpret_cast<const cpx<T>*>(w) + (size_t)row() * M;
         for (int c = t; c < CH; c += B::TPR) cp_async16(wns + (size_t)(group - 1) * M + CE * c, src + CE * c);
     }
-    // psi rows j0 - 1 .. j1 from psi-hat (sp: the group's loads in flight)
-    __device__ __forceinline__ void inverse(const BandParams<T>& p, const BandSpec<T, M>& sp) {
+    // psi-hat rows j0 - 1 .. j1 into the row buffers (cp.async)
+    __device__ __forceinline__ void load_spec(const BandParams<T>& p) {
+        if (rowed() && !wallrow()) band_load_spec<T, M>(p.hat_in + (size_t)row() * p.Hp, buf(), t);
+    }
+    // psi rows j0 - 1 .. j1 from them, once they have arrived
+    __device__ __forceinline__ void inverse(const BandParams<T>& p) {
         if (!rowed()) return;
         cpx<T>* b = buf();
         if (wallrow()) {
@@ -396,8 +384,7 @@ template <typename T, int M> struct BandCta {
             for (int n = t; n < M; n += B::TPR) b[ip_idx<M>(n)] = cpx<T>{v, v};
         } else {
             constexpr T scale = (T)0.5 / (T)M;                // the merge forms 2 Z_n
-            band_inverse<T, M>(sp, p.hat_in + (size_t)row() * p.Hp, b, tw, wN, t, group,
-                               [&](int n, const cpx<T>& z) { b[ip_idx<M>(n)] = cpx<T>{z.x * scale, z.y * scale}; });
+            band_inverse<T, M>(b, tw, wN, t, group, [&](int n, const cpx<T>& z) { b[ip_idx<M>(n)] = cpx<T>{z.x * scale, z.y * scale}; });
         }
     }
     // wall rows of w (and of the omega rows) from the psi rows; between barriers
@@ -490,16 +477,16 @@ static __global__ void __launch_bounds__(Band<M>::MAXT, 1) k_band(BandParams<T> 
     c.load_consts(p);                                         // before the wait for the previous kernel
     pdl_begin();
     const T dt = (T)p.ctl->dt;
-    BandSpec<T, M> sp;
-    if (INV && c.rowed() && !c.wallrow()) sp.load(p.hat_in + (size_t)c.row() * p.Hp, c.t);
-    if constexpr (!INV) c.load_psi(p.psi_in);
+    if constexpr (INV) c.load_spec(p);
+    else c.load_psi(p.psi_in);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
     c.load_omega(p.w_in, !INV);                               // in flight while psi is transformed
     if (p.stage > 1) c.load_omega_n(p.w_n);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
     if constexpr (INV) {
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-        __syncthreads();                                      // the tables
-        c.inverse(p, sp);
+        __syncthreads();                                      // the tables and the spectral rows
+        c.inverse(p);
     }
     cp_async_wait_all();
     __syncthreads();
@@ -555,16 +542,14 @@ static __global__ void __launch_bounds__(Band<M>::ROWS_G * Band<M>::TPR) k_rows_
     cpx<T>* psi = reinterpret_cast<cpx<T>*>(p.psi_out);
     band_load_tables<T, M>(tab, p);
     pdl_begin();
-    BandSpec<T, M> sp;
-    if (j0 + group < j1) sp.load(p.hat_in + (size_t)(j0 + group) * p.Hp, t);
+    cpx<T>* buf = rows + (size_t)group * B::ROW;
+    if (j0 + group < j1) band_load_spec<T, M>(p.hat_in + (size_t)(j0 + group) * p.Hp, buf, t);
     cp_async_wait_all();
     __syncthreads();
     if (j0 + group < j1) {
-        cpx<T>* buf = rows + (size_t)group * B::ROW;
         cpx<T>* dst = psi + (size_t)(j0 + group) * M;
         constexpr T scale = (T)0.5 / (T)M;
-        band_inverse<T, M>(sp, p.hat_in + (size_t)(j0 + group) * p.Hp, buf, SmemTw<T>{tab}, SmemTw<T>{tab + band_ntw<M>()}, t, group,
-                           [&](int n, const cpx<T>& z) {
+        band_inverse<T, M>(buf, SmemTw<T>{tab}, SmemTw<T>{tab + band_ntw<M>()}, t, group, [&](int n, const cpx<T>& z) {
             const cpx<T> o = {z.x * scale, z.y * scale};
             dst[n] = o;
             if (wall) buf[ip_idx<M>(n)] = o;

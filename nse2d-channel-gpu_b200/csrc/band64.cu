@@ -14,7 +14,7 @@ bool band_stage_ok(int M) { return M >= 32 && M <= 512; }
 // Rows per band: one band per SM while it fits, so that a launch is one wave.
 static int band_R(const Context* c, int rmax) { return std::max(1, std::min(rmax, (c->Ni + c->num_sms - 1) / c->num_sms)); }
 
-static BandParams<double> band_params(Context* c) {
+BandParams<double> band_params64(const Context* c) {
     BandParams<double> p{};
     p.hat_in = c->hat2 ? c->hat2 : c->hat; p.hat_out = c->hat; p.psi_in = c->psi; p.tw = c->tw_band; p.wN = c->wN; p.rt = c->rt; p.ctl = c->ctl;
     p.Nx = c->Nx; p.Ny = c->Ny; p.Hp = c->Hp; p.free_slip = c->cfg.free_slip;
@@ -64,20 +64,20 @@ template <int M> static int rows_inv_t(Context* c, BandParams<double>& p, cudaSt
 // psi-hat and the wall closure of w_in before it (else psi is read from the context's psi).
 int band_stage(Context* c, int stage, bool inv, double* w_in, const double* w_n, double* w_out, double* rhs_out,
                const double* closure, cudaStream_t s) {
-    BandParams<double> p = band_params(c);
+    BandParams<double> p = band_params64(c);
     p.stage = stage; p.w_in = w_in; p.w_n = w_n; p.w_out = w_out; p.rhs_out = rhs_out; p.closure = closure;
     if (inv) { NSE_BAND512_DISPATCH(band_inv_t) }
     NSE_BAND512_DISPATCH(band_psi_t)
 }
 
 int band_rows_fwd(Context* c, const double* src, int row0, int nrows, cudaStream_t s) {
-    BandParams<double> p = band_params(c);
+    BandParams<double> p = band_params64(c);
     p.src = src; p.row0 = row0; p.nrows = nrows;
     NSE_BAND_DISPATCH(rows_fwd_t)
 }
 
 int band_rows_inv(Context* c, double* psi, double* w, bool thom, bool advance, cudaStream_t s) {
-    BandParams<double> p = band_params(c);
+    BandParams<double> p = band_params64(c);
     p.psi_out = psi; p.w_in = w; p.do_thom = thom ? 1 : 0; p.advance = advance ? 1 : 0;
     NSE_BAND_DISPATCH(rows_inv_t)
 }

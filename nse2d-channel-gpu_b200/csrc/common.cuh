@@ -69,6 +69,9 @@ struct Ctl {
     int acc_every;
     double acc_last_t, acc_T;
     double mx_next[3];             // max |u|, |v|, |v| a of the current psi (the next step's dt)
+    // steps in one launch (steps.cuh): barrier arrivals, exits, and the maxima of alternate steps (all 0 between launches)
+    unsigned int bar_arrive, bar_exit;
+    unsigned long long mx2[2][3];
     // run mode (nse2d_run): stop stepping when an output, a statistics step or the end is due
     int run;                       // 1 while a run is active
     int halt;                      // set at the end of the step after which the run stops
@@ -122,6 +125,7 @@ struct Context {
     // otherwise psi-hat takes the place of omega-hat
     cpx<double>* hat2 = nullptr;
     bool band = false;             // row transforms of band.cuh: rows of 64 to 2048 points
+    int steps_R = 0;               // rows of a band of the steps in one launch (0: not used)
     bool plain_step = false;       // a step of separate transforms and stages (nse2d_step_profiled times them apart)
     double* cp = nullptr;          // elimination table [Ni][Hp]
     cpx<double>* tw = nullptr;     // per-pass twiddle pairs of the Nx/2-point transform

@@ -43,6 +43,9 @@ int band_stage(Context* c, int stage, bool inv, double* w_in, const double* w_n,
                const double* closure, cudaStream_t s);
 int band_rows_fwd(Context* c, const double* src, int row0, int nrows, cudaStream_t s);
 int band_rows_inv(Context* c, double* psi, double* w, bool thom, bool advance, cudaStream_t s);
+// whole steps in one launch (steps64.cu): store: the stage-3 rhs never (0), in the last step (1), in every one (2)
+int steps_setup(Context* c);
+int launch_steps(Context* c, int nsteps, int run, int store, cudaStream_t s);
 // learned closure (closure.cu)
 struct Cnn;
 int cnn_forward_psi(Cnn* n, const double* w, const double* psi, const double* a_node, double inv_dx, double inv_deta, double* tau,

@@ -22,8 +22,24 @@ template <int KX> struct SolveSmem {
 // threads 0 .. 255 of a CTA (bar.sync 15)
 __device__ __forceinline__ void sc_sync() { asm volatile("bar.sync 15, %0;\n" ::"n"(SC_NT) : "memory"); }
 
-template <int KX, int L, bool F32>
-__device__ __forceinline__ void solve_columns(const ThomasParams& p, int g, SolveSmem<KX>& sm) {
+// Where the coefficients come from: global memory (one solve), or the CTA's own columns in shared memory (a launch of
+// many solves, k_steps): cp[Ni][KX] and rc[Ni] = {asub, 1 / csup}.
+template <int KX> struct SolveCoefGlobal {
+    const ThomasParams& p;
+    int kx;
+    __device__ __forceinline__ double cp(int r) const { return __ldg(&p.cp[(size_t)r * p.Hp + kx]); }
+    __device__ __forceinline__ double2 row(int r) const { return make_double2(__ldg(&p.asub[r + 1]), __ldg(&p.inv_csup[r + 1])); }
+};
+template <int KX> struct SolveCoefShared {
+    const double* c;
+    const double2* rc;
+    int k;
+    __device__ __forceinline__ double cp(int r) const { return c[r * KX + k]; }
+    __device__ __forceinline__ double2 row(int r) const { return rc[r]; }
+};
+
+template <int KX, int L, bool F32, typename Coef>
+__device__ __forceinline__ void solve_columns(const ThomasParams& p, int g, SolveSmem<KX>& sm, const Coef& coef) {
     using ST2 = typename SpecT<F32>::T2;
     const int tid = threadIdx.x, k = tid % KX, q = tid / KX, lane = tid & 31, w = tid >> 5;
     const int kx = g * KX + k, lo = q * L, Ni = p.Ni;
@@ -36,10 +52,16 @@ __device__ __forceinline__ void solve_columns(const ThomasParams& p, int g, Solv
 #pragma unroll
     for (int i = 0; i < L; ++i) {                            // kx < Hp: the padding columns hold zeros
         x[i] = make_double2(0.0, 0.0);
+        if (lo + i < Ni) x[i] = spec_wide(__ldcg(hat + (size_t)(lo + i + 1) * Hp + kx));
+    }
+    // the coefficients while the spectra are on their way (be: 1 / c_i until the sweep)
+#pragma unroll
+    for (int i = 0; i < L; ++i) {
         cpv[i] = 0.0;
+        be[i] = 0.0;
         if (lo + i < Ni) {
-            x[i] = spec_wide(__ldcg(hat + (size_t)(lo + i + 1) * Hp + kx));
-            cpv[i] = __ldg(&p.cp[(size_t)(lo + i) * Hp + kx]);
+            cpv[i] = coef.cp(lo + i);
+            be[i] = coef.row(lo + i).y;
         }
     }
     // rhs = -omega-hat, with the k = 0 Dirichlet wall terms of src/poisson.cu:91-95,109-114
@@ -54,10 +76,9 @@ __device__ __forceinline__ void solve_columns(const ThomasParams& p, int g, Solv
     AffMap m{make_double2(0.0, 0.0), 1.0};
 #pragma unroll
     for (int i = 0; i < L; ++i) {
-        be[i] = 0.0;
         if (lo + i < Ni) {
-            const double alpha = cpv[i] * __ldg(&p.inv_csup[lo + i + 1]);
-            be[i] = -__ldg(&p.asub[lo + i + 1]) * alpha;
+            const double alpha = cpv[i] * be[i];
+            be[i] = -coef.row(lo + i).x * alpha;
             m.D.x = fma(be[i], m.D.x, -alpha * x[i].x);
             m.D.y = fma(be[i], m.D.y, -alpha * x[i].y);
             x[i] = m.D;
@@ -150,7 +171,7 @@ template <int KX, int L, bool F32>
 static __global__ void __launch_bounds__(SC_NT) k_thomas_cta(ThomasParams p) {
     __shared__ SolveSmem<KX> sm;
     pdl_begin();
-    solve_columns<KX, L, F32>(p, blockIdx.x, sm);
+    solve_columns<KX, L, F32>(p, blockIdx.x, sm, SolveCoefGlobal<KX>{p, (int)blockIdx.x * KX + (int)threadIdx.x % KX});
 }
 
 }  // namespace nse2d

@@ -114,7 +114,7 @@ static ThomasClusterKernel thomas_cluster_kernel(int L, bool f32 = false) {
 }
 
 // homog: the FP32-bulk step's solve, for psi' (zero on the walls) in the FP32 spectral buffer
-static ThomasParams thomas_params(const Context* c, bool homog = false) {
+ThomasParams thomas_params(const Context* c, bool homog) {
     ThomasParams p{};
     p.hat = c->hat; p.hat32 = c->hat32; p.out = c->hat2 ? c->hat2 : c->hat; p.out32 = c->hat32; p.cp = c->cp; p.asub = c->rt.asub; p.inv_csup = c->rt.inv_csup; p.csup = c->rt.csup;
     p.tconst = c->tconst; p.tmaps = c->tmaps; p.tblk = c->tblk; p.tbcarry = c->tbcarry; p.tcount = c->tcount;
@@ -492,6 +492,7 @@ int context_create(const Config& cfg, Context** out) {
             c->tc_nclusters32 = std::min(nclusters, c->Hp / TC_KX);
         }
     }
+    if (c->hat2 && steps_setup(c)) return fail();
     Ctl h{};
     h.t = 0.0; h.dt = cfg.dt_init; h.next_out = 1e300; h.next_snap = 1e300; h.next_diag = 1e300;
     if (cudaMemcpy(c->ctl, &h, sizeof(Ctl), cudaMemcpyHostToDevice) != cudaSuccess) { set_error("ctl upload"); return fail(); }
@@ -801,13 +802,19 @@ int launch_thom(Context* c, double* w, const double* psi, cudaStream_t s) {
     return 0;
 }
 
-int launch_maxuv(Context* c, const double* psi, bool set_dt, cudaStream_t s, bool next_only) {
+MaxParams max_params(const Context* c) {
     MaxParams p{};
-    p.psi = psi; p.a_node = c->rt.a_node; p.ctl = c->ctl; p.next_only = next_only ? 1 : 0;
-    p.Nx = c->Nx; p.Ny = c->Ny; p.adapt = c->cfg.adapt; p.set_dt = set_dt ? 1 : 0;
+    p.psi = c->psi; p.a_node = c->rt.a_node; p.ctl = c->ctl;
+    p.Nx = c->Nx; p.Ny = c->Ny; p.adapt = c->cfg.adapt;
     p.inv_dx = c->inv_dx; p.inv_deta = c->inv_deta; p.cfl = c->cfg.cfl; p.cvisc = c->cfg.cvisc;
     p.dx = c->dx; p.deta = c->deta; p.nu = c->nu; p.inv_dx2 = c->inv_dx2; p.inv_dymin2 = c->inv_dymin2;
     p.dt_max = c->cfg.dt_max;
+    return p;
+}
+
+int launch_maxuv(Context* c, const double* psi, bool set_dt, cudaStream_t s, bool next_only) {
+    MaxParams p = max_params(c);
+    p.psi = psi; p.next_only = next_only ? 1 : 0; p.set_dt = set_dt ? 1 : 0;
     int grid = 1;
     maxuv_plan(p, c->maxuv_ctas, c->maxuv_ctas, grid);
     return launch_step_kernel(c, k_maxuv_dt<true>, dim3(grid), dim3(256), 0, s, nullptr, p);
@@ -930,9 +937,23 @@ int refresh_maxima(Context* c, cudaStream_t s) {
     return launch_maxuv(c, c->psi, false, s, true);
 }
 
-// nsteps steps; with use_graph the step is captured once into a CUDA graph and replayed.
+// Steps in one launch (steps.cuh): where the grid's bands are all resident, without a model between the stages, and
+// not into a stream that is being captured (nor inside an ensemble, whose members share the device).
+static bool steps_ok(const Context* c, cudaStream_t s) {
+    if (!c->steps_R || !band_step(c) || c->closure_net) return false;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return st == cudaStreamCaptureStatusNone;
+}
+
+// nsteps steps: in one launch where the grid allows it; else, with use_graph, the step is captured once into a
+// CUDA graph and replayed.
 int run_steps(Context* c, int nsteps, bool use_graph, cudaStream_t s, bool store_rhs) {
     if (nsteps <= 0) return 0;
+    if (steps_ok(c, s)) return launch_steps(c, nsteps, 0, store_rhs ? 1 : 0, s);
     if (!use_graph || store_rhs) {
         for (int i = 0; i < nsteps; ++i)
             if (enqueue_step(c, s, store_rhs && i == nsteps - 1)) return -1;
@@ -970,6 +991,14 @@ static __global__ void k_loop_cond(Ctl* ctl, cudaGraphConditionalHandle h) {
 // a WHILE node whose body is one captured step followed by k_loop_cond. The run fields of the
 // control block must be set (run = 1, halt = 0, run_budget > 0) before the launch.
 int run_until_halt(Context* c, cudaStream_t s) {
+    if (!c->stats_dev && steps_ok(c, s)) {
+        for (;;) {                                           // launches of at most 8192 steps (0.1 to 0.5 s)
+            if (launch_steps(c, 8192, 1, 2, s)) return -1;
+            NSE_CUDA_TRY(cudaMemcpyAsync(c->h_ctl, c->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
+            NSE_CUDA_TRY(cudaStreamSynchronize(s));
+            if (c->h_ctl->halt || (c->h_ctl->nonfinite & 2)) return 0;
+        }
+    }
     if (!c->run_exec) {
         if (!c->cap_stream) NSE_CUDA_TRY(cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
         cudaGraph_t g = nullptr;

@@ -517,35 +517,55 @@ static __global__ void __launch_bounds__(256, 2) k_stage_tma(const __grid_consta
     }
 }
 
-// t += dt, step++, and the snap to the scheduled output times (src/main.cu:541-551): the
-// tolerance is re-evaluated after the first snap, as the reference does.
-__device__ __forceinline__ void advance_time(Ctl* ctl) {
-    const double dt = ctl->dt;
-    double t = ctl->t + dt;
-    const double ns = ctl->next_snap, nd = ctl->next_diag;
-    if (ns < 1e299 && fabs(t - ns) <= fmax(time_tol_d(t), 1e-6 * fmax(1e-300, fabs(dt)))) t = ns;
-    if (nd < 1e299 && fabs(t - nd) <= fmax(time_tol_d(t), 1e-6 * fmax(1e-300, fabs(dt)))) t = nd;
-    ctl->t = t;
-    ctl->step += 1;
-    if (ctl->run) {
+// The time of a channel and what decides when a run stops.
+struct StepClock {
+    double t, dt, next_out, next_snap, next_diag, t_end;
+    long long step;
+    int stats_every, nonfinite_halted;
+
+    __device__ __forceinline__ void load(const Ctl* c) {
+        t = c->t; dt = c->dt; next_out = c->next_out; next_snap = c->next_snap; next_diag = c->next_diag; t_end = c->t_end;
+        step = c->step; stats_every = c->stats_every; nonfinite_halted = c->nonfinite_halted;
+    }
+    __device__ __forceinline__ void store(Ctl* c) const {
+        c->t = t; c->dt = dt; c->step = step; c->nonfinite_halted = nonfinite_halted;
+    }
+    // t += dt, step++, and the snap to the scheduled output times (src/main.cu:541-551): the tolerance is
+    // re-evaluated after the first snap, as the reference does. In a run, the NSE2D_HALT_* bits of the reasons
+    // to stop after this step; nonfinite: the flags as this step began.
+    __device__ __forceinline__ int advance(int run, int nonfinite) {
+        t = t + dt;
+        if (next_snap < 1e299 && fabs(t - next_snap) <= fmax(time_tol_d(t), 1e-6 * fmax(1e-300, fabs(dt)))) t = next_snap;
+        if (next_diag < 1e299 && fabs(t - next_diag) <= fmax(time_tol_d(t), 1e-6 * fmax(1e-300, fabs(dt)))) t = next_diag;
+        step += 1;
+        if (!run) return 0;
         // the host's output and loop tests of src/main.cu:434,553-566,695 after this step
         // (with the wider snapshot tolerance, so that no due output is missed)
         const double tol = fmax(time_tol_d(t), 1e-6 * fmax(1e-300, fabs(dt)));
         int r = 0;
-        if (fmin(ns, nd) < 1e299 && t + tol >= fmin(ns, nd)) r |= 1;
-        if (ctl->stats_every > 0 && (ctl->step % ctl->stats_every) == 0) r |= 2;
-        if (!(t < ctl->t_end - 0.5 * dt)) r |= 4;
-        if (ctl->nonfinite & 2) r |= 8;     // a bounded wait gave up
+        if (fmin(next_snap, next_diag) < 1e299 && t + tol >= fmin(next_snap, next_diag)) r |= 1;
+        if (stats_every > 0 && (step % stats_every) == 0) r |= 2;
+        if (!(t < t_end - 0.5 * dt)) r |= 4;
+        if (nonfinite & 2) r |= 8;          // a bounded wait gave up
         // the first NaN or Inf a reduction meets halts the run once, so that the host sees it; the
         // run may then go on, as the reference's loop does with non-finite fields
-        if ((ctl->nonfinite & 1) && !ctl->nonfinite_halted) {
+        if ((nonfinite & 1) && !nonfinite_halted) {
             r |= 8;
-            ctl->nonfinite_halted = 1;
+            nonfinite_halted = 1;
         }
-        if (r) {
-            ctl->halt = 1;
-            ctl->halt_reason = r;
-        }
+        return r;
+    }
+};
+
+// the same on the control block, at the end of a step by launches
+__device__ __forceinline__ void advance_time(Ctl* ctl) {
+    StepClock k;
+    k.load(ctl);
+    const int r = k.advance(ctl->run, ctl->nonfinite);
+    k.store(ctl);
+    if (r) {
+        ctl->halt = 1;
+        ctl->halt_reason = r;
     }
 }
 
@@ -1959,6 +1979,10 @@ struct MaxParams {
     double inv_dx, inv_deta, cfl, cvisc, dx, deta, nu, inv_dx2, inv_dymin2, dt_max;
 };
 
+
+// parameters of the solve and of the max reduction of a context (solver.cu)
+ThomasParams thomas_params(const Context* c, bool homog = false);
+MaxParams max_params(const Context* c);
 
 // The block maxima of one reduction CTA (warp shuffles, then the warp maxima in shared memory),
 // combined across CTAs by atomic maxima in the control block; the last CTA (a last-block
