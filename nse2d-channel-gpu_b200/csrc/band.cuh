@@ -34,7 +34,8 @@ template <int M> struct Band {
     static constexpr int R0 = band_plan<M>::R(0);
     static constexpr int NB0 = M / R0;                       // pass-0 butterflies of a row
     static constexpr int TPR = M <= 128 ? 32 : 64;           // threads of a row group
-    static constexpr int ROW = M + (M >> ip_shift_a(M)) + (M >> ip_shift_b(M)) + 1;   // elements of a row buffer: 0 .. M, padded
+    // elements of a row buffer: 0 .. M, padded; even, so that what follows the buffers is 16-byte aligned in FP32 too
+    static constexpr int ROW = (M + (M >> ip_shift_a(M)) + (M >> ip_shift_b(M)) + 2) & ~1;
     static constexpr int RMAX = M <= 256 ? 6 : 4;            // rows of a band of k_band (M <= 512)
     static constexpr int MAXT = (RMAX + 2) * TPR;
     static constexpr int ROWS_G = 4;                         // row groups per CTA of the transforms alone
@@ -77,9 +78,6 @@ template <typename T> struct BandParams {
     double psi_bot, psi_top;     // psi on the walls (FP32: 0)
     double wall_bot, wall_top;   // FP32: the constant part of the wall vorticity
 };
-
-// filled by the launchers
-BandParams<double> band_params64(const Context* c);
 
 template <int TPR> __device__ __forceinline__ void row_sync(int group) {
     if constexpr (TPR == 32) __syncwarp();

@@ -157,6 +157,7 @@ struct Context {
     CUtensorMap tm_hat{}, tm_cp{};
     // precision 32: the FP32 spectral buffer [Ny][Hp] and the cluster solve's map and sizes for it
     cpx<float>* hat32 = nullptr;
+    cpx<float>* hat32b = nullptr;  // its psi-hat, where bands are used (as hat2)
     CUtensorMap tm_hat32{};
     size_t tc_smem32 = 0;
     int tc_nclusters32 = 0;
@@ -171,7 +172,7 @@ struct Context {
     float *wf = nullptr, *w1f = nullptr, *w2f = nullptr, *psif = nullptr, *rhsf = nullptr;
     double *wbar = nullptr, *psibar = nullptr;
     float* rc32 = nullptr;                 // [RC32_N][Ny] row constants of the FP32 stage
-    cpx<float> *twf = nullptr, *wNf = nullptr;
+    cpx<float> *twf = nullptr, *twf_band = nullptr, *wNf = nullptr;
     double wall_bot32 = 0.0, wall_top32 = 0.0;
     int maxuv32_ctas = 0;          // resident CTAs of k_maxuv32 (occupancy x SMs)
     // FP32 stage kernel: TMA tensor maps of psi' and of the three w' buffers (Nx >= 256)

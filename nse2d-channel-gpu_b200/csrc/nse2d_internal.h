@@ -36,16 +36,21 @@ int launch_thomas(Context* c, cudaStream_t s, bool general = false);
 int launch_thomas_maps(Context* c, cudaStream_t s, bool homog = false);
 int launch_thomas_apply(Context* c, cudaStream_t s, bool homog = false);
 int launch_thomas_cluster(Context* c, cudaStream_t s, bool homog = false);
-// row-band kernels (band64.cu)
+// row-band kernels (band64.cu, band32.cu)
 bool band_rows_ok(int M);
 bool band_stage_ok(int M);
 int band_stage(Context* c, int stage, bool inv, double* w_in, const double* w_n, double* w_out, double* rhs_out,
                const double* closure, cudaStream_t s);
 int band_rows_fwd(Context* c, const double* src, int row0, int nrows, cudaStream_t s);
 int band_rows_inv(Context* c, double* psi, double* w, bool thom, bool advance, cudaStream_t s);
-// whole steps in one launch (steps64.cu): store: the stage-3 rhs never (0), in the last step (1), in every one (2)
+int band32_stage(Context* c, int stage, bool inv, float* w_in, const float* w_n, float* w_out, float* rhs_out, cudaStream_t s);
+int band32_rows_fwd(Context* c, const float* src, cudaStream_t s);
+int band32_rows_inv(Context* c, float* w, bool advance, cudaStream_t s);
+// whole steps in one launch: store: the stage-3 rhs never (0), in the last step (1), in every one (2)
 int steps_setup(Context* c);
 int launch_steps(Context* c, int nsteps, int run, int store, cudaStream_t s);
+int steps_setup32(Context* c);
+int launch_steps32(Context* c, int nsteps, int run, int store, cudaStream_t s);
 // learned closure (closure.cu)
 struct Cnn;
 int cnn_forward_psi(Cnn* n, const double* w, const double* psi, const double* a_node, double inv_dx, double inv_deta, double* tau,
@@ -71,6 +76,8 @@ int split32(Context* c, cudaStream_t s);
 int export32(Context* c, bool with_rhs, cudaStream_t s);
 int step32_impl(Context* c, cudaStream_t s, bool store_rhs, cudaEvent_t* ev);
 const char* step32_kernel_name(const Context* c, int k);
+bool band_step32(const Context* c);
+const char* band_step_kernel_name(const Context* c, int k, bool split);
 int launch_ifft_thom(Context* c, double* psi, double* w, int stage, bool do_thom, bool closure, cudaStream_t s,
                      bool advance = false, bool general = false);
 int launch_thom(Context* c, double* w, const double* psi, cudaStream_t s);

@@ -116,7 +116,7 @@ static ThomasClusterKernel thomas_cluster_kernel(int L, bool f32 = false) {
 // homog: the FP32-bulk step's solve, for psi' (zero on the walls) in the FP32 spectral buffer
 ThomasParams thomas_params(const Context* c, bool homog) {
     ThomasParams p{};
-    p.hat = c->hat; p.hat32 = c->hat32; p.out = c->hat2 ? c->hat2 : c->hat; p.out32 = c->hat32; p.cp = c->cp; p.asub = c->rt.asub; p.inv_csup = c->rt.inv_csup; p.csup = c->rt.csup;
+    p.hat = c->hat; p.hat32 = c->hat32; p.out = c->hat2 ? c->hat2 : c->hat; p.out32 = c->hat32b ? c->hat32b : c->hat32; p.cp = c->cp; p.asub = c->rt.asub; p.inv_csup = c->rt.inv_csup; p.csup = c->rt.csup;
     p.tconst = c->tconst; p.tmaps = c->tmaps; p.tblk = c->tblk; p.tbcarry = c->tbcarry; p.tcount = c->tcount;
     p.Nx = c->Nx; p.Ny = c->Ny; p.Hp = c->Hp; p.H = c->H; p.Ni = c->Ni;
     p.nseg = c->thomas_nseg; p.nsb = c->thomas_nsb;
@@ -492,7 +492,7 @@ int context_create(const Config& cfg, Context** out) {
             c->tc_nclusters32 = std::min(nclusters, c->Hp / TC_KX);
         }
     }
-    if (c->hat2 && steps_setup(c)) return fail();
+    if ((c->hat2 || c->hat32b) && steps_setup(c)) return fail();
     Ctl h{};
     h.t = 0.0; h.dt = cfg.dt_init; h.next_out = 1e300; h.next_snap = 1e300; h.next_diag = 1e300;
     if (cudaMemcpy(c->ctl, &h, sizeof(Ctl), cudaMemcpyHostToDevice) != cudaSuccess) { set_error("ctl upload"); return fail(); }
@@ -895,6 +895,21 @@ int enqueue_step_timed(Context* c, cudaStream_t s, cudaEvent_t* ev, bool store_r
     return step_impl(c, s, store_rhs, ev);
 }
 
+// Kernel k of a band step, after the max reduction; split: every stage ends with the inverse transform.
+const char* band_step_kernel_name(const Context* c, int k, bool split) {
+    const int nt = thomas_launches(c);
+    for (int st = 1; st <= 3 && k >= 0; ++st) {
+        if (k == 0) return st > 1 && !split ? "k_band_inv_stage_fwd" : "k_band_stage_fwd";
+        if (k <= nt) return thomas_kernel_name(c, k - 1);
+        k -= 1 + nt;
+        if (st == 3 || split) {
+            if (k == 0) return "k_rows_inv";
+            --k;
+        }
+    }
+    return "";
+}
+
 // Names of the kernels of one step, in launch order (for the timed step).
 const char* step_kernel_name(const Context* c, int k) {
     if (c->prec32) return step32_kernel_name(c, k);
@@ -902,19 +917,7 @@ const char* step_kernel_name(const Context* c, int k) {
         if (k == 0) return "k_maxuv_dt";
         --k;
     }
-    if (band_step(c)) {
-        const int nt = thomas_launches(c);
-        for (int st = 1; st <= 3 && k >= 0; ++st) {
-            if (k == 0) return st > 1 && !band_split(c) ? "k_band_inv_stage_fwd" : "k_band_stage_fwd";
-            if (k <= nt) return thomas_kernel_name(c, k - 1);
-            k -= 1 + nt;
-            if (st == 3 || band_split(c)) {
-                if (k == 0) return "k_rows_inv";
-                --k;
-            }
-        }
-        return "";
-    }
+    if (band_step(c)) return band_step_kernel_name(c, k, band_split(c));
     const int per = 3 + thomas_launches(c);
     if (k < 0 || k >= 3 * per) return "";
     const int i = k % per;
@@ -925,7 +928,7 @@ const char* step_kernel_name(const Context* c, int k) {
 }
 
 int launches_per_step(const Context* c) {
-    if (c->prec32) return (c->cfg.adapt ? 1 : 0) + 3 * (3 + thomas_launches(c));
+    if (c->prec32) return (c->cfg.adapt ? 1 : 0) + (band_step32(c) ? 3 * (1 + thomas_launches(c)) + 1 : 3 * (3 + thomas_launches(c)));
     if (band_step(c)) return (c->cfg.adapt ? 1 : 0) + 3 * (1 + thomas_launches(c)) + (band_split(c) ? 3 : 1);
     return (c->cfg.adapt && !fused_max(c) ? 1 : 0) + 3 * (3 + thomas_launches(c));
 }
@@ -940,7 +943,7 @@ int refresh_maxima(Context* c, cudaStream_t s) {
 // Steps in one launch (steps.cuh): where the grid's bands are all resident, without a model between the stages, and
 // not into a stream that is being captured (nor inside an ensemble, whose members share the device).
 static bool steps_ok(const Context* c, cudaStream_t s) {
-    if (!c->steps_R || !band_step(c) || c->closure_net) return false;
+    if (!c->steps_R || !(c->prec32 ? band_step32(c) : band_step(c)) || c->closure_net) return false;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
         cudaGetLastError();

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "nse2d_internal.h"
+#include "band_fft.cuh"
 #include "bulk32.cuh"
 
 namespace nse2d {
@@ -41,7 +42,11 @@ int setup32(Context* c) {
     wN[M] = {-1.f, 0.f};
     if (M % 2 == 0) wN[M / 2] = {0.f, -1.f};
     p16_twiddle_table(M, full.data(), tw);
-    if (alloc(&c->twf, tw.size()) || alloc(&c->wNf, wN.size())) return -1;
+    std::vector<cpx<float>> tw_band;
+    plan_twiddle_table(M, band_radix_bits(M), full.data(), tw_band);
+    if (alloc(&c->twf, tw.size()) || alloc(&c->twf_band, tw_band.size()) || alloc(&c->wNf, wN.size())) return -1;
+    if (band_stage_ok(M) && alloc(&c->hat32b, (size_t)c->Ny * c->Hp)) return -1;
+    NSE_CUDA_TRY(cudaMemcpy(c->twf_band, tw_band.data(), tw_band.size() * sizeof(tw[0]), cudaMemcpyHostToDevice));
     NSE_CUDA_TRY(cudaMemcpy(c->twf, tw.data(), tw.size() * sizeof(tw[0]), cudaMemcpyHostToDevice));
     NSE_CUDA_TRY(cudaMemcpy(c->wNf, wN.data(), wN.size() * sizeof(wN[0]), cudaMemcpyHostToDevice));
     int per_sm = 0;
@@ -73,7 +78,7 @@ int setup32(Context* c) {
 
 void destroy32(Context* c) {
     for (void* p : {(void*)c->wf, (void*)c->w1f, (void*)c->w2f, (void*)c->psif, (void*)c->rhsf, (void*)c->wbar,
-                    (void*)c->psibar, (void*)c->rc32, (void*)c->twf, (void*)c->wNf, (void*)c->hat32})
+                    (void*)c->psibar, (void*)c->rc32, (void*)c->twf, (void*)c->twf_band, (void*)c->wNf, (void*)c->hat32, (void*)c->hat32b})
         if (p) cudaFree(p);
 }
 
@@ -122,6 +127,7 @@ static Fft32Params fft32_params(Context* c) {
     return p;
 }
 
+// rows of 64 to 2048 points have the row-band transforms
 template <int M> static int fft32_fwd_t(Context* c, Fft32Params& p, cudaStream_t s) {
     const size_t sm = fft32_smem_bytes(M);
     NSE_CUDA_TRY(cudaFuncSetAttribute(k_fft_fwd32<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -141,21 +147,20 @@ template <int M> static int fft32_inv_t(Context* c, Fft32Params& p, cudaStream_t
     switch (c->M) {                                                                \
         case 2: return FN<2>(c, p, s);       case 4: return FN<4>(c, p, s);        \
         case 8: return FN<8>(c, p, s);       case 16: return FN<16>(c, p, s);      \
-        case 32: return FN<32>(c, p, s);     case 64: return FN<64>(c, p, s);      \
-        case 128: return FN<128>(c, p, s);   case 256: return FN<256>(c, p, s);    \
-        case 512: return FN<512>(c, p, s);   case 1024: return FN<1024>(c, p, s);  \
         case 2048: return FN<2048>(c, p, s); case 4096: return FN<4096>(c, p, s);  \
         case 8192: return FN<8192>(c, p, s);                                       \
         default: set_error("no FFT kernel for M = %d", c->M); return -1;           \
     }
 
 static int fft32_fwd(Context* c, const float* src, cudaStream_t s) {
+    if (band_rows_ok(c->M)) return band32_rows_fwd(c, src, s);
     Fft32Params p = fft32_params(c);
     p.src = src;
     NSE_FFT32_DISPATCH(fft32_fwd_t)
 }
 
 static int fft32_inv(Context* c, float* w_out, bool advance, cudaStream_t s) {
+    if (band_rows_ok(c->M)) return band32_rows_inv(c, w_out, advance, s);
     Fft32Params p = fft32_params(c);
     p.psi = c->psif;
     p.w = w_out;
@@ -163,6 +168,8 @@ static int fft32_inv(Context* c, float* w_out, bool advance, cudaStream_t s) {
     p.advance = advance ? 1 : 0;
     NSE_FFT32_DISPATCH(fft32_inv_t)
 }
+
+bool band_step32(const Context* c) { return band_stage_ok(c->M) && !c->plain_step; }
 
 int step32_impl(Context* c, cudaStream_t s, bool store_rhs, cudaEvent_t* ev) {
     int k = 0;
@@ -186,7 +193,16 @@ int step32_impl(Context* c, cudaStream_t s, bool store_rhs, cudaEvent_t* ev) {
         if (launch_step_kernel(c, k_maxuv32, dim3(grid), dim3(256), 0, s, nullptr, q) || mark()) return -1;
     }
     float* wst[3] = {c->w1f, c->w2f, c->wf};
-    const float* win[3] = {c->wf, c->w1f, c->w2f};
+    float* win[3] = {c->wf, c->w1f, c->w2f};
+    if (band_step32(c)) {                                // per stage one launch of rows and one solve (band.cuh)
+        for (int st = 1; st <= 3; ++st) {
+            if (band32_stage(c, st, st > 1, win[st - 1], c->wf, wst[st - 1], (store_rhs && st == 3) ? c->rhsf : nullptr, s) || mark())
+                return -1;
+            for (int i = 0; i < thomas_launches(c); ++i)
+                if (launch_thomas_part(c, i, s, true) || mark()) return -1;
+        }
+        return band32_rows_inv(c, c->wf, true, s) || mark() ? -1 : 0;
+    }
     const dim3 grid((c->Nx + ST_TX - 1) / ST_TX, (c->Ny + ST_TY - 1) / ST_TY);
     for (int st = 1; st <= 3; ++st) {
         Stage32Params sp{};
@@ -219,6 +235,7 @@ const char* step32_kernel_name(const Context* c, int k) {
         if (k == 0) return "k_maxuv32";
         --k;
     }
+    if (band_step32(c)) return band_step_kernel_name(c, k, false);
     const int per = 3 + thomas_launches(c);
     if (k < 0 || k >= 3 * per) return "";
     const int i = k % per;

@@ -46,3 +46,57 @@ def test_band_step_gives_the_plain_step_and_solve_the_oracle(nse, oracle, cuda, 
     assert relerr(pd.cpu().numpy(), oracle.poisson_solve(w, 2 * np.pi, m, 0.0, 2.0)) < 1e-12
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("Nx,Ny", [(64, 5), (64, 37), (128, 150), (256, 66), (256, 301), (512, 9), (512, 301), (512, 650), (1024, 300),
+                                   (1024, 514), (2048, 40)])
+def test_fp32_band_step_gives_the_plain_step(nse, cuda, Nx, Ny):
+    """The FP32-bulk step by bands and in one launch against the one by separate kernels: the same bits; and the same
+    steps through nse2d_run."""
+    cfg = dict(Nx=Nx, Ny=Ny, Lx=2 * np.pi, stretch=1, beta=1.5, Ub=1.0, Reb=2000.0, F0=0.05, nforce=4, lin_drag=1e-3, adapt=1, precision=32)
+    a, b, c = (nse.Solver(**cfg) for _ in range(3))
+    w0 = laminar_perturbed(Nx, Ny, a.metric(0), seed=Nx + Ny, amp=2e-2)
+    for s in (a, b, c):
+        s.set_omega(w0)
+    ms = [ctypes.c_double() for _ in range(3)]
+    a.step(2, use_graph=True)
+    a.step_store_rhs(1)
+    for _ in range(3):
+        assert b.lib.nse2d_step_profiled(b.h, *[ctypes.byref(x) for x in ms], None) == 0
+    assert c.run(max_steps=3) == nse.HALT_BUDGET
+    rhs = np.empty((2, Ny, Nx))
+    for s in (b, c):
+        assert a.time() == s.time()
+        assert all(np.array_equal(x, y) for x, y in zip(a.fields(), s.fields()))
+        for q, out in zip((a, s), rhs):
+            assert q.lib.nse2d_get_field(q.h, 4, out.ctypes.data_as(ctypes.c_void_p), None) == 0
+        assert np.array_equal(rhs[0], rhs[1])
+    assert np.all(np.isfinite(a.fields()[0]))
+    for s in (a, b, c):
+        s.close()
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_steps_in_one_launch_follow_the_schedule(nse, cuda, precision):
+    """Many steps in one launch, runs to an output time and single steps give the same dt, times and fields as steps
+    one at a time (whose dt is trimmed and snapped to the same schedule)."""
+    cfg = dict(Nx=128, Ny=70, Lx=2 * np.pi, stretch=1, beta=1.5, Ub=1.0, Reb=2000.0, F0=0.05, nforce=4, lin_drag=1e-3, adapt=1,
+               precision=precision)
+    a, b = nse.Solver(**cfg), nse.Solver(**cfg)
+    w0 = laminar_perturbed(128, 70, a.metric(0), seed=3, amp=2e-2)
+    for s in (a, b):
+        s.set_omega(w0)
+    a.step(7)
+    for _ in range(7):
+        b.step(1)
+    assert a.time() == b.time()
+    t, dt = a.time()[:2]
+    t_out = t + 12.3 * dt
+    assert a.run(next_snap=t_out) & nse.HALT_OUTPUT
+    b.set_schedule(t_out, 1e300)
+    while b.time()[0] < t_out:
+        b.step(1)
+    assert a.time() == b.time() and a.time()[0] == t_out
+    assert all(np.array_equal(x, y) for x, y in zip(a.fields(), b.fields()))
+    a.close()
+    b.close()
