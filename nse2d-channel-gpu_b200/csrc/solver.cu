@@ -393,6 +393,11 @@ int context_create(const Config& cfg, Context** out) {
             return fail();
         }
     }
+    if (cudaFuncSetAttribute(k_thomas_wide<4, 8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve_wide_smem<4, 8>()) != cudaSuccess ||
+        cudaFuncSetAttribute(k_thomas_wide<4, 8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve_wide_smem<4, 8>()) != cudaSuccess) {
+        set_error("k_thomas_wide cannot be resident: %s", cudaGetErrorString(cudaGetLastError()));
+        return fail();
+    }
     // one-pass cluster solve when a cluster of at most 8 CTAs holds every interior row in
     // registers (at most 32 x 16 rows per CTA) and such clusters can be resident; otherwise the
     // two-pass form
@@ -764,11 +769,19 @@ template <bool F32> static ThomasCtaKernel thomas_cta_kernel(int kx, int L) {
     if (kx == 2) return L == 1 ? k_thomas_cta<2, 1, F32> : (L == 2 ? k_thomas_cta<2, 2, F32> : k_thomas_cta<2, 4, F32>);
     return L == 1 ? k_thomas_cta<4, 1, F32> : (L == 2 ? k_thomas_cta<4, 2, F32> : (L == 4 ? k_thomas_cta<4, 4, F32> : k_thomas_cta<4, 8, F32>));
 }
-static bool thomas_cta(const Context* c) { return c->Ni <= SC_MAX_NI; }
+static bool thomas_cta(const Context* c) { return c->Ni <= SC_WIDE_MAX_NI; }
 static int launch_thomas_cta(Context* c, cudaStream_t s, bool homog) {
-    const int kx = solve_kx(c->H, c->num_sms), L = solve_L(c->Ni, kx);
-    return launch_step_kernel(c, homog ? thomas_cta_kernel<true>(kx, L) : thomas_cta_kernel<false>(kx, L), dim3((c->H + kx - 1) / kx),
-                              dim3(SC_NT), 0, s, nullptr, thomas_params(c, homog));
+    const int kx = solve_kx(c->H, c->num_sms);
+    const dim3 grid((c->H + kx - 1) / kx);
+    if (c->Ni > SC_MAX_NI) {
+        const size_t smem = kx == 2 ? solve_wide_smem<2, 4>() : solve_wide_smem<4, 8>();
+        ThomasCtaKernel k = kx == 2 ? (homog ? k_thomas_wide<2, 4, true> : k_thomas_wide<2, 4, false>)
+                                    : (homog ? k_thomas_wide<4, 8, true> : k_thomas_wide<4, 8, false>);
+        return launch_step_kernel(c, k, grid, dim3(SC_WIDE_NT), smem, s, nullptr, thomas_params(c, homog));
+    }
+    const int L = solve_L(c->Ni, kx);
+    return launch_step_kernel(c, homog ? thomas_cta_kernel<true>(kx, L) : thomas_cta_kernel<false>(kx, L), grid, dim3(SC_NT), 0, s, nullptr,
+                              thomas_params(c, homog));
 }
 
 // Launches of one tridiagonal solve: 1 (one-CTA or cluster form) or 2 (maps, apply); part i of them.

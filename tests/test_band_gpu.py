@@ -100,3 +100,28 @@ def test_steps_in_one_launch_follow_the_schedule(nse, cuda, precision):
     assert all(np.array_equal(x, y) for x, y in zip(a.fields(), b.fields()))
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("Nx,Ny", [(64, 515), (512, 1026), (1024, 515), (1024, 777), (1024, 1026), (2048, 520), (64, 1027)])
+def test_solve_of_tall_columns(nse, oracle, cuda, Nx, Ny):
+    """The one-CTA tridiagonal solve of 513 to 1024 interior rows (two or four columns a CTA) and the first grid
+    beyond it: the Poisson solve against the oracle at the 1e-12 of the other solves, an FP32-bulk step against the
+    FP64 one at the 1e-5 of its psi."""
+    from test_fp32_gpu import omega0, rel
+    torch = cuda
+    cfg = dict(Nx=Nx, Ny=Ny, Lx=2 * np.pi, stretch=1, beta=1.5, Ub=1.0, Reb=2000.0, adapt=1)
+    a, b = nse.Solver(**cfg), nse.Solver(precision=32, **cfg)
+    m = oracle.metrics(Nx, Ny, 2 * np.pi, 1.0, 1, 1.5)
+    w = np.random.default_rng(Nx * Ny).standard_normal((Ny, Nx))
+    wd = torch.from_numpy(w).cuda()
+    pd = torch.zeros_like(wd)
+    a.poisson_solve(wd, pd)
+    torch.cuda.synchronize()
+    assert relerr(pd.cpu().numpy(), oracle.poisson_solve(w, 2 * np.pi, m, 0.0, 2.0)) < 1e-12
+    w0 = omega0(Nx, Ny, a.metric(0))
+    for s in (a, b):
+        s.set_omega(w0)
+        s.step(1)
+    assert rel(b.fields()[1], a.fields()[1]) < 1e-5
+    a.close()
+    b.close()
