@@ -43,7 +43,7 @@ constexpr int CN_LAYERS = 4;
 constexpr int CN_CIN = 5;                 // omega, psi, u, v, y
 constexpr int CN_C0 = 8;                  // channels of the stored input (padded: 16 bytes a pixel)
 constexpr int CN_NT = 256;
-constexpr int CN_OUT_PX = 1024;           // pixels per block of the output layer's weight gradient
+constexpr int CN_OUT_PX = 512;           // pixels per block of the output layer's weight gradient
 
 int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
@@ -68,6 +68,7 @@ struct Cnn {
     float* dz[2] = {};                    // dZ of two layers [Ppad][hidden]
     __nv_bfloat16* dzb[2] = {};           // the same in BF16
     float* dz_out = nullptr;              // dZ of the output layer [Ppad]
+    int sms = 0;                          // SMs of the device
     int wg_blocks = 0;                    // blocks of the weight-gradient reductions
     float* part = nullptr;                // their partials
     float* lpart = nullptr;               // loss partials [ceil(Ppad / CN_NT)]
@@ -275,7 +276,7 @@ __global__ void __launch_bounds__(CN_NT) k_wgrad_out(const __nv_bfloat16* h, con
             const int c = lane + 32 * g;
             if (c >= C) continue;
             const __nv_bfloat16* hp = h + (size_t)p0 * C + c;
-#pragma unroll 8
+#pragma unroll 16
             for (int k = 0; k < n; ++k) {
                 const float x = __bfloat162float(hp[(size_t)k * C]);
                 const float4* v = reinterpret_cast<const float4*>(sd[warp][k]);
@@ -385,23 +386,47 @@ int export_layer(Cnn* n, int l, cudaStream_t s) {
     return 0;
 }
 
-template <int C, int MODE> int conv_t(const ConvParams& p, bool setup, cudaStream_t s) {
+// a CTA's strip: up to 128 columns, two rows, or one while the strips do not fill the device twice (32 channels, 264192
+// pixels, us with one, two and four rows: forward 47, 37, 38; input gradient 52, 44, 50)
+void conv_strip(ConvParams& p, int sms) {
+    const int sx = (p.Nx + 127) / 128, nb = p.P / (p.Nx * p.Ny);
+    p.W = (p.Nx + sx - 1) / sx;
+    p.R = 2;
+    while (p.R > 1 && (long long)nb * sx * ((p.Ny + p.R - 1) / p.R) < 2 * sms) p.R /= 2;
+}
+template <int C, int MODE> int conv_t(ConvParams p, int sms, bool setup, cudaStream_t s) {
     if (setup) {
-        NSE_CUDA_TRY(cudaFuncSetAttribute(k_conv<C, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cv_smem_bytes<C>(64)));
+        NSE_CUDA_TRY(cudaFuncSetAttribute(k_conv<C, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)cv_smem_bytes<C>(64, 128, 2)));
         return 0;
     }
-    k_conv<C, MODE><<<(p.P + TG_BM - 1) / TG_BM, CV_NT, cv_smem_bytes<C>(p.N), s>>>(p);
+    conv_strip(p, sms);
+    const int blocks = p.P / (p.Nx * p.Ny) * ((p.Nx + p.W - 1) / p.W) * ((p.Ny + p.R - 1) / p.R);
+    k_conv<C, MODE><<<blocks, CV_NT, cv_smem_bytes<C>(p.N, p.W, p.R), s>>>(p);
     NSE_CUDA_TRY(cudaGetLastError());
     return 0;
 }
-// a convolution of C input channels (8: the input layer); setup: only the kernel's shared-memory limit
-template <int MODE> int conv(const ConvParams& p, int C, bool setup, cudaStream_t s) {
-    if constexpr (MODE == CV_FWD) if (C == CN_C0) return conv_t<CN_C0, MODE>(p, setup, s);
+// the input layer
+int conv_in(const ConvParams& p, cudaStream_t s) {
+    const int blocks = (p.P + TG_BM - 1) / TG_BM;
+    const size_t sm = cv_in_smem_bytes(p.N);
+    switch (p.N) {
+        case 16: k_conv_in<16><<<blocks, CV_NT, sm, s>>>(p); break;
+        case 32: k_conv_in<32><<<blocks, CV_NT, sm, s>>>(p); break;
+        case 48: k_conv_in<48><<<blocks, CV_NT, sm, s>>>(p); break;
+        case 64: k_conv_in<64><<<blocks, CV_NT, sm, s>>>(p); break;
+        default: set_error("no input convolution to %d channels", p.N); return -1;
+    }
+    NSE_CUDA_TRY(cudaGetLastError());
+    return 0;
+}
+// a convolution of C input channels; setup: only the kernel's shared-memory limit
+template <int MODE> int conv(const ConvParams& p, int C, int sms, bool setup, cudaStream_t s) {
     switch (C) {
-        case 16: return conv_t<16, MODE>(p, setup, s);
-        case 32: return conv_t<32, MODE>(p, setup, s);
-        case 48: return conv_t<48, MODE>(p, setup, s);
-        case 64: return conv_t<64, MODE>(p, setup, s);
+        case 16: return conv_t<16, MODE>(p, sms, setup, s);
+        case 32: return conv_t<32, MODE>(p, sms, setup, s);
+        case 48: return conv_t<48, MODE>(p, sms, setup, s);
+        case 64: return conv_t<64, MODE>(p, sms, setup, s);
         default: set_error("no convolution of %d channels", C); return -1;
     }
 }
@@ -478,18 +503,18 @@ static int cnn_forward_batch(Cnn* n, const PackSrc& src, const PackUv* uv, bool 
     for (int l = 0; l < CN_LAYERS; ++l) {
         const bool last = (l == CN_LAYERS - 1);
         ConvParams p{};
-        p.h = n->h[l]; p.W = n->wbf[l]; p.bias = n->b32[l]; p.err = n->err;
+        p.h = n->h[l]; p.wt = n->wbf[l]; p.bias = n->b32[l]; p.err = n->err;
         p.Nx = n->Nx; p.Ny = n->Ny; p.P = n->P; p.N = n->npad[l]; p.ldw = n->K[l];
         if (last) {
             p.z = tau ? nullptr : n->z[l];
             p.tau = tau;
             p.wall_rows = n->wall_rows;
             p.ts = n->out_tau * n->gain;
-            if (conv<CV_OUT>(p, n->cin[l], false, s)) return -1;
+            if (conv<CV_OUT>(p, n->cin[l], n->sms, false, s)) return -1;
         } else {
             p.z = keep ? n->z[l] : nullptr;
             p.hn = n->h[l + 1];
-            if (conv<CV_FWD>(p, l == 0 ? CN_C0 : n->cin[l], false, s)) return -1;
+            if (l == 0 ? conv_in(p, s) : conv<CV_FWD>(p, n->cin[l], n->sms, false, s)) return -1;
         }
     }
     return 0;
@@ -552,9 +577,9 @@ static int cnn_backward(Cnn* n, const double* tau, cudaStream_t s) {
         NSE_CUDA_TRY(fold(l, nwb, nk, H));
         if (l == 0) break;
         ConvParams p{};
-        p.h = n->dzb[cur]; p.W = n->wtbf[l]; p.zprev = n->z[l - 1]; p.z = n->dz[cur ^ 1]; p.hn = n->dzb[cur ^ 1]; p.err = n->err;
+        p.h = n->dzb[cur]; p.wt = n->wtbf[l]; p.zprev = n->z[l - 1]; p.z = n->dz[cur ^ 1]; p.hn = n->dzb[cur ^ 1]; p.err = n->err;
         p.Nx = n->Nx; p.Ny = n->Ny; p.P = n->P; p.N = n->cin[l]; p.ldw = 9 * n->npad[l];
-        if (conv<CV_DGRAD>(p, n->npad[l], false, s)) return -1;
+        if (conv<CV_DGRAD>(p, n->npad[l], n->sms, false, s)) return -1;
         cur ^= 1;
     }
     return 0;
@@ -613,7 +638,8 @@ static int cnn_create(int Nx, int Ny, int hidden, int max_batch, const double* y
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int H = n->npad[0];
-    n->wg_blocks = 2 * (sms > 0 ? sms : 148);                       // resident CTAs of k_wgrad
+    n->sms = sms > 0 ? sms : 148;
+    n->wg_blocks = 2 * n->sms;                       // resident CTAs of k_wgrad
     auto fail = [&]() { cnn_free(n); return -1; };
     for (int l = 0; l < CN_LAYERS; ++l) {
         const size_t nw = (size_t)n->npad[l] * n->K[l];
@@ -639,9 +665,9 @@ static int cnn_create(int Nx, int Ny, int hidden, int max_batch, const double* y
         ConvParams p{};
         bool bad = false;
         p.N = H;
-        bad |= conv<CV_FWD>(p, CN_C0, true, 0) || conv<CV_FWD>(p, H, true, 0) || conv<CV_DGRAD>(p, H, true, 0);
+        bad |= conv<CV_FWD>(p, H, 0, true, 0) || conv<CV_DGRAD>(p, H, 0, true, 0);
         p.N = n->npad[CN_LAYERS - 1];
-        bad |= conv<CV_OUT>(p, H, true, 0) != 0;
+        bad |= conv<CV_OUT>(p, H, 0, true, 0) != 0;
         bad |= wgrad(WgradParams{}, true, H, 0, true, 0) || wgrad(WgradParams{}, false, H, 0, true, 0);
         if (bad) return fail();
     }

@@ -33,3 +33,10 @@ def test_edges_match_the_oracle(nse, cuda, Nx, Ny, H, idx):
         gw, gb = net.get_grads(layer)
         assert _rel(gw, ref_grads[layer][0]) < 3e-2, (layer, _rel(gw, ref_grads[layer][0]))
         assert _rel(gb, ref_grads[layer][1]) < 3e-2, (layer, _rel(gb, ref_grads[layer][1]))
+
+
+@pytest.mark.parametrize("Nx,Ny,H,idx", [(256, 6, 16, (0, 2)), (130, 7, 32, (1,)), (64, 130, 32, (0, 1, 2, 3)), (66, 40, 64, (3, 0)),
+                                         (128, 150, 48, (1, 2)), (8, 161, 16, (0, 1, 2, 3))])
+def test_strips_match_the_oracle(nse, cuda, Nx, Ny, H, idx):
+    """Strips of one, two and four rows, a row of one and of several strips, and tiles that run over the rows' ends."""
+    test_edges_match_the_oracle(nse, cuda, Nx, Ny, H, idx)
