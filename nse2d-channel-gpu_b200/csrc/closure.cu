@@ -112,6 +112,7 @@ struct PackUv {
 };
 template <bool UV>
 __global__ void k_pack_input(PackSrc q, PackUv g, __nv_bfloat16* h0, int nxy, int Nx, int Ny, int P) {
+    cv_wait_for_last_layer();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= P) return;
     const int b = p / nxy, r = p - b * nxy;
@@ -136,6 +137,7 @@ __global__ void k_pack_input(PackSrc q, PackUv g, __nv_bfloat16* h0, int nxy, in
 // the x-mean of tau on every row: one CTA per row
 __global__ void __launch_bounds__(CN_NT) k_unpack_row_mean(const float* z, double* tau, int Nx, int Ny, double ts, int wall_rows) {
     __shared__ double red[CN_NT];
+    cv_wait_for_last_layer();
     const int j = blockIdx.x;
     double sum = 0.0;
     for (int i = threadIdx.x; i < Nx; i += CN_NT) sum += (double)z[(size_t)j * Nx + i];
@@ -394,6 +396,18 @@ void conv_strip(ConvParams& p, int sms) {
     p.R = 2;
     while (p.R > 1 && (long long)nb * sx * ((p.Ny + p.R - 1) / p.R) < 2 * sms) p.R /= 2;
 }
+// A kernel that begins with cv_wait_for_last_layer, launched before the one before it has ended.
+template <typename... KArgs, typename... Args>
+int launch_layer(void (*kern)(KArgs...), int blocks, int threads, size_t smem, cudaStream_t s, Args&&... args) {
+    cudaLaunchConfig_t lc{};
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    lc.gridDim = dim3(blocks); lc.blockDim = dim3(threads); lc.dynamicSmemBytes = smem; lc.stream = s;
+    lc.attrs = &at; lc.numAttrs = 1;
+    NSE_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, std::forward<Args>(args)...));
+    return 0;
+}
 template <int C, int MODE> int conv_t(ConvParams p, int sms, bool setup, cudaStream_t s) {
     if (setup) {
         NSE_CUDA_TRY(cudaFuncSetAttribute(k_conv<C, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -402,23 +416,19 @@ template <int C, int MODE> int conv_t(ConvParams p, int sms, bool setup, cudaStr
     }
     conv_strip(p, sms);
     const int blocks = p.P / (p.Nx * p.Ny) * ((p.Nx + p.W - 1) / p.W) * ((p.Ny + p.R - 1) / p.R);
-    k_conv<C, MODE><<<blocks, CV_NT, cv_smem_bytes<C>(p.N, p.W, p.R), s>>>(p);
-    NSE_CUDA_TRY(cudaGetLastError());
-    return 0;
+    return launch_layer(k_conv<C, MODE>, blocks, CV_NT, cv_smem_bytes<C>(p.N, p.W, p.R), s, p);
 }
 // the input layer
 int conv_in(const ConvParams& p, cudaStream_t s) {
     const int blocks = (p.P + TG_BM - 1) / TG_BM;
     const size_t sm = cv_in_smem_bytes(p.N);
     switch (p.N) {
-        case 16: k_conv_in<16><<<blocks, CV_NT, sm, s>>>(p); break;
-        case 32: k_conv_in<32><<<blocks, CV_NT, sm, s>>>(p); break;
-        case 48: k_conv_in<48><<<blocks, CV_NT, sm, s>>>(p); break;
-        case 64: k_conv_in<64><<<blocks, CV_NT, sm, s>>>(p); break;
+        case 16: return launch_layer(k_conv_in<16>, blocks, CV_NT, sm, s, p);
+        case 32: return launch_layer(k_conv_in<32>, blocks, CV_NT, sm, s, p);
+        case 48: return launch_layer(k_conv_in<48>, blocks, CV_NT, sm, s, p);
+        case 64: return launch_layer(k_conv_in<64>, blocks, CV_NT, sm, s, p);
         default: set_error("no input convolution to %d channels", p.N); return -1;
     }
-    NSE_CUDA_TRY(cudaGetLastError());
-    return 0;
 }
 // a convolution of C input channels; setup: only the kernel's shared-memory limit
 template <int MODE> int conv(const ConvParams& p, int C, int sms, bool setup, cudaStream_t s) {
@@ -532,8 +542,8 @@ static int cnn_forward_field(Cnn* n, const PackSrc& src, const PackUv* uv, doubl
     set_batch(n, 1);
     if (cnn_forward_batch(n, src, uv, false, n->row_mean ? nullptr : tau, s)) return -1;
     if (n->row_mean) {
-        k_unpack_row_mean<<<n->Ny, CN_NT, 0, s>>>(n->z[CN_LAYERS - 1], tau, n->Nx, n->Ny, n->out_tau * n->gain, n->wall_rows);
-        NSE_CUDA_TRY(cudaGetLastError());
+        if (launch_layer(k_unpack_row_mean, n->Ny, CN_NT, 0, s, n->z[CN_LAYERS - 1], tau, n->Nx, n->Ny, n->out_tau * n->gain, n->wall_rows))
+            return -1;
     }
     return 0;
 }

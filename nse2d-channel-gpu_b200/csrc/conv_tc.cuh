@@ -73,6 +73,15 @@ template <int C> __host__ __device__ constexpr size_t cv_smem_bytes(int N, int W
     return (ab > st ? ab : st) + 128;
 }
 
+// The layers follow one another by programmatic launches: a kernel is launched when every CTA of the one before has
+// come past this wait, does what needs none of its results (its accumulators in TMEM, its weights) and waits here until
+// that one has ended. A kernel's accumulators are allocated before it lets the next one in, so the next never keeps
+// it from them. Five steps of 256x129 with the model before every stage: 765 us without, 635 with.
+__device__ __forceinline__ void cv_wait_for_last_layer() {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
 // 16 bytes to shared memory, zeros when !ok (the address is then not read)
 __device__ __forceinline__ void cv_cp16(uint32_t s, const void* g, bool ok) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(g), "r"(ok ? 16 : 0) : "memory");
@@ -210,6 +219,8 @@ static __global__ void __launch_bounds__(CV_NT) k_conv_in(ConvParams p) {
         const int n = e / NCH, kc = e - n * NCH;
         tg_cp16(sB + (uint32_t)((((n >> 3) * NCH + kc) << 7) + ((n & 7) << 4)), p.wt + (size_t)n * p.ldw + kc * 8);
     }
+    __syncthreads();                                                       // TMEM is allocated
+    cv_wait_for_last_layer();
     if (tid < 128) {
         unsigned short k[48];
         cv_gather5(p.h, cv_pix(m0 + tid, p.P, p.Nx, p.Ny), p.Nx, p.Ny, k);
@@ -265,6 +276,13 @@ static __global__ void __launch_bounds__(CV_NT) k_conv(ConvParams p) {
         tg_bar_init(&mma_bar);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
+    // B: core matrices of 8 rows x 16 bytes, [row group][k chunk]
+    for (int e = tid; e < N * NCH; e += CV_NT) {
+        const int n = e / NCH, kc = e - n * NCH;
+        tg_cp16(sB + (uint32_t)((((n >> 3) * NCH + kc) << 7) + ((n & 7) << 4)), p.wt + (size_t)n * p.ldw + kc * 8);
+    }
+    __syncthreads();                                                       // TMEM is allocated
+    cv_wait_for_last_layer();
     // the strip and its halo, [8 channels][position]: 8 consecutive positions are a core matrix of A wherever they begin
     for (int e = tid; e < (R + 2) * Wp * C8; e += CV_NT) {
         const int pos = e / C8, ch = e - pos * C8, pr = pos / Wp, j = j0 - 1 + pr;
@@ -272,11 +290,6 @@ static __global__ void __launch_bounds__(CV_NT) k_conv(ConvParams p) {
         i = i < 0 ? i + Nx : (i >= Nx ? i - Nx : i);
         const bool ok = j >= 0 && j < Ny;
         cv_cp16(sA + (uint32_t)(ch * plane + pos * 16), p.h + (ok ? (size_t)(base + j * Nx + i) * C + ch * 8 : 0), ok);
-    }
-    // B: core matrices of 8 rows x 16 bytes, [row group][k chunk]
-    for (int e = tid; e < N * NCH; e += CV_NT) {
-        const int n = e / NCH, kc = e - n * NCH;
-        tg_cp16(sB + (uint32_t)((((n >> 3) * NCH + kc) << 7) + ((n & 7) << 4)), p.wt + (size_t)n * p.ldw + kc * 8);
     }
     cv_mma_all(&mma_bar, p.err, [&]() {
         const uint32_t idesc = tg_idesc(N), tmem = tmem_base;
