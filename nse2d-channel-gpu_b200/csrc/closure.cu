@@ -615,13 +615,13 @@ bool cnn_matches(const Cnn* n, int Nx, int Ny) { return n && n->Nx == Nx && n->N
 void cnn_free(Cnn* n) {
     if (!n) return;
     for (int l = 0; l < CN_LAYERS; ++l) {
-        cudaFree(n->w32[l]); cudaFree(n->b32[l]); cudaFree(n->gw[l]); cudaFree(n->gb[l]);
+        cudaFree(n->w32[l]); cudaFree(n->gw[l]);          // each with its bias behind it
         cudaFree(n->mw[l]); cudaFree(n->vw[l]); cudaFree(n->mb[l]); cudaFree(n->vb[l]);
         cudaFree(n->wbf[l]); cudaFree(n->wtbf[l]); cudaFree(n->h[l]); cudaFree(n->z[l]);
     }
     for (int k = 0; k < 2; ++k) { cudaFree(n->dz[k]); cudaFree(n->dzb[k]); }
     cudaFree(n->dz_out); cudaFree(n->part); cudaFree(n->lpart);
-    cudaFree(n->loss); cudaFree(n->y); cudaFree(n->idx); cudaFree(n->err);
+    cudaFree(n->loss); cudaFree(n->y); cudaFree(n->idx);
     delete n;
 }
 
@@ -653,20 +653,23 @@ static int cnn_create(int Nx, int Ny, int hidden, int max_batch, const double* y
     auto fail = [&]() { cnn_free(n); return -1; };
     for (int l = 0; l < CN_LAYERS; ++l) {
         const size_t nw = (size_t)n->npad[l] * n->K[l];
-        if (cn_alloc(&n->w32[l], nw) || cn_alloc(&n->b32[l], n->npad[l]) || cn_alloc(&n->gw[l], nw) ||
-            cn_alloc(&n->gb[l], n->npad[l]) || cn_alloc(&n->mw[l], nw) || cn_alloc(&n->vw[l], nw) ||
+        // weights and biases, and their gradients, in one piece each: one copy takes a layer to the host
+        if (cn_alloc(&n->w32[l], nw + n->npad[l]) || cn_alloc(&n->gw[l], nw + n->npad[l]) || cn_alloc(&n->mw[l], nw) || cn_alloc(&n->vw[l], nw) ||
             cn_alloc(&n->mb[l], n->npad[l]) || cn_alloc(&n->vb[l], n->npad[l]) || cn_alloc(&n->wbf[l], nw) ||
             cn_alloc(&n->h[l], (size_t)Pmax * (l == 0 ? CN_C0 : n->cin[l])) ||
             cn_alloc(&n->z[l], (size_t)Pmax * (l == CN_LAYERS - 1 ? 1 : n->npad[l])))
             return fail();
+        n->b32[l] = n->w32[l] + nw;
+        n->gb[l] = n->gw[l] + nw;
         if (l >= 1 && l < CN_LAYERS - 1 && cn_alloc(&n->wtbf[l], (size_t)n->cin[l] * 9 * n->npad[l])) return fail();
     }
     for (int k = 0; k < 2; ++k)
         if (cn_alloc(&n->dz[k], (size_t)Pmax * H) || cn_alloc(&n->dzb[k], (size_t)Pmax * H)) return fail();
     const size_t npart = std::max((size_t)wgrad_blocks(n) * (9 * H + 1) * H, (size_t)((Pmax + CN_OUT_PX - 1) / CN_OUT_PX) * (9 * H + 1));
     if (cn_alloc(&n->dz_out, Pmax) || cn_alloc(&n->part, npart) || cn_alloc(&n->lpart, (size_t)(Pmax + CN_NT - 1) / CN_NT) ||
-        cn_alloc(&n->loss, 1) || cn_alloc(&n->y, Ny) || cn_alloc(&n->idx, max_batch) || cn_alloc(&n->err, 1))
+        cn_alloc(&n->loss, 2) || cn_alloc(&n->y, Ny) || cn_alloc(&n->idx, max_batch))
         return fail();
+    n->err = reinterpret_cast<int*>(n->loss + 1);                  // read with the loss
     if (cudaMemcpy(n->y, y_host, sizeof(double) * Ny, cudaMemcpyHostToDevice) != cudaSuccess) {
         set_error("nse2d_cnn_create: y upload");
         return fail();
@@ -773,29 +776,29 @@ int nse2d_cnn_set_params(nse2d_cnn* c, int layer, const float* w, const float* b
     return 0;
 }
 
-static int get_layer(Cnn* n, int layer, const float* dw, const float* db, float* w, float* b) {
+// dw: a layer's weights [npad][K] and, behind them, its biases
+static int get_layer(Cnn* n, int layer, const float* dw, float* w, float* b) {
     const int ci = layer == 0 ? CN_CIN : n->cout[layer - 1], co = n->cout[layer], K = n->K[layer], np = n->npad[layer];
-    std::vector<float> wp((size_t)np * K), bp(np);
+    std::vector<float> wp((size_t)np * (K + 1));
     NSE_CUDA_TRY(cudaDeviceSynchronize());
     NSE_CUDA_TRY(cudaMemcpy(wp.data(), dw, wp.size() * 4, cudaMemcpyDeviceToHost));
-    NSE_CUDA_TRY(cudaMemcpy(bp.data(), db, bp.size() * 4, cudaMemcpyDeviceToHost));
     for (int o = 0; o < co; ++o) {
         if (w)
             for (int tap = 0; tap < 9; ++tap)
                 for (int ch = 0; ch < ci; ++ch) w[((size_t)o * 9 + tap) * ci + ch] = wp[(size_t)o * K + tap * n->cin[layer] + ch];
-        if (b) b[o] = bp[o];
+        if (b) b[o] = wp[(size_t)np * K + o];
     }
     return 0;
 }
 
 int nse2d_cnn_get_params(nse2d_cnn* c, int layer, float* w, float* b) {
     if (!c || layer < 0 || layer >= CN_LAYERS) { set_error("nse2d_cnn_get_params: bad layer"); return -1; }
-    return get_layer(c->n, layer, c->n->w32[layer], c->n->b32[layer], w, b);
+    return get_layer(c->n, layer, c->n->w32[layer], w, b);
 }
 
 int nse2d_cnn_get_grads(nse2d_cnn* c, int layer, float* w, float* b) {
     if (!c || layer < 0 || layer >= CN_LAYERS) { set_error("nse2d_cnn_get_grads: bad layer"); return -1; }
-    return get_layer(c->n, layer, c->n->gw[layer], c->n->gb[layer], w, b);
+    return get_layer(c->n, layer, c->n->gw[layer], w, b);
 }
 
 int nse2d_cnn_set_scales(nse2d_cnn* c, const double* in_scales, double tau_scale) {
@@ -854,29 +857,49 @@ static int batch_setup(Cnn* n, const int* idx, int nb, cudaStream_t s) {
     return 0;
 }
 
-int nse2d_cnn_gradients(nse2d_cnn* c, const double* w, const double* psi, const double* u, const double* v,
-                        const double* tau, const int* idx, int nb, float* loss, cudaStream_t s) {
+// The forward and backward pass of a batch, without waiting for them.
+static int enqueue_gradients(nse2d_cnn* c, const double* w, const double* psi, const double* u, const double* v, const double* tau,
+                             const int* idx, int nb, cudaStream_t s) {
     if (!c || !w || !psi || !u || !v || !tau) { set_error("nse2d_cnn_gradients: null argument"); return -1; }
     Cnn* n = c->n;
     if (batch_setup(n, idx, nb, s)) return -1;
     const int rc = (cnn_forward_batch(n, pack_src(n, w, psi, u, v), nullptr, true, nullptr, s) || cnn_backward(n, tau, s)) ? -1 : 0;
     // slot 0 back to sample 0 for inference
-    const int zero = 0;
-    NSE_CUDA_TRY(cudaMemcpyAsync(n->idx, &zero, sizeof(int), cudaMemcpyHostToDevice, s));
+    NSE_CUDA_TRY(cudaMemsetAsync(n->idx, 0, sizeof(int), s));
+    return rc;
+}
+// the loss and the error flag, once the stream has come to them
+static int finish_gradients(Cnn* n, float* loss, int* err, cudaStream_t s) {
+    struct { float loss; int err; } r{};
+    static_assert(sizeof(r) == 8, "the flag lies behind the loss");
+    NSE_CUDA_TRY(cudaMemcpyAsync(&r, n->loss, sizeof(r), cudaMemcpyDeviceToHost, s));
     NSE_CUDA_TRY(cudaStreamSynchronize(s));
-    if (rc) return -1;
-    if (loss) NSE_CUDA_TRY(cudaMemcpy(loss, n->loss, sizeof(float), cudaMemcpyDeviceToHost));
+    if (loss) *loss = r.loss;
+    *err = r.err;
     return 0;
+}
+
+int nse2d_cnn_gradients(nse2d_cnn* c, const double* w, const double* psi, const double* u, const double* v,
+                        const double* tau, const int* idx, int nb, float* loss, cudaStream_t s) {
+    const int rc = enqueue_gradients(c, w, psi, u, v, tau, idx, nb, s);
+    if (rc) {
+        cudaStreamSynchronize(s);
+        return -1;
+    }
+    int e = 0;
+    return finish_gradients(c->n, loss, &e, s);
 }
 
 int nse2d_cnn_train_step(nse2d_cnn* c, const double* w, const double* psi, const double* u, const double* v,
                          const double* tau, const int* idx, int nb, float lr, float weight_decay, float* loss,
                          cudaStream_t s) {
-    if (nse2d_cnn_gradients(c, w, psi, u, v, tau, idx, nb, loss, s)) return -1;
+    if (enqueue_gradients(c, w, psi, u, v, tau, idx, nb, s)) {
+        cudaStreamSynchronize(s);
+        return -1;
+    }
     if (cnn_adamw(c->n, lr, weight_decay, s)) return -1;
-    NSE_CUDA_TRY(cudaStreamSynchronize(s));
     int e = 0;
-    NSE_CUDA_TRY(cudaMemcpy(&e, c->n->err, sizeof(int), cudaMemcpyDeviceToHost));
+    if (finish_gradients(c->n, loss, &e, s)) return -1;
     if (e) { set_error("nse2d_cnn_train_step: a tensor-core wait ran out"); return -1; }
     return 0;
 }
