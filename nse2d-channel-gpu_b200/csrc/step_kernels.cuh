@@ -673,6 +673,8 @@ __device__ __forceinline__ void fwd_last_pass_split(const cpx<T>* buf, const cpx
 // a row is read as M complex points z_n = x_2n + i x_2n+1, scattered by cp.async into the
 // digit-reversed layout; after the passes the split step writes X_k, k = 0..M:
 //   E_k = (Z_k + conj Z_{M-k}) / 2,  O_k = -i (Z_k - conj Z_{M-k}) / 2,  X_k = E_k + W_{2M}^k O_k.
+// The rows go from the last to the first: the stage before has just written the last ones, which are still in L2 on
+// grids whose fields are not (4096x2049, 67 MB a field: 27.7 -> 25.9 us; FP32 fields no change, first to last there).
 template <int M>
 static __global__ void __launch_bounds__(IP_NT, 5) k_fft_fwd(FftParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -680,7 +682,7 @@ static __global__ void __launch_bounds__(IP_NT, 5) k_fft_fwd(FftParams p) {
     cpx<double>* buf = reinterpret_cast<cpx<double>*>(smem_raw);
     const int je = p.row0 + p.nrows;
     constexpr int R0 = p16_plan<M>::R(0), NB0 = M / R0;
-    for (int j = p.row0 + blockIdx.x; j < je; j += gridDim.x) {      // rows strided over one wave of CTAs
+    for (int j = je - 1 - blockIdx.x; j >= p.row0; j -= gridDim.x) {  // rows strided over one wave of CTAs, last first
         const double2* row = reinterpret_cast<const double2*>(p.src + (size_t)j * p.Nx);
         // pass 0 from global: thread t transforms the points t + NB0 r (a coalesced column)
 #pragma unroll 1
@@ -1096,11 +1098,11 @@ static __global__ void __launch_bounds__(IP_NT, 3) k_fft_fwd_pf(FftParams p) {
         mbar_expect_tx(bar, FftPf<M>::row_bytes);
         bulk_load(const_cast<double2*>(stage), p.src + (size_t)j * p.Nx, FftPf<M>::row_bytes, bar);
     };
-    const int jfirst = p.row0 + blockIdx.x;
-    if (threadIdx.x == 0 && jfirst < je) issue(jfirst);
+    const int jfirst = je - 1 - blockIdx.x;            // the last rows first, as k_fft_fwd
+    if (threadIdx.x == 0 && jfirst >= p.row0) issue(jfirst);
     unsigned parity = 0;
     bool live = true;
-    for (int j = jfirst; j < je; j += gridDim.x) {
+    for (int j = jfirst; j >= p.row0; j -= gridDim.x) {
         if (live) {
             live = __syncthreads_and(mbar_wait_bounded(bar, parity));
             if (live) parity ^= 1u;
@@ -1120,9 +1122,9 @@ static __global__ void __launch_bounds__(IP_NT, 3) k_fft_fwd_pf(FftParams p) {
             for (int q = 0; q < 16; ++q) buf[ip_idx<M>(p0 + q)] = v[q];
         }
         __syncthreads();                               // pass 0 done: the staging buffer is free
-        if (threadIdx.x == 0 && live && j + (int)gridDim.x < je) {
+        if (threadIdx.x == 0 && live && j - (int)gridDim.x >= p.row0) {
             fence_proxy_async_smem();
-            issue(j + (int)gridDim.x);
+            issue(j - (int)gridDim.x);
         }
         p16_pass<double, M, 1, false, IP_NT>(buf, p.tw);
         __syncthreads();
