@@ -21,8 +21,10 @@ namespace nse2d {
     NSE_BAND512_DISPATCH(FN, __VA_ARGS__)
 
 template <typename T, int M, bool INV> int band_kernel_t(Context* c, BandParams<T>& p, cudaStream_t s) {
-    // rows per band: one band per SM while it fits, so that a launch is one wave
-    const int R = std::max(1, std::min(Band<M>::RMAX, (c->Ni + c->num_sms - 1) / c->num_sms));
+    // rows per band: one band per SM while it fits, so that a launch is one wave; the bands of channels that run
+    // together are counted together, since every band transforms two halo rows more than its own (an ensemble step of 4,
+    // 8 and 12 channels of 256 to 1024 points by 129 to 513 rows: 118, 139 and 210 us without, 111, 115 and 183 with it)
+    const int R = std::max(1, (int)std::min<long long>(Band<M>::RMAX, ((long long)c->Ni * c->band_share + c->num_sms - 1) / c->num_sms));
     const size_t sm = band_smem_bytes<T, M>(R);
     NSE_CUDA_TRY(cudaFuncSetAttribute(k_band<T, M, INV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)band_smem_bytes<T, M>(Band<M>::RMAX)));

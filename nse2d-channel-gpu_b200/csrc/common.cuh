@@ -105,6 +105,11 @@ struct RowTables {
     double* mms_s2k;
 };
 
+// Channels together that still step by bands. More of them fill the device, and the halo rows that bands transform
+// twice are then time lost (an ensemble step of 4, 8, 12, 16, 32 and 64 channels, us: FP64 bands 111, 115, 183, 188, 518
+// and 1054, separate kernels 116, 116, 182, 181, 506 and 976; FP32 88, 92, 141, 140, 398 and 808 against 92, 91, 131,
+// 127, 353 and 706).
+constexpr int kBandShareMax = 8;
 struct Context {
     Config cfg;
     int Nx = 0, Ny = 0, M = 0, H = 0, Hp = 0, Ni = 0;
@@ -125,6 +130,7 @@ struct Context {
     // otherwise psi-hat takes the place of omega-hat
     cpx<double>* hat2 = nullptr;
     bool band = false;             // row transforms of band.cuh: rows of 64 to 2048 points
+    int band_share = 1;            // channels that run at the same time as this one (the branches of an ensemble)
     int steps_R = 0;               // rows of a band of the steps in one launch (0: not used)
     bool plain_step = false;       // a step of separate transforms and stages (nse2d_step_profiled times them apart)
     double* cp = nullptr;          // elimination table [Ni][Hp]

@@ -72,7 +72,11 @@ int ensemble_build(Ensemble* e, int groups, bool force = false) {
     cudaEventRecord(ev[0], e->cap);                                   // fork
     for (int b = 0; b < groups && rc == 0; ++b) {
         cudaStreamWaitEvent(e->branch[b], ev[0], 0);
-        for (int i = b; i < n && rc == 0; i += groups) rc = enqueue_step(e->m[i], e->branch[b], false);
+        for (int i = b; i < n && rc == 0; i += groups) {
+            e->m[i]->band_share = groups;
+            rc = enqueue_step(e->m[i], e->branch[b], false);
+            e->m[i]->band_share = 1;
+        }
         cudaEventRecord(ev[1 + b], e->branch[b]);                     // join
         cudaStreamWaitEvent(e->cap, ev[1 + b], 0);
     }

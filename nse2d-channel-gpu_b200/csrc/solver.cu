@@ -844,7 +844,9 @@ int poisson_solve(Context* c, const double* w, double* psi, cudaStream_t s, bool
 
 // The steps that the row-band kernels take: without the MMS forcing and the wall-update bookkeeping of
 // closure_diag (verification runs and diagnostics of their own), which the separate kernels have.
-static bool band_step(const Context* c) { return c->band && band_stage_ok(c->M) && !c->cfg.mms && !c->closure_diag && !c->plain_step; }
+static bool band_step(const Context* c) {
+    return c->band && band_stage_ok(c->M) && !c->cfg.mms && !c->closure_diag && !c->plain_step && c->band_share <= kBandShareMax;
+}
 
 // A stage of the band step begins with the inverse transform, except stage 1 (psi is the step's) and,
 // with a model that runs before every stage, stages 2 and 3 (the model needs psi of the stage).

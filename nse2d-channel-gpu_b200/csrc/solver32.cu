@@ -169,7 +169,7 @@ static int fft32_inv(Context* c, float* w_out, bool advance, cudaStream_t s) {
     NSE_FFT32_DISPATCH(fft32_inv_t)
 }
 
-bool band_step32(const Context* c) { return band_stage_ok(c->M) && !c->plain_step; }
+bool band_step32(const Context* c) { return band_stage_ok(c->M) && !c->plain_step && c->band_share <= kBandShareMax; }
 
 int step32_impl(Context* c, cudaStream_t s, bool store_rhs, cudaEvent_t* ev) {
     int k = 0;

@@ -77,3 +77,29 @@ def test_tridiag_forms_agree(nse, cuda):
     assert np.max(np.abs(a.fields()[1] - b.fields()[1])) <= 1e-12 * np.max(np.abs(pa))
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("n", [2, 8, 9])
+def test_members_step_as_alone_however_many(nse, cuda, precision, n):
+    """Bands of the height that 2 and 8 channels together get, and the separate kernels that 9 take: the bits of the
+    channels alone."""
+    import numpy as np
+    grids = [(128, 129), (256, 70), (512, 65), (1024, 40), (64, 200), (256, 33), (1024, 129), (128, 60), (512, 130)][:n]
+    alone, members = [], []
+    for k, (Nx, Ny) in enumerate(grids):
+        pair = [nse.Solver(Nx=Nx, Ny=Ny, Lx=2 * np.pi, stretch=1, beta=1.5, Ub=1.0, Reb=2000.0, F0=0.05, nforce=4, adapt=1,
+                           precision=precision) for _ in range(2)]
+        rng = np.random.default_rng(k)
+        w0 = np.repeat((3.0 * pair[0].metric(0))[:, None], Nx, 1) + 1e-2 * rng.standard_normal((Ny, Nx))
+        for s in pair:
+            s.set_omega(w0)
+        alone.append(pair[0])
+        members.append(pair[1])
+    ens = nse.Ensemble(members)
+    ens.step(3)
+    for a, m in zip(alone, members):
+        a.step(3, use_graph=True)
+        assert a.time() == m.time()
+        assert all(np.array_equal(x, y) for x, y in zip(a.fields(), m.fields()))
+    ens.close()
