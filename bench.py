@@ -663,8 +663,8 @@ def run_ensemble(args):
                        "points": pts, "master_seed": ENSEMBLE_SEED, "branches": groups},
             "sequential": {"value": round(pts * K / (seq_ms * 1e-3), 1), "unit": "points/s",
                            "ms_per_step": round(seq_ms / K, 4),
-                           "how": "the same 64 channels with the same plans, each replaying its own one-step graph "
-                                  "K times, one after another"},
+                           "how": "the same 64 channels with the same plans, each taking its K steps, "
+                                  "one after another"},
             "speedup_vs_sequential": round(seq_ms / ens_ms, 3), "clocks": ck}
 
 

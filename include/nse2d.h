@@ -120,20 +120,24 @@ int  nse2d_get_field(nse2d_ctx* ctx, int which, double* host, cudaStream_t s);
 
 /* Advance nsteps SSPRK(3,3) steps, asynchronously. With adapt, dt is computed on the
  * device before every step (max |u|, |v|, |v| a, CFL and viscous limits, trimming to
- * the next output time); otherwise the dt of nse2d_set_dt / dt_init is used. use_graph:
- * replay one captured CUDA graph per step. */
+ * the next output time); otherwise the dt of nse2d_set_dt / dt_init is used. Grids of up to
+ * 514 rows of 64 to 1024 points (without a model, MMS forcing or closure_diag) take all nsteps
+ * in one cooperative launch, unless s is being captured; use_graph: the others replay one
+ * captured CUDA graph per step. */
 int  nse2d_step(nse2d_ctx* ctx, int nsteps, int use_graph, cudaStream_t s);
 /* The tridiagonal solve of the Poisson step: clusters != 0 selects the one-pass form on
  * persistent thread-block clusters (the default where it can be resident: fastest for a
  * channel that has the device to itself), 0 the two-pass form on plain grids (which shares
  * the device with concurrent work). Both give the reference's solve to round-off, not the
- * same bits. Synchronises the device when the form changes (the step graph is captured
- * again). */
+ * same bits. Grids of up to 1026 rows have a third form in their steps and solves (all rows of
+ * two or four columns in one CTA), whatever is chosen here. Synchronises the device when the
+ * form changes (the step graph is captured again). */
 int  nse2d_set_tridiag_form(nse2d_ctx* ctx, int clusters);
 /* The kernel forms of a context's step (no counterpart in the reference, which has one form of
  * each operator): stage_tma, the persistent stage kernel fed by TMA boxes (1) or the one with a
  * CTA per tile and plain halo loads (0; grids with Nx < 128, or Nx < 256 in precision 32, have
- * only this one); tridiag_clusters, as nse2d_set_tridiag_form; rowfft_prefetch, the row
+ * only this one; rows of 64 to 1024 points take their stages in bands of rows, without either, and
+ * have one form of the step but for pdl); tridiag_clusters, as nse2d_set_tridiag_form; rowfft_prefetch, the row
  * transforms whose rows are prefetched into shared memory by bulk copies (1; Nx = 4096 in
  * precision 64 only) or read by plain loads (0); max_fused, with the prefetching transforms in an
  * adaptive FP64 step, the max reduction of psi inside the stage-3 inverse transform and dt
@@ -160,12 +164,12 @@ int  nse2d_autotune_plan(nse2d_ctx* ctx, int trial_steps, nse2d_plan* best, doub
  * context (field 4), which the next nse2d_diagnostics(t0_row = 0) pairs with omega for the
  * dOmega_rhs column (src/main.cu:586). */
 int  nse2d_step_store_rhs(nse2d_ctx* ctx, int nsteps, cudaStream_t s);
-/* As nse2d_step without a graph, with CUDA events on s around every kernel; kernel_ms[k]
+/* As nse2d_step by launches and without a graph, with CUDA events on s around every kernel; kernel_ms[k]
  * receives the summed duration of the k-th kernel of a step over the nsteps steps
  * (nse2d_launches_per_step entries). Synchronous. */
 int  nse2d_step_timed(nse2d_ctx* ctx, int nsteps, double* kernel_ms, cudaStream_t s);
-/* One step (storing its stage-3 rhs, as nse2d_step_store_rhs) with CUDA events around every
- * kernel: the step's device time, the time of its row transforms and of its tridiagonal
+/* One step (storing its stage-3 rhs, as nse2d_step_store_rhs) by separate stages and row
+ * transforms, with CUDA events around every kernel: the step's device time, the time of its row transforms and of its tridiagonal
  * solves, in ms (the step_ms, fft_ms and tridiag_ms columns of the reference's timing.csv,
  * src/main.cu:746-753; any output may be NULL). Synchronous. */
 int  nse2d_step_profiled(nse2d_ctx* ctx, double* step_ms, double* fft_ms, double* tridiag_ms,
@@ -182,7 +186,8 @@ int  nse2d_get_time(nse2d_ctx* ctx, double* t, double* dt, long long* step, doub
                     cudaStream_t s);
 
 /* Run the time loop on the device (src/main.cu:434-551) until something needs the host:
- * steps are taken inside one CUDA graph launch (a WHILE node around the captured step) and
+ * steps are taken inside one CUDA graph launch (a WHILE node around the captured step), or one
+ * cooperative launch (see nse2d_step; at most 8192 steps each, without device statistics), and
  * the run stops after the step at which
  *   NSE2D_HALT_OUTPUT     t has reached min(next_snap, next_diag) (within the snap tolerance),
  *   NSE2D_HALT_STATS      the step count is a multiple of stats_every (0: never),
@@ -275,7 +280,8 @@ int  nse2d_scalar(nse2d_ctx* ctx, int which, double* out);
  * graph's WHILE node repeats one step of every member; members are dealt round-robin onto
  * `groups` concurrent branches. Results do not depend on the grouping. Creating the ensemble
  * sets its members to the two-pass tridiagonal solve (nse2d_set_tridiag_form(m, 0)), whose
- * plain grids share the device with the other branches. */
+ * plain grids share the device with the other branches (members of up to 1026 rows: the one-CTA
+ * form). Members' steps are by launches, with the bits of the steps in one launch. */
 typedef struct nse2d_ensemble nse2d_ensemble;
 int  nse2d_ensemble_create(nse2d_ctx* const* members, int n, nse2d_ensemble** out);
 int  nse2d_ensemble_destroy(nse2d_ensemble* e);

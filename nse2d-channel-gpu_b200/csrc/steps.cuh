@@ -16,9 +16,9 @@
 // gives up sets bit 1 of the non-finite flag and the CTA returns; the others then give up too, and later launches do
 // nothing until a state is set. The launch is cooperative, so all CTAs are resident.
 //
-// What bounds it: at 128x129 (127 CTAs of one row) the barriers, about 3000 clocks each of 35000 a step (drain of
+// What bounds it: at 128x129 (127 CTAs of one row) the barriers, about 3000 clocks each of 42000 a step (drain of
 // the stores, arrival, poll: three trips to L2); at 1024x513 the latency of the phases (stage 6000 clocks, solve
-// 6600, inverse 5500, forward 3400, barriers 3000 to 6000 with their skew, of 91000). Steps by launches and here:
+// 6600, inverse 5500, forward 3400, barriers 3000 to 6000 with their skew, of 103000). Steps by launches and here:
 // 128x129 30.7 and 21.2 us, 256x257 32.8 and 25.1, 1024x513 59.4 and 52.3; FP32 512x301 48 and 28.9. Polling with
 // relaxed loads and one fence at the end: 0.3 us a barrier more. The rhs of stage 1, which needs no dt, between arriving
 // at the maxima's barrier and waiting there: a second copy of the stage in the kernel, 128x129 23.0 us.
