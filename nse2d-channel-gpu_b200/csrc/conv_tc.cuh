@@ -422,8 +422,11 @@ static __global__ void __launch_bounds__(WG_NT, 2) k_wgrad(WgradParams p) {
             float x[4] = {v.x, v.y, v.z, v.w}, y[4], w[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const float hi = __bfloat162float(__float2bfloat16_rn(x[i]));
-                const float r1 = x[i] - hi;                            // exact
+                // an infinity (or a NaN) is its own first term, and a finite value that would round to one is cut there
+                const bool finite = fabsf(x[i]) <= 3.402823466e38f;
+                float hi = __bfloat162float(__float2bfloat16_rn(x[i]));
+                if (finite && !(fabsf(hi) <= 3.402823466e38f)) hi = __uint_as_float(__float_as_uint(x[i]) & 0xffff0000u);
+                const float r1 = finite ? x[i] - hi : 0.f;             // exact
                 const float mid = __bfloat162float(__float2bfloat16_rn(r1));
                 w[i] = r1 - mid;                                       // exact, at most 8 bits
                 y[i] = mid;

@@ -40,3 +40,24 @@ def test_edges_match_the_oracle(nse, cuda, Nx, Ny, H, idx):
 def test_strips_match_the_oracle(nse, cuda, Nx, Ny, H, idx):
     """Strips of one, two and four rows, a row of one and of several strips, and tiles that run over the rows' ends."""
     test_edges_match_the_oracle(nse, cuda, Nx, Ny, H, idx)
+
+
+@pytest.mark.parametrize("H", [16, 32, 48, 64])
+def test_an_infinite_target_gives_infinite_gradients(nse, cuda, H):
+    """One infinite tau at a pixel whose whole neighbourhood is away from the walls, with weights, biases and inputs
+    that are all positive: its dZ is -inf in every channel of every layer and every activation that it meets is
+    positive, so every gradient is -inf; a NaN would come of a split of dZ that subtracts infinities."""
+    torch = cuda
+    Nx, Ny = 32, 33
+    net = nse.Cnn(Nx, Ny, np.linspace(0.5, 1.5, Ny), H, 1)
+    rng = np.random.default_rng(H)
+    for layer in range(4):
+        ci, co_ = net.shape(layer)
+        net.set_params(layer, rng.uniform(0.01, 0.02, (co_, 9, ci)), rng.uniform(0.1, 0.2, co_))
+    net.set_scales(*SCALES)
+    f = [rng.uniform(0.5, 1.0, (Ny, Nx)) for _ in range(5)]
+    f[4][16, 9] = np.inf
+    assert net.gradients(*[_dev(torch, a[None]) for a in f]) == np.inf
+    for layer in range(4):
+        for g in net.get_grads(layer):
+            assert np.all(g == -np.inf), (layer, np.unique(g)[:4])
