@@ -265,7 +265,8 @@ int  nse2d_rhs_at_state(nse2d_ctx* ctx, double t, cudaStream_t s);
 int  nse2d_uv(nse2d_ctx* ctx, double* d_u, double* d_v, cudaStream_t s);
 /* Non-finite and timeout flags since the state was last set (nse2d_set_omega / nse2d_set_state):
  * bit 0 a max reduction met NaN or Inf in psi, bit 1 a bounded wait of a kernel timed out.
- * Synchronous. */
+ * After a wait that timed out the fields are void until a state is set: steps in one launch do
+ * nothing, and a run halts with NSE2D_HALT_NONFINITE. Synchronous. */
 int  nse2d_nonfinite(nse2d_ctx* ctx, int* flag, cudaStream_t s);
 /* Host copy of a metric: 0 y, 1 a_node, 2 a_edge (Ny-1), 3 dy_edge (Ny-1), 4 w_node. */
 int  nse2d_metrics(nse2d_ctx* ctx, int which, double* out);

@@ -242,7 +242,9 @@ int nse2d_run(nse2d_ctx* ctx, double next_snap, double next_diag, int stats_ever
     if (run_until_halt(c, s)) return -1;
     NSE_CUDA_TRY(cudaMemcpyAsync(h, c->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
     NSE_CUDA_TRY(cudaStreamSynchronize(s));
-    if (reason) *reason = h->halt_reason;
+    // a wait that gave up ends the steps in one launch, and those of later launches, without a reason of their own
+    // (which the step by launches gives); here and not in k_steps, where the code for it cost 0.3 us a step at 128x129
+    if (reason) *reason = h->halt_reason | ((h->nonfinite & 2) ? NSE2D_HALT_NONFINITE : 0);
     const int zero = 0;
     NSE_CUDA_TRY(cudaMemcpyAsync(&c->ctl->run, &zero, sizeof(int), cudaMemcpyHostToDevice, s));
     NSE_CUDA_TRY(cudaStreamSynchronize(s));

@@ -1,0 +1,68 @@
+// States of a context that the C ABI cannot set, for test_internals_gpu.py: a driver that includes the library's
+// internal headers and is linked with it. Prints "name value" lines.
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+#include <string>
+#include <vector>
+
+#include "../include/nse2d.h"
+#include "../nse2d-channel-gpu_b200/csrc/nse2d_internal.h"
+
+using nse2d::Context;
+
+#define OK(x)                                                                            \
+    do {                                                                                 \
+        if ((x) != 0) {                                                                  \
+            std::fprintf(stderr, "%s: %s\n", #x, nse2d_last_error());                    \
+            std::exit(1);                                                                \
+        }                                                                                \
+    } while (0)
+
+static nse2d_ctx* channel(int Nx, int Ny, int precision) {
+    nse2d_config c;
+    nse2d_config_default(&c);
+    c.Nx = Nx; c.Ny = Ny; c.stretch = 1; c.beta = 2.0; c.Reb = 2000.0; c.F0 = 0.05; c.nforce = 4; c.adapt = 1;
+    c.precision = precision;
+    nse2d_ctx* x = nullptr;
+    OK(nse2d_create(&c, &x));
+    return x;
+}
+static void start(nse2d_ctx* x) {
+    const Context* c = x->c;
+    std::vector<double> w((size_t)c->Nx * c->Ny), y(c->Ny);
+    OK(nse2d_metrics(x, 0, y.data()));
+    for (int j = 0; j < c->Ny; ++j)
+        for (int i = 0; i < c->Nx; ++i) w[(size_t)j * c->Nx + i] = 3.0 * y[j] + 0.05 * std::sin(M_PI * (y[j] + 1.0)) * std::cos(2.0 * M_PI * i / c->Nx);
+    OK(nse2d_set_omega(x, w.data(), 0, nullptr));
+}
+static long long steps_taken(nse2d_ctx* x) {
+    long long n = 0;
+    OK(nse2d_get_time(x, nullptr, nullptr, &n, nullptr, nullptr));
+    return n;
+}
+
+// A wait that has timed out: the flag that the kernel would have left, then a run, steps, and a new state.
+static void gave_up(int precision) {
+    nse2d_ctx* x = channel(128, 65, precision);
+    start(x);
+    std::printf("one_launch %d\n", x->c->steps_R > 0);
+    const int flag = 2;
+    OK(cudaMemcpy(&x->c->ctl->nonfinite, &flag, sizeof(int), cudaMemcpyHostToDevice));
+    int reason = -1;
+    OK(nse2d_run(x, 1e300, 1e300, 0, 1e300, 5, &reason, nullptr));
+    std::printf("reason %d\n", reason);
+    OK(nse2d_step(x, 3, 1, nullptr));
+    std::printf("steps_of_a_void_state %lld\n", steps_taken(x));
+    start(x);
+    OK(nse2d_run(x, 1e300, 1e300, 0, 1e300, 5, &reason, nullptr));
+    std::printf("reason_of_a_new_state %d\nsteps_of_a_new_state %lld\n", reason, steps_taken(x));
+    OK(nse2d_destroy(x));
+}
+
+int main(int argc, char** argv) {
+    const std::string what = argc > 1 ? argv[1] : "";
+    if (what == "gave_up") gave_up(std::atoi(argv[2]));
+    else return 2;
+    return 0;
+}

@@ -1,0 +1,38 @@
+"""States that the C ABI cannot set, through a driver that sees the library's internals (internals_driver.cu), on a
+B200. A wait that has timed out is not made to happen: the flag that it leaves is written by the host.
+"""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from conftest import PKG, ROOT
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def driver(nse, cuda, tmp_path_factory):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    exe = str(tmp_path_factory.mktemp("internals") / "internals_driver")
+    subprocess.run([nvcc, "-O1", "-std=c++17", "--expt-relaxed-constexpr", "-gencode", "arch=compute_100a,code=sm_100a",
+                    os.path.join(ROOT, "tests", "internals_driver.cu"), "-L", PKG, "-lnse2d_b200", "-Xlinker", "-rpath", "-Xlinker", PKG,
+                    "-o", exe], check=True, capture_output=True, timeout=600)
+
+    def run(*args):
+        r = subprocess.run([exe, *map(str, args)], capture_output=True, text=True, timeout=120)
+        assert r.returncode == 0, r.stderr
+        return {k: float(v) for k, v in (ln.split() for ln in r.stdout.splitlines())}
+    return run
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_a_run_after_a_wait_that_timed_out_says_so(nse, driver, precision):
+    """The reason is NSE2D_HALT_NONFINITE (a host loop that waits for t_end would otherwise never end); a new state
+    runs as ever."""
+    got = driver("gave_up", precision)
+    assert got["one_launch"] == 1
+    assert int(got["reason"]) & nse.HALT_NONFINITE
+    assert got["steps_of_a_void_state"] == 0
+    assert got["reason_of_a_new_state"] == nse.HALT_BUDGET and got["steps_of_a_new_state"] == 5
