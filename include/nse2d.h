@@ -349,10 +349,13 @@ int  nse2d_cnn_set_application(nse2d_cnn* c, int wall_rows, double gain, int row
 int  nse2d_cnn_forward(nse2d_cnn* c, const double* w, const double* psi, const double* u, const double* v, double* tau,
                        cudaStream_t s);
 /* loss = mean over the interior pixels of the batch of (output - tau / tau_scale)^2 and its
- * gradients; waits, and stores the loss when loss != NULL */
+ * gradients; waits, and stores the loss when loss != NULL. An error when a bounded wait of the
+ * model's kernels timed out, here or in a forward pass since the last such call: loss and gradients
+ * are then void */
 int  nse2d_cnn_gradients(nse2d_cnn* c, const double* w, const double* psi, const double* u, const double* v,
                          const double* tau, const int* idx, int nb, float* loss, cudaStream_t s);
-/* gradients, then one AdamW step (beta1 0.9, beta2 0.999, eps 1e-8, decoupled weight decay) */
+/* gradients, then one AdamW step (beta1 0.9, beta2 0.999, eps 1e-8, decoupled weight decay); an error as
+ * nse2d_cnn_gradients, without a step */
 int  nse2d_cnn_train_step(nse2d_cnn* c, const double* w, const double* psi, const double* u, const double* v,
                           const double* tau, const int* idx, int nb, float lr, float weight_decay, float* loss,
                           cudaStream_t s);

@@ -334,8 +334,9 @@ __device__ __forceinline__ void export_one(const LayerParams& q, int e) {
         q.wt[(size_t)c * 9 * q.npad + tap * q.npad + n] = b;
     }
 }
-// grid: (blocks of the largest layer, layers)
-__global__ void __launch_bounds__(CN_NT) k_adamw(AllLayers all, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2) {
+// grid: (blocks of the largest layer, layers). err: a wait of the passes before timed out, and the gradients are void.
+__global__ void __launch_bounds__(CN_NT) k_adamw(AllLayers all, const int* err, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2) {
+    if (*err) return;
     const LayerParams& q = all.l[blockIdx.y];
     const int e = blockIdx.x * CN_NT + threadIdx.x;
     if (e < q.npad * q.K) {
@@ -605,11 +606,12 @@ static int cnn_adamw(Cnn* n, float lr, float wd, cudaStream_t s) {
         all.l[l] = layer_params(n, l);
         most = std::max(most, n->npad[l] * n->K[l]);
     }
-    k_adamw<<<dim3(grid_of(most), CN_LAYERS), CN_NT, 0, s>>>(all, lr, b1, b2, eps, wd, bc1, bc2);
+    k_adamw<<<dim3(grid_of(most), CN_LAYERS), CN_NT, 0, s>>>(all, n->err, lr, b1, b2, eps, wd, bc1, bc2);
     NSE_CUDA_TRY(cudaGetLastError());
     return 0;
 }
 
+int* cnn_wait_flag(Cnn* n) { return n->err; }
 bool cnn_matches(const Cnn* n, int Nx, int Ny) { return n && n->Nx == Nx && n->Ny == Ny; }
 
 void cnn_free(Cnn* n) {
@@ -692,10 +694,6 @@ static int cnn_create(int Nx, int Ny, int hidden, int max_batch, const double* y
 }  // namespace nse2d
 
 using namespace nse2d;
-
-struct nse2d_cnn {
-    Cnn* n;
-};
 
 extern "C" {
 
@@ -868,15 +866,19 @@ static int enqueue_gradients(nse2d_cnn* c, const double* w, const double* psi, c
     NSE_CUDA_TRY(cudaMemsetAsync(n->idx, 0, sizeof(int), s));
     return rc;
 }
-// the loss and the error flag, once the stream has come to them
-static int finish_gradients(Cnn* n, float* loss, int* err, cudaStream_t s) {
+// the loss and the error flag, once the stream has come to them. A wait that timed out, in this call or in a forward
+// pass since the last one, is reported once: the flag is then cleared
+static int finish_gradients(Cnn* n, const char* who, float* loss, cudaStream_t s) {
     struct { float loss; int err; } r{};
     static_assert(sizeof(r) == 8, "the flag lies behind the loss");
     NSE_CUDA_TRY(cudaMemcpyAsync(&r, n->loss, sizeof(r), cudaMemcpyDeviceToHost, s));
     NSE_CUDA_TRY(cudaStreamSynchronize(s));
     if (loss) *loss = r.loss;
-    *err = r.err;
-    return 0;
+    if (!r.err) return 0;
+    NSE_CUDA_TRY(cudaMemsetAsync(n->err, 0, sizeof(int), s));
+    NSE_CUDA_TRY(cudaStreamSynchronize(s));
+    set_error("%s: a tensor-core wait ran out", who);
+    return -1;
 }
 
 int nse2d_cnn_gradients(nse2d_cnn* c, const double* w, const double* psi, const double* u, const double* v,
@@ -886,8 +888,7 @@ int nse2d_cnn_gradients(nse2d_cnn* c, const double* w, const double* psi, const 
         cudaStreamSynchronize(s);
         return -1;
     }
-    int e = 0;
-    return finish_gradients(c->n, loss, &e, s);
+    return finish_gradients(c->n, "nse2d_cnn_gradients", loss, s);
 }
 
 int nse2d_cnn_train_step(nse2d_cnn* c, const double* w, const double* psi, const double* u, const double* v,
@@ -898,9 +899,10 @@ int nse2d_cnn_train_step(nse2d_cnn* c, const double* w, const double* psi, const
         return -1;
     }
     if (cnn_adamw(c->n, lr, weight_decay, s)) return -1;
-    int e = 0;
-    if (finish_gradients(c->n, loss, &e, s)) return -1;
-    if (e) { set_error("nse2d_cnn_train_step: a tensor-core wait ran out"); return -1; }
+    if (finish_gradients(c->n, "nse2d_cnn_train_step", loss, s)) {
+        c->n->step -= 1;                          // no update was made
+        return -1;
+    }
     return 0;
 }
 

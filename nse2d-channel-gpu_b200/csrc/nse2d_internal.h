@@ -55,6 +55,7 @@ int launch_steps32(Context* c, int nsteps, int run, int store, cudaStream_t s);
 struct Cnn;
 int cnn_forward_psi(Cnn* n, const double* w, const double* psi, const double* a_node, double inv_dx, double inv_deta, double* tau,
                     cudaStream_t s);
+int* cnn_wait_flag(Cnn* n);        // device flag of the model's bounded waits
 bool cnn_matches(const Cnn* n, int Nx, int Ny);
 int thomas_launches(const Context* c);
 const char* thomas_kernel_name(const Context* c, int i);
@@ -109,4 +110,7 @@ bool compat_free_slip();
 // The C ABI's handle: one solver context.
 struct nse2d_ctx {
     nse2d::Context* c;
+};
+struct nse2d_cnn {
+    nse2d::Cnn* n;
 };

@@ -60,9 +60,73 @@ static void gave_up(int precision) {
     OK(nse2d_destroy(x));
 }
 
+// A wait of the model's kernels that has timed out: gradients and a training step, and the same once it is reported.
+struct Model {
+    static constexpr int Nx = 32, Ny = 17, H = 16;
+    nse2d_cnn* n = nullptr;
+    double* f = nullptr;                                     // five fields
+    Model() {
+        std::vector<double> y(Ny), h((size_t)5 * Nx * Ny);
+        for (int j = 0; j < Ny; ++j) y[j] = -1.0 + 2.0 * j / (Ny - 1);
+        for (size_t i = 0; i < h.size(); ++i) h[i] = std::sin(0.37 * (double)i);
+        OK(nse2d_cnn_create(Nx, Ny, H, 1, y.data(), &n));
+        for (int l = 0; l < 4; ++l) {
+            int ci = 0, co = 0;
+            OK(nse2d_cnn_layer_shape(n, l, &ci, &co));
+            std::vector<float> w((size_t)co * 9 * ci), b(co, 0.1f);
+            for (size_t i = 0; i < w.size(); ++i) w[i] = 0.1f * std::cos(0.71f * (float)i);
+            OK(nse2d_cnn_set_params(n, l, w.data(), b.data()));
+        }
+        OK(cudaMalloc((void**)&f, h.size() * sizeof(double)));
+        OK(cudaMemcpy(f, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
+    }
+    ~Model() { nse2d_cnn_destroy(n); cudaFree(f); }
+    const double* field(int k) const { return f + (size_t)k * Nx * Ny; }
+    int gradients(float* loss) {
+        const int idx = 0;
+        return nse2d_cnn_gradients(n, field(0), field(1), field(2), field(3), field(4), &idx, 1, loss, nullptr);
+    }
+    int train() {
+        const int idx = 0;
+        return nse2d_cnn_train_step(n, field(0), field(1), field(2), field(3), field(4), &idx, 1, 1e-2f, 1e-4f, nullptr, nullptr);
+    }
+    void timed_out() {
+        const int one = 1;
+        OK(cudaMemcpy(nse2d::cnn_wait_flag(n->n), &one, sizeof(int), cudaMemcpyHostToDevice));
+    }
+    std::vector<float> weights() {
+        std::vector<float> all;
+        for (int l = 0; l < 4; ++l) {
+            int ci = 0, co = 0;
+            OK(nse2d_cnn_layer_shape(n, l, &ci, &co));
+            std::vector<float> w((size_t)co * 9 * ci), b(co);
+            OK(nse2d_cnn_get_params(n, l, w.data(), b.data()));
+            all.insert(all.end(), w.begin(), w.end());
+            all.insert(all.end(), b.begin(), b.end());
+        }
+        return all;
+    }
+};
+static void model_wait() {
+    Model a, b;
+    float loss = 0.f, ref = 0.f;
+    OK(b.gradients(&ref));
+    a.timed_out();
+    std::printf("gradients %d\n", a.gradients(&loss));
+    std::printf("gradients_after %d\nloss_after_is_right %d\n", a.gradients(&loss), loss == ref);
+    const std::vector<float> w0 = a.weights();
+    a.timed_out();
+    std::printf("train %d\n", a.train());
+    std::printf("weights_kept %d\n", a.weights() == w0);
+    std::printf("train_after %d\n", a.train());
+    OK(b.train());
+    std::printf("weights_after_are_the_first_steps %d\n", a.weights() == b.weights() && a.weights() != w0);
+}
+
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "gave_up") gave_up(std::atoi(argv[2]));
+    else if (what == "model_wait") model_wait();
     else return 2;
     return 0;
 }

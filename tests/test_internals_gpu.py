@@ -36,3 +36,13 @@ def test_a_run_after_a_wait_that_timed_out_says_so(nse, driver, precision):
     assert int(got["reason"]) & nse.HALT_NONFINITE
     assert got["steps_of_a_void_state"] == 0
     assert got["reason_of_a_new_state"] == nse.HALT_BUDGET and got["steps_of_a_new_state"] == 5
+
+
+def test_a_model_wait_that_timed_out_is_an_error_once(driver):
+    """nse2d_cnn_gradients and nse2d_cnn_train_step return an error, the weights and the step count stay as they were,
+    and the calls after it work: the next training step is the first one, to the bit."""
+    got = driver("model_wait")
+    assert got["gradients"] == -1 and got["train"] == -1
+    assert got["gradients_after"] == 0 and got["loss_after_is_right"] == 1
+    assert got["weights_kept"] == 1
+    assert got["train_after"] == 0 and got["weights_after_are_the_first_steps"] == 1
