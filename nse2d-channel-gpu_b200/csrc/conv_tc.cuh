@@ -422,15 +422,25 @@ static __global__ void __launch_bounds__(WG_NT, 2) k_wgrad(WgradParams p) {
             float x[4] = {v.x, v.y, v.z, v.w}, y[4], w[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                // an infinity (or a NaN) is its own first term, and a finite value that would round to one is cut there
-                const bool finite = fabsf(x[i]) <= 3.402823466e38f;
-                float hi = __bfloat162float(__float2bfloat16_rn(x[i]));
-                if (finite && !(fabsf(hi) <= 3.402823466e38f)) hi = __uint_as_float(__float_as_uint(x[i]) & 0xffff0000u);
-                const float r1 = finite ? x[i] - hi : 0.f;             // exact
+                const float hi = __bfloat162float(__float2bfloat16_rn(x[i]));
+                const float r1 = x[i] - hi;                            // exact
                 const float mid = __bfloat162float(__float2bfloat16_rn(r1));
                 w[i] = r1 - mid;                                       // exact, at most 8 bits
                 y[i] = mid;
                 x[i] = hi;
+            }
+            // above the largest finite BF16 value: an infinity is its own first term, a finite value is cut there instead
+            // of being rounded to one
+            if (fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))) > 3.38953139e38f) {
+                const float t[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (!(fabsf(t[i]) > 3.38953139e38f)) continue;     // a NaN has stayed one
+                    const bool inf = fabsf(t[i]) > 3.402823466e38f;
+                    x[i] = __uint_as_float(__float_as_uint(t[i]) & 0xffff0000u);
+                    y[i] = inf ? 0.f : __bfloat162float(__float2bfloat16_rn(t[i] - x[i]));
+                    w[i] = inf ? 0.f : t[i] - x[i] - y[i];
+                }
             }
             __nv_bfloat16* d = sB + px * LDB + c;
             *reinterpret_cast<uint2*>(d) = make_uint2(cv_pack2(x[0], x[1]), cv_pack2(x[2], x[3]));
