@@ -22,6 +22,7 @@ int band32_rows_inv(Context* c, float* w, bool advance, cudaStream_t s) {
     return band_rows_inv_impl(c, band_params(c), c->psif, w, true, advance, s);
 }
 
+int band_setup32(Context* c) { return band_setup_impl<float>(c); }
 int steps_setup32(Context* c) { return steps_setup_impl<float>(c); }
 int launch_steps32(Context* c, int nsteps, int run, int store, cudaStream_t s) {
     StepsParams<float> p{};

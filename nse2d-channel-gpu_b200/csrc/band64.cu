@@ -4,7 +4,7 @@
 namespace nse2d {
 
 // The transforms of rows of 64 to 2048 points: longer rows have their own kernels (prefetched rows at 4096),
-// shorter ones have fewer points than a warp. Bands: see band.cuh for where the line lies.
+// shorter ones have fewer points than a warp. Bands: of rows of up to 1024 points (see band.cuh), by band_setup.
 bool band_rows_ok(int M) { return M >= 32 && M <= 1024; }
 bool band_stage_ok(int M) { return M >= 32 && M <= 512; }
 
@@ -29,6 +29,7 @@ int band_rows_inv(Context* c, double* psi, double* w, bool thom, bool advance, c
     return band_rows_inv_impl(c, band_params(c), psi, w, thom, advance, s);
 }
 
+int band_setup(Context* c) { return band_setup_impl<double>(c); }
 int steps_setup(Context* c) { return c->prec32 ? steps_setup32(c) : steps_setup_impl<double>(c); }
 int launch_steps(Context* c, int nsteps, int run, int store, cudaStream_t s) {
     if (c->prec32) return launch_steps32(c, nsteps, run, store, s);

@@ -45,6 +45,28 @@ template <typename T, int M> int rows_inv_t(Context* c, BandParams<T>& p, cudaSt
     return launch_step_kernel(c, k_rows_inv<T, M>, dim3((c->Ni + G - 1) / G), dim3(G * Band<M>::TPR), sm, s, nullptr, p);
 }
 
+// Whether a channel steps by bands: while all of them, of the most rows, are resident at once; of rows of up to 256
+// points, whose bands are the short ones, in two rounds. Beyond that line a band is a second (third) wave in which most
+// SMs idle, its two halo rows are transformed by CTAs that have no time left over, and psi-hat's own buffer is one more
+// in L2; the separate kernels have finer tiles. A step by bands and by separate kernels either side of it, us: FP64
+// 1024x594 65 and 76, 1024x600 87 and 84; 512x890 58 and 70, 512x900 78 and 70; 128x1778 57 and 59, 128x1800 66 and 60;
+// FP32 58 and 68, 75 and 72; 50 and 62, 66 and 60; 128x3552 64 and 70, 128x3600 72 and 70. Far beyond: FP64 1024x4097
+// 322 and 264, FP32 251 and 207, 512x8193 413 and 351.
+template <typename T, int M> int band_setup_t(Context* c) {
+    using B = Band<M>;
+    int per_sm = 0;
+    NSE_CUDA_TRY(cudaFuncSetAttribute(k_band<T, M, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)band_smem_bytes<T, M>(B::RMAX)));
+    NSE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_band<T, M, true>, B::MAXT, band_smem_bytes<T, M>(B::RMAX)));
+    if (per_sm < 1) return 0;                                // separate kernels
+    c->band_load = (double)((c->Ni + B::RMAX - 1) / B::RMAX) / ((double)per_sm * c->num_sms);
+    c->band_fit = c->band_load <= (M <= 128 ? 2.0 : 1.0);
+    return 0;
+}
+template <typename T> int band_setup_impl(Context* c) {
+    if (!band_stage_ok(c->M)) return 0;
+    NSE_BAND512_DISPATCH(band_setup_t, c)
+}
+
 // Stage `stage` of the step and the forward transform of its omega^(s+1); inv: the inverse transform of
 // psi-hat and the wall closure of w_in before it (else psi is read from the context's psi).
 template <typename T>

@@ -105,11 +105,16 @@ struct RowTables {
     double* mms_s2k;
 };
 
-// Channels together that still step by bands. More of them fill the device, and the halo rows that bands transform
-// twice are then time lost (an ensemble step of 4, 8, 12, 16, 32 and 64 channels, us: FP64 bands 111, 115, 183, 188, 518
-// and 1054, separate kernels 116, 116, 182, 181, 506 and 976; FP32 88, 92, 141, 140, 398 and 808 against 92, 91, 131,
-// 127, 353 and 706).
+// Channels that run together (the branches of an ensemble) step by bands while there are at most 8 of them and their
+// bands, of the most rows, are at most four times what the device holds at once. Beyond that they fill it, and the halo
+// rows that bands transform twice are time lost. An ensemble step by bands and by separate kernels, us: FP64 mixed sizes
+// (256 to 1024 points, 129 to 513 rows) 4 channels 63 and 71, 8 94 and 100, 12 229 and 218, 64 977 and 957; FP32 54 and
+// 66, 77 and 87, 172 and 156, 736 and 674. Of one size: FP32 1024x513, 2 channels (1.7 times the device) 79 and 82, 4
+// (3.5) 128 and 118, 6 (5.2) 192 and 169, 8 255 and 220; FP64 4 168 and 168, 6 243 and 235, 8 321 and 306; FP64
+// 128x1500, 2 (3.4) 97 and 93, 3 (5.1) 122 and 104, 8 251 and 172. More than 8 small ones would still gain by bands (16
+// of 64x65: 50 and 74).
 constexpr int kBandShareMax = 8;
+constexpr double kBandLoadMax = 4.0;
 struct Context {
     Config cfg;
     int Nx = 0, Ny = 0, M = 0, H = 0, Hp = 0, Ni = 0;
@@ -130,9 +135,11 @@ struct Context {
     // otherwise psi-hat takes the place of omega-hat
     cpx<double>* hat2 = nullptr;
     bool band = false;             // row transforms of band.cuh: rows of 64 to 2048 points
+    bool band_fit = false;         // the steps go by bands of rows (band_setup)
+    double band_load = 0.0;        // its bands, of the most rows, over those that the device holds at once
     int band_share = 1;            // channels that run at the same time as this one (the branches of an ensemble)
     int steps_R = 0;               // rows of a band of the steps in one launch (0: not used)
-    bool plain_step = false;       // a step of separate transforms and stages (nse2d_step_profiled times them apart)
+    bool plain_step = false;       // a step of separate transforms and stages (nse2d_step_profiled times them apart; ensembles)
     double* cp = nullptr;          // elimination table [Ni][Hp]
     cpx<double>* tw = nullptr;     // per-pass twiddle pairs of the Nx/2-point transform
     cpx<double>* tw_band = nullptr;  // the same for the row-band kernels' plan

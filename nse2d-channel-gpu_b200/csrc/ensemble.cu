@@ -69,13 +69,18 @@ int ensemble_build(Ensemble* e, int groups, bool force = false) {
     err = cudaStreamBeginCaptureToGraph(e->cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (err != cudaSuccess) { set_error("ensemble capture: %s", cudaGetErrorString(err)); return done(-1); }
     int rc = 0;
+    double load = 0.0;                                                // of the members that run at a time, on average
+    for (const Context* c : e->m) load += c->band_load * groups / n;
+    const bool bands = groups <= kBandShareMax && load <= kBandLoadMax;
     cudaEventRecord(ev[0], e->cap);                                   // fork
     for (int b = 0; b < groups && rc == 0; ++b) {
         cudaStreamWaitEvent(e->branch[b], ev[0], 0);
         for (int i = b; i < n && rc == 0; i += groups) {
             e->m[i]->band_share = groups;
+            e->m[i]->plain_step = !bands;
             rc = enqueue_step(e->m[i], e->branch[b], false);
             e->m[i]->band_share = 1;
+            e->m[i]->plain_step = false;
         }
         cudaEventRecord(ev[1 + b], e->branch[b]);                     // join
         cudaStreamWaitEvent(e->cap, ev[1 + b], 0);

@@ -39,6 +39,8 @@ int launch_thomas_cluster(Context* c, cudaStream_t s, bool homog = false);
 // row-band kernels (band64.cu, band32.cu)
 bool band_rows_ok(int M);
 bool band_stage_ok(int M);
+int band_setup(Context* c);              // band_fit and band_load of a channel (before its psi-hat is allocated)
+int band_setup32(Context* c);
 int band_stage(Context* c, int stage, bool inv, double* w_in, const double* w_n, double* w_out, double* rhs_out,
                const double* closure, cudaStream_t s);
 int band_rows_fwd(Context* c, const double* src, int row0, int nrows, cudaStream_t s);

@@ -328,7 +328,7 @@ int context_create(const Config& cfg, Context** out) {
         dalloc(&c->wN, (size_t)c->M + 1))
         return fail();
     c->band = band_rows_ok(c->M);
-    if (c->band && cfg.precision == 64 && band_stage_ok(c->M) && dalloc(&c->hat2, (size_t)Ny * c->Hp)) return fail();
+    if (cfg.precision == 64 && (band_setup(c) || (c->band_fit && dalloc(&c->hat2, (size_t)Ny * c->Hp)))) return fail();
     c->thomas_nseg = (c->Ni + TS_ROWS - 1) / TS_ROWS;
     c->thomas_nsb = (c->thomas_nseg + TS_NW - 1) / TS_NW;
     if (dalloc(&c->tconst, (size_t)c->thomas_nseg * 3 * c->Hp) || dalloc(&c->tmaps, (size_t)c->thomas_nseg * 4 * c->Hp) ||
@@ -845,7 +845,7 @@ int poisson_solve(Context* c, const double* w, double* psi, cudaStream_t s, bool
 // The steps that the row-band kernels take: without the MMS forcing and the wall-update bookkeeping of
 // closure_diag (verification runs and diagnostics of their own), which the separate kernels have.
 static bool band_step(const Context* c) {
-    return c->band && band_stage_ok(c->M) && !c->cfg.mms && !c->closure_diag && !c->plain_step && c->band_share <= kBandShareMax;
+    return c->band_fit && !c->cfg.mms && !c->closure_diag && !c->plain_step;
 }
 
 // A stage of the band step begins with the inverse transform, except stage 1 (psi is the step's) and,

@@ -45,7 +45,7 @@ int setup32(Context* c) {
     std::vector<cpx<float>> tw_band;
     plan_twiddle_table(M, band_radix_bits(M), full.data(), tw_band);
     if (alloc(&c->twf, tw.size()) || alloc(&c->twf_band, tw_band.size()) || alloc(&c->wNf, wN.size())) return -1;
-    if (band_stage_ok(M) && alloc(&c->hat32b, (size_t)c->Ny * c->Hp)) return -1;
+    if (band_setup32(c) || (c->band_fit && alloc(&c->hat32b, (size_t)c->Ny * c->Hp))) return -1;
     NSE_CUDA_TRY(cudaMemcpy(c->twf_band, tw_band.data(), tw_band.size() * sizeof(tw[0]), cudaMemcpyHostToDevice));
     NSE_CUDA_TRY(cudaMemcpy(c->twf, tw.data(), tw.size() * sizeof(tw[0]), cudaMemcpyHostToDevice));
     NSE_CUDA_TRY(cudaMemcpy(c->wNf, wN.data(), wN.size() * sizeof(wN[0]), cudaMemcpyHostToDevice));
@@ -169,7 +169,7 @@ static int fft32_inv(Context* c, float* w_out, bool advance, cudaStream_t s) {
     NSE_FFT32_DISPATCH(fft32_inv_t)
 }
 
-bool band_step32(const Context* c) { return band_stage_ok(c->M) && !c->plain_step && c->band_share <= kBandShareMax; }
+bool band_step32(const Context* c) { return c->band_fit && !c->plain_step; }
 
 int step32_impl(Context* c, cudaStream_t s, bool store_rhs, cudaEvent_t* ev) {
     int k = 0;

@@ -15,7 +15,7 @@ from test_parity_gpu import laminar_perturbed, relerr
 pytestmark = pytest.mark.gpu
 
 GRIDS = [(64, 5), (64, 6), (64, 11), (64, 900), (128, 150), (128, 1333), (256, 151), (256, 300), (512, 9), (512, 597), (1024, 6),
-         (1024, 595), (1024, 745), (2048, 5), (2048, 61)]
+         (1024, 594), (1024, 595), (1024, 745), (2048, 5), (2048, 61)]
 
 
 @pytest.mark.parametrize("Nx,Ny", GRIDS)
@@ -125,3 +125,16 @@ def test_solve_of_tall_columns(nse, oracle, cuda, Nx, Ny):
     assert rel(b.fields()[1], a.fields()[1]) < 1e-5
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("precision,Nx,Ny,bands", [
+    (64, 1024, 594, True), (64, 1024, 595, False), (64, 1024, 4097, False), (64, 512, 890, True), (64, 512, 891, False), (64, 512, 2049, False),
+    (64, 128, 1778, True), (64, 128, 1779, False), (64, 64, 4097, False), (32, 1024, 594, True), (32, 1024, 595, False), (32, 512, 2049, False),
+    (32, 128, 3554, True), (32, 128, 3555, False), (32, 64, 8193, False)])
+def test_bands_while_they_fit_the_device(nse, cuda, precision, Nx, Ny, bands):
+    """The step by bands of rows is taken while its bands are resident at once (of rows of up to 256 points: in two
+    rounds), on 148 SMs; taller grids take the separate kernels, which are the faster ones there."""
+    s = nse.Solver(Nx=Nx, Ny=Ny, Lx=2 * np.pi, stretch=1, beta=1.0, Ub=1.0, Reb=2000.0, adapt=1, precision=precision)
+    names = [s.lib.nse2d_step_kernel_name(s.h, k).decode() for k in range(s.launches_per_step())]
+    assert ("k_band_inv_stage_fwd" in names) == bands, names
+    s.close()

@@ -103,3 +103,26 @@ def test_members_step_as_alone_however_many(nse, cuda, precision, n):
         assert a.time() == m.time()
         assert all(np.array_equal(x, y) for x, y in zip(a.fields(), m.fields()))
     ens.close()
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_members_that_fill_the_device_step_as_alone(nse, cuda, precision):
+    """A few members whose bands are more than four times what the device holds take the separate kernels, and give
+    the bits of the channels alone (in the two-pass solve that members of this height take), which step by bands."""
+    grids = [(128, 1500)] * (4 if precision == 64 else 6)
+    alone, members = [], []
+    for k, (Nx, Ny) in enumerate(grids):
+        pair = [make(nse, dict(Nx=Nx, Ny=Ny, beta=1.2, Reb=2000.0, nforce=4, precision=precision), k) for _ in range(2)]
+        for s in pair:
+            s.set_tridiag_form(False)
+        alone.append(pair[0])
+        members.append(pair[1])
+    assert "k_band_inv_stage_fwd" in [n for n, _ in alone[0].step_timed(1)]
+    members[0].step(1)
+    ens = nse.Ensemble(members)
+    ens.step(3)
+    for k, (a, m) in enumerate(zip(alone, members)):
+        a.step(3, use_graph=True)
+        assert a.time() == m.time()
+        assert all(np.array_equal(x, y) for x, y in zip(a.fields(), m.fields())), k
+    ens.close()
