@@ -101,24 +101,24 @@ def kernel_bytes(name, stage, Nx, Ny, precision=64):
     C = 8 if precision == 32 else 16                            # bytes per spectral value
     if name.startswith("k_stage32"):                              # k_stage32, k_stage32_tma
         return 4 * N * (2 if stage == 1 else 3) + 4 * N
-    if name.startswith("k_fft_fwd32"):
+    if name.startswith("k_fft_fwd32") or (name == "k_rows_fwd" and precision == 32):
         return 4 * Nx * Ni + 8 * H * Ni
-    if name.startswith("k_ifft_thom32"):
+    if name.startswith("k_ifft_thom32") or (name == "k_rows_inv" and precision == 32):
         return 8 * H * Ni + 4 * N + 4 * 6 * Nx
     if name == "k_maxuv32":
         return 4 * N
     if name.startswith("k_stage"):
         return 8 * N * (2 if stage == 1 else 3) + 8 * N          # psi, omega^(s) [, omega^n] -> omega^(s+1)
-    if name == "k_fft_fwd":
+    if name in ("k_fft_fwd", "k_rows_fwd") and precision == 64:
         return 8 * Nx * Ni + 16 * H * Ni                         # omega^(s+1) rows -> omega-hat
-    if name == "k_thomas_cluster":
+    if name in ("k_thomas_cluster", "k_thomas_cta", "k_thomas_wide"):
         return C * H * Ni + 8 * H * Ni + C * H * Ny              # omega-hat and cp read, psi-hat written
     if name == "k_thomas_maps":
         return C * H * Ni + 8 * H * Ni                           # omega-hat, cp read once
     if name == "k_thomas_apply":
         return C * H * Ni                                        # psi-hat written (its re-read of
                                                                  # omega-hat and cp is not counted)
-    if name == "k_ifft_thom":
+    if name in ("k_ifft_thom", "k_rows_inv") and precision == 64:
         return 16 * H * Ni + 8 * N + 8 * 6 * Nx                  # psi-hat -> psi, + Thom rows
     if name == "k_maxuv_dt":
         return 8 * N

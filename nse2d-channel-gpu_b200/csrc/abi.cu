@@ -175,7 +175,7 @@ int nse2d_step_profiled(nse2d_ctx* ctx, double* step_ms, double* fft_ms, double*
             cudaEventElapsedTime(&ms, ev[k], ev[k + 1]);
             const std::string name = step_kernel_name(c, k);
             tot += ms;
-            if (name.rfind("k_fft_fwd", 0) == 0 || name.rfind("k_ifft", 0) == 0) fft += ms;
+            if (name.rfind("k_fft_fwd", 0) == 0 || name.rfind("k_ifft", 0) == 0 || name.rfind("k_rows", 0) == 0) fft += ms;
             if (name.rfind("k_thomas", 0) == 0) tri += ms;
         }
         if (step_ms) *step_ms = tot;

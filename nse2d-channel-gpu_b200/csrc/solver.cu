@@ -787,7 +787,7 @@ static int launch_thomas_cta(Context* c, cudaStream_t s, bool homog) {
 // Launches of one tridiagonal solve: 1 (one-CTA or cluster form) or 2 (maps, apply); part i of them.
 int thomas_launches(const Context* c) { return thomas_cta(c) || c->thomas_cluster ? 1 : 2; }
 const char* thomas_kernel_name(const Context* c, int i) {
-    if (thomas_cta(c)) return "k_thomas_cta";
+    if (thomas_cta(c)) return c->Ni > SC_MAX_NI ? "k_thomas_wide" : "k_thomas_cta";
     if (c->thomas_cluster) return "k_thomas_cluster";
     return i == 0 ? "k_thomas_maps" : "k_thomas_apply";
 }
@@ -937,8 +937,8 @@ const char* step_kernel_name(const Context* c, int k) {
     if (k < 0 || k >= 3 * per) return "";
     const int i = k % per;
     if (i == 0) return c->stage_tma ? "k_stage_tma" : "k_stage";
-    if (i == 1) return "k_fft_fwd";
-    if (i == per - 1) return "k_ifft_thom";
+    if (i == 1) return c->band ? "k_rows_fwd" : "k_fft_fwd";
+    if (i == per - 1) return c->band ? "k_rows_inv" : "k_ifft_thom";
     return thomas_kernel_name(c, i - 2);
 }
 

@@ -153,14 +153,14 @@ template <int M> static int fft32_inv_t(Context* c, Fft32Params& p, cudaStream_t
     }
 
 static int fft32_fwd(Context* c, const float* src, cudaStream_t s) {
-    if (band_rows_ok(c->M)) return band32_rows_fwd(c, src, s);
+    if (c->band) return band32_rows_fwd(c, src, s);
     Fft32Params p = fft32_params(c);
     p.src = src;
     NSE_FFT32_DISPATCH(fft32_fwd_t)
 }
 
 static int fft32_inv(Context* c, float* w_out, bool advance, cudaStream_t s) {
-    if (band_rows_ok(c->M)) return band32_rows_inv(c, w_out, advance, s);
+    if (c->band) return band32_rows_inv(c, w_out, advance, s);
     Fft32Params p = fft32_params(c);
     p.psi = c->psif;
     p.w = w_out;
@@ -240,8 +240,8 @@ const char* step32_kernel_name(const Context* c, int k) {
     if (k < 0 || k >= 3 * per) return "";
     const int i = k % per;
     if (i == 0) return c->stage32_tma ? "k_stage32_tma" : "k_stage32";
-    if (i == 1) return "k_fft_fwd32";
-    if (i == per - 1) return "k_ifft_thom32";
+    if (i == 1) return c->band ? "k_rows_fwd" : "k_fft_fwd32";
+    if (i == per - 1) return c->band ? "k_rows_inv" : "k_ifft_thom32";
     return thomas_kernel_name(c, i - 2);
 }
 

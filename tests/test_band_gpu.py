@@ -138,3 +138,21 @@ def test_bands_while_they_fit_the_device(nse, cuda, precision, Nx, Ny, bands):
     names = [s.lib.nse2d_step_kernel_name(s.h, k).decode() for k in range(s.launches_per_step())]
     assert ("k_band_inv_stage_fwd" in names) == bands, names
     s.close()
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("Nx,Ny,names", [
+    (1024, 700, ("k_rows_fwd", "k_thomas_wide", "k_rows_inv")), (2048, 300, ("k_rows_fwd", "k_thomas_cta", "k_rows_inv")),
+    (16, 129, ("k_fft_fwd", "k_thomas_cta", "k_ifft_thom")), (4096, 1500, ("k_fft_fwd", "k_thomas_cluster", "k_ifft_thom"))])
+def test_the_names_are_those_of_the_kernels(nse, cuda, precision, Nx, Ny, names):
+    """A step by separate kernels names the transforms and the solve that its grid uses, and nse2d_step_profiled counts
+    them as transforms and as solve."""
+    s = nse.Solver(Nx=Nx, Ny=Ny, Lx=2 * np.pi, stretch=1, beta=1.0, Ub=1.0, Reb=2000.0, adapt=1, precision=precision)
+    got = [n for n, _ in s.step_timed(1)]
+    want = [n + "32" if precision == 32 and n in ("k_fft_fwd", "k_ifft_thom") else n for n in names]
+    assert [n for n in got if not n.startswith(("k_stage", "k_maxuv"))] == want * 3, got
+    ms = [ctypes.c_double() for _ in range(3)]
+    assert s.lib.nse2d_step_profiled(s.h, *[ctypes.byref(x) for x in ms], None) == 0
+    step, fft, tri = (x.value for x in ms)
+    assert fft > 0 and tri > 0 and fft + tri < step
+    s.close()
