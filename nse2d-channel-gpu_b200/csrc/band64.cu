@@ -7,6 +7,21 @@ namespace nse2d {
 // shorter ones have fewer points than a warp. Bands: of rows of up to 1024 points (see band.cuh), by band_setup.
 bool band_rows_ok(int M) { return M >= 32 && M <= 1024; }
 bool band_stage_ok(int M) { return M >= 32 && M <= 512; }
+// Rows of 2048 points have four to a CTA of 256 threads, and two (FP32: three) CTAs to an SM: a launch takes as long as
+// its last round over the SMs. Where that round is less than a quarter full (the fourth, which begins the next wave in
+// FP32: half) the transforms of one row per CTA are faster. A step by four rows and by one, us: FP64 2048x600 123 and
+// 117, x1184 166 and 182, x1200 193 and 187, x1800 254 and 249, x2300 293 and 316; FP32 x600 96 and 94, x1184 119 and
+// 126, x1200 133 and 129, x1800 184 and 170, x2049 193 and 182, x2300 214 and 225.
+static int row_round(const Context* c) { return Band<1024>::ROWS_G * c->num_sms; }
+bool rows_by_band(const Context* c) {
+    if (!band_rows_ok(c->M)) return false;
+    if (c->M < 1024) return true;
+    const int round = row_round(c), full = c->Ni / round, rest = c->Ni % round;
+    return full < 1 || full > 3 || rest == 0 || rest >= (full == 3 ? round / 2 : round / 4);
+}
+// The Poisson solve alone, three launches from the host, also while the rows of 2048 points are fewer than a round:
+// 2048x33 20.7 and 16.6 us, 2048x300 24.7 and 21.8 (in a step the four rows to a CTA are the faster there too, 66 and 68).
+bool solve_rows_by_band(const Context* c) { return c->band && !(c->M == 1024 && c->Ni < row_round(c)); }
 
 static BandParams<double> band_params(const Context* c) {
     BandParams<double> p{};

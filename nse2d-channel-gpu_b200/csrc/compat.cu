@@ -632,7 +632,7 @@ void Poisson2D_Z2Z::solve(const Real* d_omega, Real* d_psi, Real, Real psi_bot, 
     cudaEvent_t* e = impl_->e;
     int rc = 0;
     if (profile) cudaEventRecord(e[0], s);
-    rc |= launch_fft_fwd(c, d_omega, s);
+    rc |= launch_fft_fwd(c, d_omega, s, !solve_rows_by_band(c));
     if (profile) { cudaEventRecord(e[1], s); cudaEventRecord(e[2], s); }
     rc |= launch_thomas(c, s);
     if (profile) cudaEventRecord(e[3], s);
@@ -645,7 +645,7 @@ void Poisson2D_Z2Z::solve(const Real* d_omega, Real* d_psi, Real, Real psi_bot, 
         acc_tridiag_ms += b;
         cudaEventRecord(e[0], s);
     }
-    rc |= launch_ifft_thom(c, d_psi, nullptr, 0, false, false, s);
+    rc |= launch_ifft_thom(c, d_psi, nullptr, 0, false, false, s, false, !solve_rows_by_band(c));
     if (profile) {
         cudaEventRecord(e[1], s);
         cudaEventSynchronize(e[1]);

@@ -31,7 +31,7 @@ int context_create(const Config& cfg, Context** out);
 void context_destroy(Context* c);
 int launch_stage(Context* c, int stage, const double* w_in, const double* w_n, double* w_out, cudaStream_t s,
                  double* rhs_out = nullptr);
-int launch_fft_fwd(Context* c, const double* src, cudaStream_t s, bool general = false);
+int launch_fft_fwd(Context* c, const double* src, cudaStream_t s, bool general = false);   // general: not k_rows_*
 int launch_thomas(Context* c, cudaStream_t s, bool general = false);
 int launch_thomas_maps(Context* c, cudaStream_t s, bool homog = false);
 int launch_thomas_apply(Context* c, cudaStream_t s, bool homog = false);
@@ -39,6 +39,8 @@ int launch_thomas_cluster(Context* c, cudaStream_t s, bool homog = false);
 // row-band kernels (band64.cu, band32.cu)
 bool band_rows_ok(int M);
 bool band_stage_ok(int M);
+bool rows_by_band(const Context* c);           // which row transforms a channel takes
+bool solve_rows_by_band(const Context* c);     // and its Poisson solve alone
 int band_setup(Context* c);              // band_fit and band_load of a channel (before its psi-hat is allocated)
 int band_setup32(Context* c);
 int band_stage(Context* c, int stage, bool inv, double* w_in, const double* w_n, double* w_out, double* rhs_out,

@@ -327,7 +327,7 @@ int context_create(const Config& cfg, Context** out) {
     if (dalloc(&c->hat, (size_t)Ny * c->Hp) || dalloc(&c->cp, (size_t)c->Ni * c->Hp) ||
         dalloc(&c->wN, (size_t)c->M + 1))
         return fail();
-    c->band = band_rows_ok(c->M);
+    c->band = rows_by_band(c);
     if (cfg.precision == 64 && (band_setup(c) || (c->band_fit && dalloc(&c->hat2, (size_t)Ny * c->Hp)))) return fail();
     c->thomas_nseg = (c->Ni + TS_ROWS - 1) / TS_ROWS;
     c->thomas_nsb = (c->thomas_nseg + TS_NW - 1) / TS_NW;
@@ -836,9 +836,10 @@ int launch_maxuv(Context* c, const double* psi, bool set_dt, cudaStream_t s, boo
 // Poisson solve of the reference (src/poisson.cuh:83-118): omega -> psi. general: by the transforms and the solve
 // that every grid has, whatever this one uses in its steps.
 int poisson_solve(Context* c, const double* w, double* psi, cudaStream_t s, bool general) {
-    if (launch_fft_fwd(c, w, s, general)) return -1;
+    const bool rows = general || !solve_rows_by_band(c);
+    if (launch_fft_fwd(c, w, s, rows)) return -1;
     if (launch_thomas(c, s, general)) return -1;
-    if (launch_ifft_thom(c, psi, nullptr, 0, false, false, s, false, general)) return -1;
+    if (launch_ifft_thom(c, psi, nullptr, 0, false, false, s, false, rows)) return -1;
     return 0;
 }
 

@@ -127,7 +127,7 @@ static Fft32Params fft32_params(Context* c) {
     return p;
 }
 
-// rows of 64 to 2048 points have the row-band transforms
+// rows of 64 to 2048 points have the row-band transforms, but for some grids of 2048 (rows_by_band)
 template <int M> static int fft32_fwd_t(Context* c, Fft32Params& p, cudaStream_t s) {
     const size_t sm = fft32_smem_bytes(M);
     NSE_CUDA_TRY(cudaFuncSetAttribute(k_fft_fwd32<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -147,8 +147,8 @@ template <int M> static int fft32_inv_t(Context* c, Fft32Params& p, cudaStream_t
     switch (c->M) {                                                                \
         case 2: return FN<2>(c, p, s);       case 4: return FN<4>(c, p, s);        \
         case 8: return FN<8>(c, p, s);       case 16: return FN<16>(c, p, s);      \
-        case 2048: return FN<2048>(c, p, s); case 4096: return FN<4096>(c, p, s);  \
-        case 8192: return FN<8192>(c, p, s);                                       \
+        case 1024: return FN<1024>(c, p, s); case 2048: return FN<2048>(c, p, s);  \
+        case 4096: return FN<4096>(c, p, s); case 8192: return FN<8192>(c, p, s);  \
         default: set_error("no FFT kernel for M = %d", c->M); return -1;           \
     }
 

@@ -673,8 +673,10 @@ __device__ __forceinline__ void fwd_last_pass_split(const cpx<T>* buf, const cpx
 // a row is read as M complex points z_n = x_2n + i x_2n+1, scattered by cp.async into the
 // digit-reversed layout; after the passes the split step writes X_k, k = 0..M:
 //   E_k = (Z_k + conj Z_{M-k}) / 2,  O_k = -i (Z_k - conj Z_{M-k}) / 2,  X_k = E_k + W_{2M}^k O_k.
-// The rows go from the last to the first: the stage before has just written the last ones, which are still in L2 on
-// grids whose fields are not (4096x2049, 67 MB a field: 27.7 -> 25.9 us; FP32 fields no change, first to last there).
+// Rows of 4096 points and more go from the last to the first: the stage before has just written the last ones, which are
+// still in L2 on grids whose fields are not (4096x2049, 67 MB a field: 32.4 -> 30.6 us; FP32 fields no change, first to
+// last there). Fields of shorter rows are in L2 as a whole, where that order gains nothing (2048x2300, both orders: step
+// 308 first to last, 316 last to first).
 template <int M>
 static __global__ void __launch_bounds__(IP_NT, 5) k_fft_fwd(FftParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -682,7 +684,9 @@ static __global__ void __launch_bounds__(IP_NT, 5) k_fft_fwd(FftParams p) {
     cpx<double>* buf = reinterpret_cast<cpx<double>*>(smem_raw);
     const int je = p.row0 + p.nrows;
     constexpr int R0 = p16_plan<M>::R(0), NB0 = M / R0;
-    for (int j = je - 1 - blockIdx.x; j >= p.row0; j -= gridDim.x) {  // rows strided over one wave of CTAs, last first
+    constexpr bool kLastFirst = M >= 2048;
+    for (int r = p.row0 + blockIdx.x; r < je; r += gridDim.x) {      // rows strided over one wave of CTAs
+        const int j = kLastFirst ? je - 1 - (r - p.row0) : r;
         const double2* row = reinterpret_cast<const double2*>(p.src + (size_t)j * p.Nx);
         // pass 0 from global: thread t transforms the points t + NB0 r (a coalesced column)
 #pragma unroll 1

@@ -156,3 +156,32 @@ def test_the_names_are_those_of_the_kernels(nse, cuda, precision, Nx, Ny, names)
     step, fft, tri = (x.value for x in ms)
     assert fft > 0 and tri > 0 and fft + tri < step
     s.close()
+
+
+@pytest.mark.parametrize("Ny,rows", [(5, True), (594, True), (595, False), (739, False), (742, True), (1778, True), (1779, False), (2073, False),
+                                     (2074, True), (2371, True)])
+def test_rows_of_2048_points_either_side_of_a_round(nse, oracle, cuda, Ny, rows):
+    """Four rows of 2048 points to a CTA, unless their last round over 148 SMs is nearly empty: the transforms named in
+    the step, the Poisson solve (which takes one row to a CTA on grids of less than a round too) against the oracle at
+    the 1e-12 of the other solves, and an FP32-bulk step against the FP64 one at the 1e-5 of its psi."""
+    from test_fp32_gpu import omega0, rel
+    torch = cuda
+    cfg = dict(Nx=2048, Ny=Ny, Lx=2 * np.pi, stretch=1, beta=1.0, Ub=1.0, Reb=2000.0, adapt=1)
+    a, b = nse.Solver(**cfg), nse.Solver(precision=32, **cfg)
+    for s in (a, b):
+        names = [s.lib.nse2d_step_kernel_name(s.h, k).decode() for k in range(s.launches_per_step())]
+        assert ("k_rows_fwd" in names) == rows and ("k_rows_inv" in names) == rows, names
+    w = np.random.default_rng(Ny).standard_normal((Ny, 2048))
+    wd = torch.from_numpy(w).cuda()
+    pd = torch.zeros_like(wd)
+    a.poisson_solve(wd, pd)
+    torch.cuda.synchronize()
+    m = oracle.metrics(2048, Ny, 2 * np.pi, 1.0, 1, 1.0)
+    assert relerr(pd.cpu().numpy(), oracle.poisson_solve(w, 2 * np.pi, m, 0.0, 2.0)) < 1e-12
+    w0 = omega0(2048, Ny, a.metric(0))
+    for s in (a, b):
+        s.set_omega(w0)
+        s.step(1)
+    assert rel(b.fields()[1], a.fields()[1]) < 1e-5
+    a.close()
+    b.close()
