@@ -121,9 +121,10 @@ int  nse2d_get_field(nse2d_ctx* ctx, int which, double* host, cudaStream_t s);
 /* Advance nsteps SSPRK(3,3) steps, asynchronously. With adapt, dt is computed on the
  * device before every step (max |u|, |v|, |v| a, CFL and viscous limits, trimming to
  * the next output time); otherwise the dt of nse2d_set_dt / dt_init is used. Grids of up to
- * 514 rows of 64 to 1024 points (without a model, MMS forcing or closure_diag) take all nsteps
- * in one cooperative launch, unless s is being captured; use_graph: the others replay one
- * captured CUDA graph per step. */
+ * 514 rows of 64 to 1024 points (without a model, MMS forcing or closure_diag) take up to 64
+ * steps in one cooperative launch, unless s is being captured or another channel of the process
+ * has steps in flight on another stream of the device; use_graph: the others replay one
+ * captured CUDA graph per step. The fields are the same to the bit in either form. */
 int  nse2d_step(nse2d_ctx* ctx, int nsteps, int use_graph, cudaStream_t s);
 /* The tridiagonal solve of the Poisson step: clusters != 0 selects the one-pass form on
  * persistent thread-block clusters (the default where it can be resident: fastest for a
@@ -187,7 +188,7 @@ int  nse2d_get_time(nse2d_ctx* ctx, double* t, double* dt, long long* step, doub
 
 /* Run the time loop on the device (src/main.cu:434-551) until something needs the host:
  * steps are taken inside one CUDA graph launch (a WHILE node around the captured step), or one
- * cooperative launch (see nse2d_step; at most 8192 steps each, without device statistics), and
+ * cooperative launch (see nse2d_step; at most 256 steps each, without device statistics), and
  * the run stops after the step at which
  *   NSE2D_HALT_OUTPUT     t has reached min(next_snap, next_diag) (within the snap tolerance),
  *   NSE2D_HALT_STATS      the step count is a multiple of stats_every (0: never),

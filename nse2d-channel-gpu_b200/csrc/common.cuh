@@ -139,6 +139,13 @@ struct Context {
     double band_load = 0.0;        // its bands, of the most rows, over those that the device holds at once
     int band_share = 1;            // channels that run at the same time as this one (the branches of an ensemble)
     int steps_R = 0;               // rows of a band of the steps in one launch (0: not used)
+    // the last call that stepped the channel, for the others of this process (beside_others); under their mutex
+    int device = 0;
+    bool stepped = false;
+    bool steps_pending = false;    // steps_done was recorded and not yet seen to have passed
+    bool overlapped = false;       // it ran beside another channel's steps
+    cudaStream_t steps_on = nullptr;
+    cudaEvent_t steps_done = nullptr;
     bool plain_step = false;       // a step of separate transforms and stages (nse2d_step_profiled times them apart; ensembles)
     double* cp = nullptr;          // elimination table [Ni][Hp]
     cpx<double>* tw = nullptr;     // per-pass twiddle pairs of the Nx/2-point transform

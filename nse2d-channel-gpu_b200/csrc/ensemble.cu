@@ -102,6 +102,7 @@ int ensemble_step(Ensemble* e, int nsteps, cudaStream_t s) {
     NSE_CUDA_TRY(cudaMemcpyAsync(e->d_count, &nsteps, sizeof(int), cudaMemcpyHostToDevice, s));
     NSE_CUDA_TRY(cudaStreamSynchronize(s));     // nsteps lives on this stack frame
     NSE_CUDA_TRY(cudaGraphLaunch(e->exec, s));
+    note_steps(e->m[0], s);                     // one member stands for all of them
     return 0;
 }
 

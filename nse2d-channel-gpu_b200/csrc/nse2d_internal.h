@@ -90,6 +90,7 @@ int launch_maxuv(Context* c, const double* psi, bool set_dt, cudaStream_t s, boo
 int poisson_solve(Context* c, const double* w, double* psi, cudaStream_t s, bool general = false);
 int enqueue_step(Context* c, cudaStream_t s, bool store_rhs);
 int launches_per_step(const Context* c);
+void note_steps(Context* c, cudaStream_t s);       // steps of c were enqueued on s
 int enqueue_step_timed(Context* c, cudaStream_t s, cudaEvent_t* ev, bool store_rhs = false);
 const char* step_kernel_name(const Context* c, int k);
 int run_steps(Context* c, int nsteps, bool use_graph, cudaStream_t s, bool store_rhs);

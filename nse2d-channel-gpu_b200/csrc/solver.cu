@@ -2,6 +2,7 @@
 // SSPRK(3,3) step. Written for this project; the setup follows the reference's
 // src/grid.cu:7-94 (metrics), src/main.cu:49-87 (derived constants), src/poisson.cu:16-68
 // (kx^2 and the elimination table) and src/main.cu:210-213 (initial solve + Thom).
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstring>
@@ -261,6 +262,80 @@ template <typename T> static int dalloc(T** p, size_t n) {
     return 0;
 }
 
+// ---- channels that are stepped at the same time ----
+// Steps in one launch want the device: two cooperative launches run one after the other, where steps by launches
+// overlap. us for a step of each of n channels on n streams, in one launch and by launches: 128x129 n = 2 44 and 34, 4
+// 87 and 41, 16 345 and 99; 1024x513 n = 2 106 and 88, 16 842 and 634; FP32 256x257 n = 4 91 and 46. So a call that
+// steps looks whether another channel of the process still has steps in flight on another stream of the device, or
+// came beside its own last ones (one channel in one launch and the others by launches would be the slowest: 256x257
+// n = 2 62 us; both in one launch 50, both by launches 39). Channels whose launches fit the device together do run at
+// the same time (64x65 n = 2 22 and 32). The list holds the contexts that exist, and each context what its last
+// stepping call left; nothing else depends on it, and the fields are the same to the bit either way.
+struct Channels {
+    std::mutex m;
+    std::vector<Context*> all;
+};
+static Channels& channels() {
+    static Channels* c = new Channels;                       // outlives every context
+    return *c;
+}
+static void channels_enter(Context* c) {
+    std::lock_guard<std::mutex> lock(channels().m);
+    channels().all.push_back(c);
+}
+static void channels_leave(Context* c) {
+    std::lock_guard<std::mutex> lock(channels().m);
+    auto& a = channels().all;
+    a.erase(std::remove(a.begin(), a.end(), c), a.end());
+}
+// an event query is refused while another thread captures a stream in the global mode
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+// one handle stands for a stream of every thread
+static bool same_stream(cudaStream_t a, cudaStream_t b) { return a == b && a != cudaStreamPerThread; }
+static bool beside_others(Context* c, cudaStream_t s) {
+    std::lock_guard<std::mutex> lock(channels().m);
+    bool busy = false;
+    auto ctas = [](const Context* x) { return x->steps_R ? std::min(x->num_sms, x->Ni) : x->num_sms; };
+    int used = ctas(c);                                      // an SM holds one CTA of k_steps
+    for (Context* o : channels().all) {
+        if (o == c || !o->steps_pending || o->device != c->device || same_stream(o->steps_on, s)) continue;
+        RelaxedCapture relaxed;
+        const cudaError_t e = cudaEventQuery(o->steps_done);
+        if (e == cudaErrorNotReady) {
+            cudaGetLastError();
+            used += ctas(o);
+            if ((busy = used > c->num_sms)) {
+                o->overlapped = true;
+                break;
+            }
+            continue;
+        }
+        o->steps_pending = false;
+    }
+    const bool beside = busy || c->overlapped;
+    c->overlapped = busy;
+    return beside;
+}
+// Called after every enqueueing of steps. Channels that all step on the legacy default stream never overlap, and need
+// no event.
+void note_steps(Context* c, cudaStream_t s) {
+    std::lock_guard<std::mutex> lock(channels().m);
+    auto& a = channels().all;
+    c->stepped = true;
+    c->steps_on = s;
+    c->steps_pending = false;
+    if (a.size() < 2) return;
+    bool seen = s != nullptr && s != cudaStreamLegacy;
+    for (const Context* o : a) seen = seen || (o != c && o->stepped && o->device == c->device && !same_stream(o->steps_on, s));
+    if (!seen) return;
+    c->steps_pending = cudaEventRecord(c->steps_done, s) == cudaSuccess;
+    if (!c->steps_pending) cudaGetLastError();
+}
+
 int context_create(const Config& cfg, Context** out) {
     *out = nullptr;
     if (cfg.Nx < 4 || (cfg.Nx & (cfg.Nx - 1)) != 0) {
@@ -501,12 +576,17 @@ int context_create(const Config& cfg, Context** out) {
     Ctl h{};
     h.t = 0.0; h.dt = cfg.dt_init; h.next_out = 1e300; h.next_snap = 1e300; h.next_diag = 1e300;
     if (cudaMemcpy(c->ctl, &h, sizeof(Ctl), cudaMemcpyHostToDevice) != cudaSuccess) { set_error("ctl upload"); return fail(); }
+    c->device = dev;
+    if (cudaEventCreateWithFlags(&c->steps_done, cudaEventDisableTiming) != cudaSuccess) { set_error("event"); return fail(); }
+    channels_enter(c);
     *out = c;
     return 0;
 }
 
 void context_destroy(Context* c) {
     if (!c) return;
+    channels_leave(c);
+    if (c->steps_done) cudaEventDestroy(c->steps_done);
     RowTables& rt = c->rt;
     for (double* p : {rt.y, rt.a_node, rt.a_edge, rt.dy_edge, rt.w_node, rt.wt_node, rt.frow, rt.fx, rt.st_cj, rt.st_ap, rt.st_am, rt.asub, rt.csup,
                       rt.inv_csup, rt.mms_g, rt.mms_gpp, rt.mms_sin2, rt.mms_sk, rt.mms_s2k, c->w, c->w1, c->w2,
@@ -956,23 +1036,43 @@ int refresh_maxima(Context* c, cudaStream_t s) {
     return launch_maxuv(c, c->psi, false, s, true);
 }
 
-// Steps in one launch (steps.cuh): where the grid's bands are all resident, without a model between the stages, and
-// not into a stream that is being captured (nor inside an ensemble, whose members share the device).
-static bool steps_ok(const Context* c, cudaStream_t s) {
-    if (!c->steps_R || !(c->prec32 ? band_step32(c) : band_step(c)) || c->closure_net) return false;
+static bool capturing(cudaStream_t s) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return true;
     }
-    return st == cudaStreamCaptureStatusNone;
+    return st != cudaStreamCaptureStatusNone;
 }
+// Steps in one launch (steps.cuh): where the grid's bands are all resident, without a model between the stages, not
+// into a stream that is being captured, nor inside an ensemble, whose members share the device, nor beside the steps
+// of another channel.
+static bool steps_ok(Context* c, cudaStream_t s) {
+    if (!c->steps_R || !(c->prec32 ? band_step32(c) : band_step(c)) || c->closure_net) return false;
+    return !capturing(s) && !beside_others(c, s);
+}
+// Steps of a launch. The launch keeps the device, and a kernel of another stream waits until it ends, so a long call is
+// cut: 64 steps are 1.3 to 3.4 ms, and the next launch costs 0.1 us a step (128x129 21.6 us a step instead of 21.5,
+// 1024x513 52.2 and 52.2; of 500 steps of 1024x513 in one launch another stream's small kernel waited 26 ms). A run,
+// whose host looks for the halt after every launch, takes 256 (0.05 us a step).
+constexpr int kStepsPerLaunch = 64, kRunStepsPerLaunch = 256;
 
-// nsteps steps: in one launch where the grid allows it; else, with use_graph, the step is captured once into a
-// CUDA graph and replayed.
+static int enqueue_steps(Context* c, int nsteps, bool use_graph, cudaStream_t s, bool store_rhs);
+
+// nsteps steps: in one launch (of kStepsPerLaunch each) where the grid allows it; else, with use_graph, the step is
+// captured once into a CUDA graph and replayed.
 int run_steps(Context* c, int nsteps, bool use_graph, cudaStream_t s, bool store_rhs) {
     if (nsteps <= 0) return 0;
-    if (steps_ok(c, s)) return launch_steps(c, nsteps, 0, store_rhs ? 1 : 0, s);
+    const int rc = enqueue_steps(c, nsteps, use_graph, s, store_rhs);
+    if (!capturing(s)) note_steps(c, s);
+    return rc;
+}
+static int enqueue_steps(Context* c, int nsteps, bool use_graph, cudaStream_t s, bool store_rhs) {
+    if (steps_ok(c, s)) {
+        for (int left = nsteps; left > 0; left -= kStepsPerLaunch)
+            if (launch_steps(c, std::min(left, kStepsPerLaunch), 0, store_rhs && left <= kStepsPerLaunch ? 1 : 0, s)) return -1;
+        return 0;
+    }
     if (!use_graph || store_rhs) {
         for (int i = 0; i < nsteps; ++i)
             if (enqueue_step(c, s, store_rhs && i == nsteps - 1)) return -1;
@@ -1010,13 +1110,12 @@ static __global__ void k_loop_cond(Ctl* ctl, cudaGraphConditionalHandle h) {
 // a WHILE node whose body is one captured step followed by k_loop_cond. The run fields of the
 // control block must be set (run = 1, halt = 0, run_budget > 0) before the launch.
 int run_until_halt(Context* c, cudaStream_t s) {
-    if (!c->stats_dev && steps_ok(c, s)) {
-        for (;;) {                                           // launches of at most 8192 steps (0.1 to 0.5 s)
-            if (launch_steps(c, 8192, 1, 2, s)) return -1;
-            NSE_CUDA_TRY(cudaMemcpyAsync(c->h_ctl, c->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
-            NSE_CUDA_TRY(cudaStreamSynchronize(s));
-            if (c->h_ctl->halt || (c->h_ctl->nonfinite & 2)) return 0;
-        }
+    while (!c->stats_dev && steps_ok(c, s)) {                // by launches from where another channel begins to step
+        if (launch_steps(c, kRunStepsPerLaunch, 1, 2, s)) return -1;
+        note_steps(c, s);
+        NSE_CUDA_TRY(cudaMemcpyAsync(c->h_ctl, c->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
+        NSE_CUDA_TRY(cudaStreamSynchronize(s));
+        if (c->h_ctl->halt || (c->h_ctl->nonfinite & 2)) return 0;
     }
     if (!c->run_exec) {
         if (!c->cap_stream) NSE_CUDA_TRY(cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
@@ -1054,6 +1153,7 @@ int run_until_halt(Context* c, cudaStream_t s) {
         NSE_CUDA_TRY(e);
     }
     NSE_CUDA_TRY(cudaGraphLaunch(c->run_exec, s));
+    note_steps(c, s);
     return 0;
 }
 

@@ -60,6 +60,38 @@ static void gave_up(int precision) {
     OK(nse2d_destroy(x));
 }
 
+// Two channels on two streams: the form of a step while the other one's steps are in flight, and alone.
+static void shared(int precision) {
+    cudaStream_t q[2];
+    for (auto& s : q) OK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    nse2d_ctx *a = channel(1024, 513, precision), *b = channel(128, 129, precision), *c = channel(128, 129, precision);
+    for (nse2d_ctx* x : {a, b, c}) start(x);
+    std::printf("one_launch %d\n", a->c->steps_R > 0 && b->c->steps_R > 0);
+    OK(nse2d_step(a, 2000, 1, q[0]));                        // 0.1 s
+    OK(nse2d_step(b, 3, 1, q[1]));
+    const bool busy = cudaStreamQuery(q[0]) == cudaErrorNotReady;
+    std::printf("still_busy %d\nby_launches_beside_another %d\n", busy, b->c->graph_exec != nullptr);
+    OK(cudaDeviceSynchronize());
+    OK(nse2d_step(c, 3, 1, q[1]));
+    std::printf("by_launches_alone %d\n", c->c->graph_exec != nullptr);
+    OK(cudaDeviceSynchronize());
+    // a was found in flight: its next call is by launches, and the one after that, with nobody beside it, is not
+    for (int k = 0; k < 2; ++k) {
+        if (a->c->graph_exec) { cudaGraphExecDestroy(a->c->graph_exec); a->c->graph_exec = nullptr; }
+        OK(nse2d_step(a, 2, 1, q[0]));
+        std::printf("first_channel_by_launches_%d %d\n", k, a->c->graph_exec != nullptr);
+        OK(cudaDeviceSynchronize());
+    }
+    const size_t n = (size_t)128 * 129;
+    std::vector<double> f[4];
+    for (auto& v : f) v.resize(n);
+    OK(nse2d_get_fields(b, f[0].data(), f[1].data(), 0, nullptr));
+    OK(nse2d_get_fields(c, f[2].data(), f[3].data(), 0, nullptr));
+    std::printf("same_bits %d\n", f[0] == f[2] && f[1] == f[3]);
+    for (nse2d_ctx* x : {a, b, c}) OK(nse2d_destroy(x));
+    for (auto& s : q) cudaStreamDestroy(s);
+}
+
 // A wait of the model's kernels that has timed out: gradients and a training step, and the same once it is reported.
 struct Model {
     static constexpr int Nx = 32, Ny = 17, H = 16;
@@ -127,6 +159,7 @@ int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "gave_up") gave_up(std::atoi(argv[2]));
     else if (what == "model_wait") model_wait();
+    else if (what == "shared") shared(std::atoi(argv[2]));
     else return 2;
     return 0;
 }

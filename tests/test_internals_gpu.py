@@ -46,3 +46,15 @@ def test_a_model_wait_that_timed_out_is_an_error_once(driver):
     assert got["gradients_after"] == 0 and got["loss_after_is_right"] == 1
     assert got["weights_kept"] == 1
     assert got["train_after"] == 0 and got["weights_after_are_the_first_steps"] == 1
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_steps_beside_another_channels_are_by_launches(driver, precision):
+    """A step while another channel's steps are in flight on another stream is by launches, which overlap, and so is
+    the next one of the channel that it came beside; in one launch otherwise. The same bits either way."""
+    got = driver("shared", precision)
+    assert got["one_launch"] == 1 and got["still_busy"] == 1
+    assert got["by_launches_beside_another"] == 1
+    assert got["by_launches_alone"] == 0
+    assert got["first_channel_by_launches_0"] == 1 and got["first_channel_by_launches_1"] == 0
+    assert got["same_bits"] == 1
