@@ -157,7 +157,8 @@ typedef struct nse2d_plan {
 int  nse2d_get_plan(nse2d_ctx* ctx, nse2d_plan* plan);
 int  nse2d_set_plan(nse2d_ctx* ctx, const nse2d_plan* plan);
 /* Times every plan the context can use over trial_steps graph-replayed steps from the current state
- * and keeps the fastest (best and its ms per step are reported; either may be NULL). The fields
+ * and keeps the fastest (best and its ms per step are reported; either may be NULL). The steps are
+ * by launches on every grid, also where nse2d_step takes them in one (whose time no plan changes). The fields
  * and the control block are saved before and restored after, so only the plan changes; two
  * temporary fields are allocated for that. Synchronous. */
 int  nse2d_autotune_plan(nse2d_ctx* ctx, int trial_steps, nse2d_plan* best, double* ms_per_step, cudaStream_t s);

@@ -278,8 +278,10 @@ int nse2d_set_plan(nse2d_ctx* ctx, const nse2d_plan* plan) {
 }
 
 // Every plan the context can use, timed over trial_steps graph-replayed steps from the current
-// state; the state (fields and control block) is saved before and restored after, so only the
-// plan changes. The fastest plan stays set.
+// state, on grids whose steps go in one launch too: there the plan governs what else is launched
+// (steps of an ensemble, beside another channel, with a model; the profiled step). The state
+// (fields and control block) is saved before and restored after, so only the plan changes. The
+// fastest plan stays set.
 int nse2d_autotune_plan(nse2d_ctx* ctx, int trial_steps, nse2d_plan* best, double* ms_per_step, cudaStream_t s) {
     CHECK_CTX(ctx);
     if (trial_steps <= 0) { set_error("nse2d_autotune_plan: trial_steps must be positive"); return -1; }
@@ -309,6 +311,11 @@ int nse2d_autotune_plan(nse2d_ctx* ctx, int trial_steps, nse2d_plan* best, doubl
         NSE_CUDA_TRY(cudaStreamSynchronize(s));
         return 0;
     };
+    struct ByLaunches {
+        Context* c;
+        explicit ByLaunches(Context* x) : c(x) { c->by_launches = true; }
+        ~ByLaunches() { c->by_launches = false; }
+    } by_launches(c);
     const bool st_ok = c->prec32 ? c->stage32_tma_ok : c->stage_tma_ok;
     const bool mf_ok = c->rowfft_pf_ok && c->cfg.adapt && !c->prec32;   // the fused max needs the prefetching form
     if (cudaEventCreate(&a) != cudaSuccess || cudaEventCreate(&b) != cudaSuccess) { set_error("event"); rc = -1; }

@@ -139,6 +139,7 @@ struct Context {
     double band_load = 0.0;        // its bands, of the most rows, over those that the device holds at once
     int band_share = 1;            // channels that run at the same time as this one (the branches of an ensemble)
     int steps_R = 0;               // rows of a band of the steps in one launch (0: not used)
+    bool by_launches = false;      // no steps in one launch (while plans are timed: they govern the steps by launches)
     // the last call that stepped the channel, for the others of this process (beside_others); under their mutex
     int device = 0;
     bool stepped = false;

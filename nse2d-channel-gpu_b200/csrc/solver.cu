@@ -1048,7 +1048,7 @@ static bool capturing(cudaStream_t s) {
 // into a stream that is being captured, nor inside an ensemble, whose members share the device, nor beside the steps
 // of another channel.
 static bool steps_ok(Context* c, cudaStream_t s) {
-    if (!c->steps_R || !(c->prec32 ? band_step32(c) : band_step(c)) || c->closure_net) return false;
+    if (!c->steps_R || c->by_launches || !(c->prec32 ? band_step32(c) : band_step(c)) || c->closure_net) return false;
     return !capturing(s) && !beside_others(c, s);
 }
 // Steps of a launch. The launch keeps the device, and a kernel of another stream waits until it ends, so a long call is

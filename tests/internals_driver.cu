@@ -92,6 +92,22 @@ static void shared(int precision) {
     for (auto& s : q) cudaStreamDestroy(s);
 }
 
+// The tuner of the plans on a grid whose steps go in one launch: what it times is by launches, what follows is not.
+static void autotune() {
+    nse2d_ctx* x = channel(256, 129, 64);
+    start(x);
+    OK(nse2d_step(x, 2, 1, nullptr));
+    std::printf("one_launch %d\n", x->c->steps_R > 0 && !x->c->cap_stream);
+    nse2d_plan best;
+    double ms = 0.0;
+    OK(nse2d_autotune_plan(x, 2, &best, &ms, nullptr));
+    std::printf("graphs_captured %d\n", x->c->cap_stream != nullptr);
+    if (x->c->graph_exec) { cudaGraphExecDestroy(x->c->graph_exec); x->c->graph_exec = nullptr; }
+    OK(nse2d_step(x, 2, 1, nullptr));
+    std::printf("one_launch_after %d\n", !x->c->graph_exec);
+    OK(nse2d_destroy(x));
+}
+
 // A wait of the model's kernels that has timed out: gradients and a training step, and the same once it is reported.
 struct Model {
     static constexpr int Nx = 32, Ny = 17, H = 16;
@@ -159,6 +175,7 @@ int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "gave_up") gave_up(std::atoi(argv[2]));
     else if (what == "model_wait") model_wait();
+    else if (what == "autotune") autotune();
     else if (what == "shared") shared(std::atoi(argv[2]));
     else return 2;
     return 0;

@@ -58,3 +58,11 @@ def test_steps_beside_another_channels_are_by_launches(driver, precision):
     assert got["by_launches_alone"] == 0
     assert got["first_channel_by_launches_0"] == 1 and got["first_channel_by_launches_1"] == 0
     assert got["same_bits"] == 1
+
+
+def test_the_tuner_times_the_steps_that_a_plan_governs(driver):
+    """On a grid whose steps go in one launch, every plan would time the same kernel: the tuner replays graphs there."""
+    got = driver("autotune")
+    assert got["one_launch"] == 1
+    assert got["graphs_captured"] == 1
+    assert got["one_launch_after"] == 1
