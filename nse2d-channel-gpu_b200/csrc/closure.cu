@@ -710,7 +710,7 @@ int nse2d_gemm_bf16(const void* A, const void* B, const float* bias, float* Cf, 
     p.Cf = Cf;
     p.Cb = static_cast<__nv_bfloat16*>(Cb);
     p.err = static_cast<int*>(e);
-    p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.act = relu ? 1 : 0;
+    p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.relu = relu ? 1 : 0;
     if (tc_gemm_launch(p, s)) return -1;
     int h = 0;
     NSE_CUDA_TRY(cudaMemcpyAsync(&h, e, sizeof(int), cudaMemcpyDeviceToHost, s));

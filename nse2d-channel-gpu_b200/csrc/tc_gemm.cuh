@@ -15,8 +15,8 @@
 //   - one thread issues four tcgen05.mma (M = 128, N, K = 16) and tcgen05.commit, which arrives
 //     on the buffer's mbarrier when the MMAs have read it.
 // After the last block all threads wait on that barrier; warp w reads TMEM lanes 32w..32w+31
-// (rows of C) with tcgen05.ld 32x32b.x16 and applies the epilogue: + bias[n], an activation,
-// FP32 and/or BF16 stores (the BF16 output after the activation: ReLU or GELU).
+// (rows of C) with tcgen05.ld 32x32b.x16 and applies the epilogue: + bias[n], FP32 and/or BF16
+// stores (of the BF16 output, after ReLU where it is asked for).
 //
 // Every mbarrier wait is bounded. A wait that runs out sets *err and the CTA still waits
 // (bounded) for its MMAs before it frees its TMEM and returns.
@@ -38,11 +38,11 @@ struct TcGemmParams {
     const __nv_bfloat16* A;  // [M][K]
     const __nv_bfloat16* B;  // [N][K]
     const float* bias;       // [N] or null
-    float* Cf;               // [M][ldc] FP32 (pre-activation) or null
-    __nv_bfloat16* Cb;       // [M][ldc] BF16 (after the activation) or null
+    float* Cf;               // [M][ldc] FP32 (before ReLU) or null
+    __nv_bfloat16* Cb;       // [M][ldc] BF16 (after ReLU where asked for) or null
     int* err;                // set to 1 by a wait that ran out
     int M, N, K, ldc;
-    int act;                 // activation of the BF16 output: 0 none, 1 ReLU, 2 GELU (tanh form)
+    int relu;                // of the BF16 output
 };
 
 // GELU, tanh form: 0.5 x (1 + tanh(sqrt(2/pi) (x + 0.044715 x^3))), and its derivative.
@@ -180,7 +180,7 @@ static __global__ void __launch_bounds__(TG_THREADS) k_tc_gemm(TcGemmParams p) {
                 if (p.bias) z += p.bias[c0 + i];
                 if (p.Cf) p.Cf[(size_t)row * p.ldc + c0 + i] = z;
                 if (p.Cb) {
-                    const float a = p.act == 1 ? fmaxf(z, 0.f) : (p.act == 2 ? tg_gelu(z) : z);
+                    const float a = p.relu ? fmaxf(z, 0.f) : z;
                     p.Cb[(size_t)row * p.ldc + c0 + i] = __float2bfloat16_rn(a);
                 }
             }
