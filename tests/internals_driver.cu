@@ -92,6 +92,16 @@ static void shared(int precision) {
     for (auto& s : q) cudaStreamDestroy(s);
 }
 
+// Whether a grid's steps go in one launch: no graph was captured by a step that would replay one.
+static void form(int Nx, int Ny, int precision) {
+    nse2d_ctx* x = channel(Nx, Ny, precision);
+    start(x);
+    OK(nse2d_step(x, 2, 1, nullptr));
+    OK(cudaDeviceSynchronize());
+    std::printf("one_launch %d\nrows_a_cta %d\n", !x->c->graph_exec, x->c->steps_R);
+    OK(nse2d_destroy(x));
+}
+
 // The tuner of the plans on a grid whose steps go in one launch: what it times is by launches, what follows is not.
 static void autotune() {
     nse2d_ctx* x = channel(256, 129, 64);
@@ -176,6 +186,7 @@ int main(int argc, char** argv) {
     if (what == "gave_up") gave_up(std::atoi(argv[2]));
     else if (what == "model_wait") model_wait();
     else if (what == "autotune") autotune();
+    else if (what == "form") form(std::atoi(argv[2]), std::atoi(argv[3]), std::atoi(argv[4]));
     else if (what == "shared") shared(std::atoi(argv[2]));
     else return 2;
     return 0;

@@ -38,7 +38,7 @@ def test_edges_match_the_oracle(nse, cuda, Nx, Ny, H, idx):
 @pytest.mark.parametrize("Nx,Ny,H,idx", [(256, 6, 16, (0, 2)), (130, 7, 32, (1,)), (64, 130, 32, (0, 1, 2, 3)), (66, 40, 64, (3, 0)),
                                          (128, 150, 48, (1, 2)), (8, 161, 16, (0, 1, 2, 3))])
 def test_strips_match_the_oracle(nse, cuda, Nx, Ny, H, idx):
-    """Strips of one, two and four rows, a row of one and of several strips, and tiles that run over the rows' ends."""
+    """Strips of one and of two rows, a row of one and of several strips, and tiles that run over the rows' ends."""
     test_edges_match_the_oracle(nse, cuda, Nx, Ny, H, idx)
 
 
@@ -61,3 +61,11 @@ def test_an_infinite_target_gives_infinite_gradients(nse, cuda, H):
     for layer in range(4):
         for g in net.get_grads(layer):
             assert np.all(g == -np.inf), (layer, np.unique(g)[:4])
+
+
+@pytest.mark.parametrize("H", [16, 32, 48, 64])
+@pytest.mark.parametrize("Nx,Ny", [(128, 150), (250, 80)])
+def test_strips_of_two_rows_and_two_tiles_match_the_oracle(nse, cuda, Nx, Ny, H):
+    """Four fields whose strips of two rows fill the device twice, so that a CTA has two tiles, of one row each."""
+    assert 4 * -(-Nx // 128) * -(-Ny // 2) >= 2 * 148
+    test_edges_match_the_oracle(nse, cuda, Nx, Ny, H, (3, 0, 2, 1))

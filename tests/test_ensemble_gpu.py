@@ -1,7 +1,7 @@
 """Batched ensembles (nse2d_ensemble_*) on a B200: one graph launch advances every member, and the
 result of each member equals that member stepped alone, to the bit, whatever the grouping of the
-members into concurrent branches. Ensemble members take the two-pass tridiagonal solve, so the
-solo runs they are compared with do too."""
+members into concurrent branches. Ensemble members of more than 1026 rows take the two-pass
+tridiagonal solve, so the solo runs that they are compared with do too."""
 import numpy as np
 import pytest
 

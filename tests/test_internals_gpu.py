@@ -66,3 +66,14 @@ def test_the_tuner_times_the_steps_that_a_plan_governs(driver):
     assert got["one_launch"] == 1
     assert got["graphs_captured"] == 1
     assert got["one_launch_after"] == 1
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("Nx,Ny,rows", [(64, 65, 1), (64, 514, 4), (128, 129, 1), (128, 300, 3), (256, 514, 4), (512, 257, 2), (512, 514, 4),
+                                        (1024, 131, 1), (1024, 300, 3), (1024, 446, 3), (1024, 513, 4), (1024, 514, 4), (1024, 515, 0),
+                                        (64, 5, 0), (32, 129, 0), (2048, 257, 0)])
+def test_the_grids_whose_steps_go_in_one_launch(driver, Nx, Ny, rows, precision):
+    """64 to 1024 points by up to 514 rows, with as many bands as the solve has groups of columns: bands of one to four
+    rows on 148 SMs."""
+    got = driver("form", Nx, Ny, precision)
+    assert got["rows_a_cta"] == rows and got["one_launch"] == (rows > 0)
