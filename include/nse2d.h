@@ -137,8 +137,8 @@ int  nse2d_set_tridiag_form(nse2d_ctx* ctx, int clusters);
 /* The kernel forms of a context's step (no counterpart in the reference, which has one form of
  * each operator): stage_tma, the persistent stage kernel fed by TMA boxes (1) or the one with a
  * CTA per tile and plain halo loads (0; grids with Nx < 128, or Nx < 256 in precision 32, have
- * only this one; rows of 64 to 1024 points take their stages in bands of rows, without either, and
- * have one form of the step but for pdl); tridiag_clusters, as nse2d_set_tridiag_form; rowfft_prefetch, the row
+ * only this one; rows of 64 to 1024 points take their stages in bands of rows, without either,
+ * while the bands fit the device); tridiag_clusters, as nse2d_set_tridiag_form; rowfft_prefetch, the row
  * transforms whose rows are prefetched into shared memory by bulk copies (1; Nx = 4096 in
  * precision 64 only) or read by plain loads (0); max_fused, with the prefetching transforms in an
  * adaptive FP64 step, the max reduction of psi inside the stage-3 inverse transform and dt
@@ -150,7 +150,8 @@ int  nse2d_set_tridiag_form(nse2d_ctx* ctx, int clusters);
  * the same step to round-off (the two stage forms, the two max forms and the two launch forms
  * to the bit). nse2d_set_plan falls back to the form a context can use and synchronises the
  * device when a form changes (the step graphs are captured again); nse2d_get_plan reports the
- * forms in use (max_fused as it takes effect). */
+ * forms chosen (max_fused as it takes effect). Where a grid has one form of a part (above), the
+ * choice governs only what still has both. */
 typedef struct nse2d_plan {
     int stage_tma, tridiag_clusters, rowfft_prefetch, max_fused, pdl;
 } nse2d_plan;

@@ -130,9 +130,10 @@ int nse2d_ensemble_create(nse2d_ctx* const* members, int n, nse2d_ensemble** out
             if (members[k]->c == members[i]->c) { delete en; set_error("nse2d_ensemble_create: member %d repeated", i); return -1; }
         en->e.m.push_back(members[i]->c);
     }
-    // Members take the two-pass tridiagonal solve: its plain grids share the SMs with the other
-    // branches' kernels, while the cluster form's persistent clusters, sized to fill the device,
-    // serialise the branches (64-channel workload: 1.33 against 1.92 ms per ensemble step).
+    // Members of more than 1026 rows take the two-pass tridiagonal solve: its plain grids share the
+    // SMs with the other branches' kernels, while the cluster form's persistent clusters, sized to
+    // fill the device, serialise the branches (64 channels, all in these forms: 1.33 against 1.92 ms
+    // per ensemble step). Shorter members have the one-CTA solve, a plain grid, in either form.
     for (Context* c : en->e.m)
         if (set_tridiag_form(c, false)) { delete en; return -1; }
     if (cudaMalloc((void**)&en->e.d_count, sizeof(int)) != cudaSuccess ||

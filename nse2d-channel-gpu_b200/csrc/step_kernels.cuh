@@ -122,8 +122,10 @@ __device__ __forceinline__ double thom_value(double A, double B, double e1, doub
 // attribute may be launched while the kernel before it in the stream is still finishing (its
 // CTAs trigger the next launch as they exit). Every step kernel begins with pdl_begin: it waits
 // until the grids it depends on have completed and their writes are visible (a no-op for a kernel
-// launched without the attribute). Nothing is read or written before the wait. An explicit trigger
-// right after the wait, which lets the next kernel's CTAs become resident early, measured slower.
+// launched without the attribute). Nothing that a step kernel writes is read before the wait, and
+// nothing is written; the row-band kernels copy their tables and row constants, which no step
+// writes, to shared memory before it. An explicit trigger right after the wait, which lets the next
+// kernel's CTAs become resident early, measured slower.
 __device__ __forceinline__ void pdl_begin() {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
 }

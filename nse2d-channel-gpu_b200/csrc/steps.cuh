@@ -1,7 +1,8 @@
 // Whole steps in one launch, for grids of up to 514 rows of up to 1024 points. Written for this project.
 //
 // On such a grid a step by launches is eight kernels of 2 to 3 us each and as much again between them. Here one
-// cooperative launch takes any number of steps: a CTA keeps its band of rows (band.cuh) in shared memory from step
+// cooperative launch takes any number of steps (run_steps asks for 64 at most, so that other streams come in between, and
+// steps beside those of another channel by launches): a CTA keeps its band of rows (band.cuh) in shared memory from step
 // to step, the tridiagonal solve (solve_cta.cuh) is dealt over the same CTAs, and a barrier across the grid
 // separates the two: seven barriers a step (six without an adaptive dt). Per step
 //   3 x { stage of the band; forward transform -> omega-hat | barrier | solve of the CTA's columns -> psi-hat, the
