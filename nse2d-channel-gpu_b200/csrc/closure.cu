@@ -82,6 +82,7 @@ struct Cnn {
     double gain = 1.0;                    // factor on the applied tau
     bool row_mean = false;                // apply the x-mean of tau on every row (the mean-flow part)
     long long step = 0;
+    unsigned settings = 0;                // changes of the scales and of the application
 };
 
 int tc_gemm_launch(const TcGemmParams& p0, cudaStream_t s);
@@ -611,6 +612,7 @@ static int cnn_adamw(Cnn* n, float lr, float wd, cudaStream_t s) {
     return 0;
 }
 
+unsigned cnn_settings(const Cnn* n) { return n->settings; }
 int* cnn_wait_flag(Cnn* n) { return n->err; }
 bool cnn_matches(const Cnn* n, int Nx, int Ny) { return n && n->Nx == Nx && n->Ny == Ny; }
 
@@ -806,6 +808,7 @@ int nse2d_cnn_set_scales(nse2d_cnn* c, const double* in_scales, double tau_scale
         c->n->in_scale[k] = in_scales[k];
     }
     c->n->out_tau = tau_scale;
+    c->n->settings += 1;
     return 0;
 }
 
@@ -817,6 +820,7 @@ int nse2d_cnn_set_application(nse2d_cnn* c, int wall_rows, double gain, int row_
     c->n->wall_rows = wall_rows;
     c->n->gain = gain;
     c->n->row_mean = row_mean != 0;
+    c->n->settings += 1;
     return 0;
 }
 
@@ -825,6 +829,7 @@ int nse2d_set_closure(nse2d_ctx* ctx, nse2d_cnn* net, int every_stage) {
     Context* c = ctx->c;
     if (c->run_exec) { cudaGraphExecDestroy(c->run_exec); c->run_exec = nullptr; }
     if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
+    c->closure_changes += 1;
     if (!net) { c->closure_net = nullptr; return 0; }
     if (!cnn_matches(net->n, c->Nx, c->Ny)) {
         set_error("nse2d_set_closure: the model is for %dx%d, the context is %dx%d", net->n->Nx, net->n->Ny, c->Nx, c->Ny);

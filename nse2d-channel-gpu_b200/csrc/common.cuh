@@ -115,6 +115,16 @@ struct RowTables {
 // of 64x65: 50 and 74).
 constexpr int kBandShareMax = 8;
 constexpr double kBandLoadMax = 4.0;
+
+// What a captured step holds by value and a later call can change: the wall constants of the FP32-bulk step (of the
+// state that was set), the model that is attached and its settings (both counted).
+struct Held {
+    double wall_bot32 = 0.0, wall_top32 = 0.0;
+    unsigned model = 0, settings = 0;
+    bool operator!=(const Held& o) const {
+        return wall_bot32 != o.wall_bot32 || wall_top32 != o.wall_top32 || model != o.model || settings != o.settings;
+    }
+};
 struct Context {
     Config cfg;
     int Nx = 0, Ny = 0, M = 0, H = 0, Hp = 0, Ni = 0;
@@ -186,6 +196,7 @@ struct Context {
     int maxuv_ctas = 0;            // resident CTAs of k_maxuv_dt (occupancy x SMs)
     // learned closure: the model evaluated before every stage and its output tau [Ny][Nx]
     struct Cnn* closure_net = nullptr;
+    unsigned closure_changes = 0;        // calls that attached or detached one
     double* closure_tau = nullptr;       // tau [Ny][Nx]
     bool closure_every_stage = true;     // false: tau of the step's first stage for all three
     // FP32-bulk variant (precision 32): base profiles (FP64) and FP32 fluctuations
@@ -213,6 +224,7 @@ struct Context {
     cudaStream_t cap_stream = nullptr;     // private stream used only for graph capture
     cudaGraphExec_t graph_exec = nullptr;  // one captured step
     cudaGraphExec_t run_exec = nullptr;    // WHILE(no halt) { step } for nse2d_run
+    Held held;                             // of graph_exec and run_exec
     double* spec_acc = nullptr;            // [2][Hp] accumulated E_u, E_v of the 1-D spectra
     double* moments = nullptr;             // [5][Ny] row sums of u, v, u^2, v^2, u v
     double* stats_acc = nullptr;           // [5][Ny] time-weighted row means (statistics on the device)

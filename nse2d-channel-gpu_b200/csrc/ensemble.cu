@@ -32,6 +32,7 @@ struct Ensemble {
     cudaStream_t cap = nullptr;
     std::vector<cudaStream_t> branch;
     cudaGraphExec_t exec = nullptr;
+    std::vector<Held> held;        // of the members, in exec
 };
 
 int ensemble_build(Ensemble* e, int groups, bool force = false) {
@@ -93,12 +94,19 @@ int ensemble_build(Ensemble* e, int groups, bool force = false) {
     err = cudaGraphInstantiate(&e->exec, g, 0);
     if (err != cudaSuccess) { set_error("ensemble instantiate: %s", cudaGetErrorString(err)); return done(-1); }
     e->groups = groups;
+    e->held.clear();
+    for (const Context* c : e->m) e->held.push_back(held_now(c));
     return done(0);
 }
 
 int ensemble_step(Ensemble* e, int nsteps, cudaStream_t s) {
     if (nsteps <= 0) return 0;
-    if (!e->exec && ensemble_build(e, e->groups > 0 ? e->groups : (int)e->m.size())) return -1;
+    bool stale = !e->exec;
+    for (size_t i = 0; !stale && i < e->m.size(); ++i) stale = held_now(e->m[i]) != e->held[i];
+    if (stale) {
+        if (e->exec) NSE_CUDA_TRY(cudaDeviceSynchronize());
+        if (ensemble_build(e, e->groups > 0 ? e->groups : (int)e->m.size(), true)) return -1;
+    }
     NSE_CUDA_TRY(cudaMemcpyAsync(e->d_count, &nsteps, sizeof(int), cudaMemcpyHostToDevice, s));
     NSE_CUDA_TRY(cudaStreamSynchronize(s));     // nsteps lives on this stack frame
     NSE_CUDA_TRY(cudaGraphLaunch(e->exec, s));

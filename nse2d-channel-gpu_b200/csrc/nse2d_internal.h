@@ -59,6 +59,7 @@ int launch_steps32(Context* c, int nsteps, int run, int store, cudaStream_t s);
 struct Cnn;
 int cnn_forward_psi(Cnn* n, const double* w, const double* psi, const double* a_node, double inv_dx, double inv_deta, double* tau,
                     cudaStream_t s);
+unsigned cnn_settings(const Cnn* n);  // counts the changes of its scales and application
 int* cnn_wait_flag(Cnn* n);        // device flag of the model's bounded waits
 bool cnn_matches(const Cnn* n, int Nx, int Ny);
 int thomas_launches(const Context* c);
@@ -90,6 +91,7 @@ int launch_maxuv(Context* c, const double* psi, bool set_dt, cudaStream_t s, boo
 int poisson_solve(Context* c, const double* w, double* psi, cudaStream_t s, bool general = false);
 int enqueue_step(Context* c, cudaStream_t s, bool store_rhs);
 int launches_per_step(const Context* c);
+Held held_now(const Context* c);
 void note_steps(Context* c, cudaStream_t s);       // steps of c were enqueued on s
 int enqueue_step_timed(Context* c, cudaStream_t s, cudaEvent_t* ev, bool store_rhs = false);
 const char* step_kernel_name(const Context* c, int k);

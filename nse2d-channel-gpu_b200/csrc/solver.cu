@@ -1059,6 +1059,25 @@ constexpr int kStepsPerLaunch = 64, kRunStepsPerLaunch = 256;
 
 static int enqueue_steps(Context* c, int nsteps, bool use_graph, cudaStream_t s, bool store_rhs);
 
+Held held_now(const Context* c) {
+    Held h;
+    h.wall_bot32 = c->wall_bot32; h.wall_top32 = c->wall_top32;
+    h.model = c->closure_changes;
+    if (c->closure_net) h.settings = cnn_settings(c->closure_net);
+    return h;
+}
+// Drops captured steps that hold what has changed since.
+static int refresh_graphs(Context* c) {
+    const Held now = held_now(c);
+    if (!(now != c->held)) return 0;
+    c->held = now;
+    if (!c->graph_exec && !c->run_exec) return 0;
+    NSE_CUDA_TRY(cudaDeviceSynchronize());
+    if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
+    if (c->run_exec) { cudaGraphExecDestroy(c->run_exec); c->run_exec = nullptr; }
+    return 0;
+}
+
 // nsteps steps: in one launch (of kStepsPerLaunch each) where the grid allows it; else, with use_graph, the step is
 // captured once into a CUDA graph and replayed.
 int run_steps(Context* c, int nsteps, bool use_graph, cudaStream_t s, bool store_rhs) {
@@ -1078,6 +1097,7 @@ static int enqueue_steps(Context* c, int nsteps, bool use_graph, cudaStream_t s,
             if (enqueue_step(c, s, store_rhs && i == nsteps - 1)) return -1;
         return 0;
     }
+    if (refresh_graphs(c)) return -1;
     if (!c->graph_exec) {
         if (!c->cap_stream) NSE_CUDA_TRY(cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
         NSE_CUDA_TRY(cudaStreamBeginCapture(c->cap_stream, cudaStreamCaptureModeThreadLocal));
@@ -1117,6 +1137,7 @@ int run_until_halt(Context* c, cudaStream_t s) {
         NSE_CUDA_TRY(cudaStreamSynchronize(s));
         if (c->h_ctl->halt || (c->h_ctl->nonfinite & 2)) return 0;
     }
+    if (refresh_graphs(c)) return -1;
     if (!c->run_exec) {
         if (!c->cap_stream) NSE_CUDA_TRY(cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
         cudaGraph_t g = nullptr;
