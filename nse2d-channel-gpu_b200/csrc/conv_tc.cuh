@@ -17,14 +17,18 @@
 // MODE CV_FWD: z = acc + bias (FP32, stored when z is given) and GELU(z) in BF16, the next layer's input.
 // MODE CV_OUT: the output layer, of whose N = 16 padded channels only channel 0 exists: z [P], tau.
 // MODE CV_DGRAD: the gradient of the layer's input as a convolution of dZ with the flipped taps (K = 9 npad,
-// N = cin), times GELU' of the layer below's pre-activation: dZ of that layer in FP32 and BF16.
+// N = cin), times GELU' of the layer below's pre-activation: dZ of that layer in FP32 and BF16. An accumulator in TMEM
+// truncates at every K step, so the nine taps go to two accumulators (64 channels: three), which ordinary additions join:
+// in one, the sums' error against 64 bits was up to twice that of a product per tap added in FP32 (64 channels, db of a
+// layer below 5.0e-7, with three 1.5e-7, per tap 2.5e-7; 32 channels 2.2e-7, 1.2e-7 and 2.3e-7).
 // k_conv_in, the input layer: 5 channels, padded to one 16-byte load per tap and packed to K = 45 (48).
 //
 // k_wgrad<C, N, TG>: dW[n][k] = sum_p dZ[p][n] A[p][k], a contraction over the pixels, on the tensor cores
 // through mma.sync (both operands are stored pixel-major and transposed on the way by ldmatrix; the
 // contraction is bound by the gather of A, not by the MMA rate). dZ stays FP32: it is split into three BF16
-// terms whose sum is its 24-bit significand, so every product is exact, and the sums of each 64 pixels are
-// added to FP32 accumulators by ordinary additions. The taps and dZ of the next tile are on their way while one is
+// terms whose sum is its 24-bit significand, so every product is exact, and the sums of each 32 pixels are
+// added to FP32 accumulators by ordinary additions (the MMA truncates: error of dW against 64 bits 7.4e-8, with sums of
+// 64 pixels 9.9e-8, by FP32 multiply-adds 2.4e-7). The taps and dZ of the next tile are on their way while one is
 // multiplied. Per-CTA partials are folded in a fixed order. Hidden layer of 32 channels, 264192 pixels: im2col,
 // CUDA-core products and a serial fold 975 us; 69 and 9 for the fold without the overlap, 60 with it (tensor pipe 40%,
 // 12 warps an SM by their registers); input layer 55 and 32.
@@ -66,7 +70,9 @@ __host__ __device__ constexpr int cv_tiles(int W, int R) {
 template <int C> __host__ __device__ constexpr int cv_plane(int W, int R) {
     return ((R + 2) * (W + 2) * 16 + 127) / 128 * 128 + (C == 16 ? 64 : (C == 32 ? 32 : 16));
 }
-__host__ __device__ constexpr int cv_cols(int N) { return N == 48 ? 64 : N; }    // TMEM columns of a tile
+__host__ __device__ constexpr int cv_cols(int N) { return N == 48 ? 64 : N; }    // TMEM columns of an accumulator
+// accumulators of a tile
+template <int C, int MODE> __host__ __device__ constexpr int cv_groups() { return MODE != CV_DGRAD || C == 16 ? 1 : (C == 64 ? 3 : 2); }
 template <int C> __host__ __device__ constexpr size_t cv_smem_bytes(int N, int W, int R) {
     const size_t ab = ((size_t)cv_plane<C>(W, R) * (C / 8) + 127) / 128 * 128 + (size_t)N * cv_nch<C>() * 16;
     const size_t st = (size_t)cv_tiles(W, R) * 128 * (N + 1) * 4;
@@ -268,7 +274,7 @@ static __global__ void __launch_bounds__(CV_NT) k_conv(ConvParams p) {
     u /= sx;
     const int j0 = (u % rb) * R, base = (u / rb) * Nx * Ny;
     const uint32_t sA = tg_smem_u32(sm), sB = sA + (uint32_t)((plane * C8 + 127) / 128 * 128);
-    constexpr int tcol = cv_cols(N);
+    constexpr int G = cv_groups<C, MODE>(), TPG = (9 + G - 1) / G, gcol = cv_cols(N), tcol = G * gcol;
     uint32_t ncols = 32;
     while ((int)ncols < T * tcol) ncols *= 2;
     if (warp == 0) cv_tmem_alloc(&tmem_base, ncols);
@@ -299,9 +305,12 @@ static __global__ void __launch_bounds__(CV_NT) k_conv(ConvParams p) {
             for (int tap = 0; tap < 9; ++tap) {
                 const int ty = MODE == CV_DGRAD ? 2 - tap / 3 : tap / 3, tx = MODE == CV_DGRAD ? 2 - tap % 3 : tap % 3;
 #pragma unroll
-                for (int c = 0; c < C8; c += 2)
-                    cv_mma(d, tg_desc(a0 + (uint32_t)((ty * Wp + tx) * 16 + c * plane), (uint32_t)plane, 128),
-                           tg_desc(sB + (uint32_t)((tap * C8 + c) << 7), 128, NCH * 128), idesc, tap > 0 || c > 0);
+                for (int c = 0; c < C8; c += 2) {
+                    const uint64_t da = tg_desc(a0 + (uint32_t)((ty * Wp + tx) * 16 + c * plane), (uint32_t)plane, 128);
+                    const uint64_t db = tg_desc(sB + (uint32_t)((tap * C8 + c) << 7), 128, NCH * 128);
+                    if constexpr (G == 1) cv_mma(d, da, db, idesc, tap > 0 || c > 0);
+                    else cv_mma(d + (uint32_t)(tap / TPG * gcol), da, db, idesc, tap % TPG > 0 || c > 0);
+                }
             }
         }
     });
@@ -337,6 +346,13 @@ static __global__ void __launch_bounds__(CV_NT) k_conv(ConvParams p) {
             uint32_t v[16];
             cv_tmem_ld16(tlane + (uint32_t)(t * tcol + c0), v);
 #pragma unroll
+            for (int k = 1; k < G; ++k) {
+                uint32_t u[16];
+                cv_tmem_ld16(tlane + (uint32_t)(t * tcol + k * gcol + c0), u);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(u[i]));
+            }
+#pragma unroll
             for (int i = 0; i < 16; ++i) st[(t * 128 + row) * ld + c0 + i] = __uint_as_float(v[i]);
         }
     }
@@ -368,6 +384,12 @@ __device__ __forceinline__ void wg_ldsm4t(uint32_t (&r)[4], uint32_t addr) {
 __device__ __forceinline__ void wg_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// the first of a sum
+__device__ __forceinline__ void wg_mma0(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};\n"
+                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
 
 template <int C, int N, int TG>
@@ -449,34 +471,44 @@ static __global__ void __launch_bounds__(WG_NT, 2) k_wgrad(WgradParams p) {
         }
         __syncthreads();
         if (t + (int)gridDim.x < ntiles) fetch(t + gridDim.x, b ^ 1);
-        float s[MPW][N8][4] = {};
 #pragma unroll 1
-        for (int k0 = 0; k0 < WG_PX; k0 += 16) {
-            uint32_t a[MPW][4];
+        for (int k0 = 0; k0 < WG_PX; k0 += 32) {
+            float s[MPW][N8][4];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int k1 = k0 + 16 * h;
+                uint32_t a[MPW][4];
+#pragma unroll
+                for (int m = 0; m < MPW; ++m)
+                    if (warp + 6 * m < MT) wg_ldsm4t(a[m], tg_smem_u32(sA + (k1 + lpx) * LDA + (warp + 6 * m) * 16 + lcol));
+#pragma unroll
+                for (int term = 2; term >= 0; --term)                  // smallest first
+#pragma unroll
+                    for (int n = 0; n < N8; n += 2) {
+                        // two n tiles: matrices (pixels 0-7, 0-7, 8-15, 8-15) x (n, n + 8, n, n + 8)
+                        uint32_t b[4];
+                        wg_ldsm4t(b, tg_smem_u32(sB + (k1 + lpx) * LDB + term * N + n * 8 + lcol));
+#pragma unroll
+                        for (int m = 0; m < MPW; ++m)
+                            if (warp + 6 * m < MT) {
+                                if (h == 0 && term == 2) {
+                                    wg_mma0(s[m][n], a[m], b[0], b[2]);
+                                    wg_mma0(s[m][n + 1], a[m], b[1], b[3]);
+                                } else {
+                                    wg_mma(s[m][n], a[m], b[0], b[2]);
+                                    wg_mma(s[m][n + 1], a[m], b[1], b[3]);
+                                }
+                            }
+                    }
+            }
 #pragma unroll
             for (int m = 0; m < MPW; ++m)
-                if (warp + 6 * m < MT) wg_ldsm4t(a[m], tg_smem_u32(sA + (k0 + lpx) * LDA + (warp + 6 * m) * 16 + lcol));
+                if (warp + 6 * m < MT)
 #pragma unroll
-            for (int term = 2; term >= 0; --term)                      // smallest first
+                    for (int n = 0; n < N8; ++n)
 #pragma unroll
-                for (int n = 0; n < N8; n += 2) {
-                    // two n tiles: matrices (pixels 0-7, 0-7, 8-15, 8-15) x (n, n + 8, n, n + 8)
-                    uint32_t b[4];
-                    wg_ldsm4t(b, tg_smem_u32(sB + (k0 + lpx) * LDB + term * N + n * 8 + lcol));
-#pragma unroll
-                    for (int m = 0; m < MPW; ++m)
-                        if (warp + 6 * m < MT) {
-                            wg_mma(s[m][n], a[m], b[0], b[2]);
-                            wg_mma(s[m][n + 1], a[m], b[1], b[3]);
-                        }
-                }
+                        for (int i = 0; i < 4; ++i) acc[m][n][i] += s[m][n][i];
         }
-#pragma unroll
-        for (int m = 0; m < MPW; ++m)
-#pragma unroll
-            for (int n = 0; n < N8; ++n)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) acc[m][n][i] += s[m][n][i];
         __syncthreads();                                               // the tiles are read
     }
     // accumulator (m, n): rows lane / 4 and lane / 4 + 8 of the m tile, columns 2 (lane mod 4), + 1 of the n tile
