@@ -11,8 +11,8 @@
 // gradients leave as whole 16-byte chunks of consecutive channels; one thread per row storing its own
 // channels 4 bytes at a time was most of the old GEMM's time. What bounds it at 32 -> 32 channels and 264192 pixels
 // (eight 256x129 fields): instructions, 54% of the issue slots, most of them the GELU (FP32 tanh) and the
-// epilogue's; DRAM 10 of 34 us. im2col + GEMM 268 us, taps gathered 57 (input gradient 70), strips 34 (42); of one
-// field 47, 13 and 11.
+// epilogue's; DRAM 10 of 34 us. im2col + GEMM 268 us, taps gathered 57 (input gradient 70), strips 34 (42, with
+// two accumulators 45); of one field 47, 13 and 11.
 //
 // MODE CV_FWD: z = acc + bias (FP32, stored when z is given) and GELU(z) in BF16, the next layer's input.
 // MODE CV_OUT: the output layer, of whose N = 16 padded channels only channel 0 exists: z [P], tau.
@@ -31,7 +31,7 @@
 // 64 pixels 9.9e-8, by FP32 multiply-adds 2.4e-7). The taps and dZ of the next tile are on their way while one is
 // multiplied. Per-CTA partials are folded in a fixed order. Hidden layer of 32 channels, 264192 pixels: im2col,
 // CUDA-core products and a serial fold 975 us; 69 and 9 for the fold without the overlap, 60 with it (tensor pipe 40%,
-// 12 warps an SM by their registers); input layer 55 and 32.
+// 12 warps an SM by their registers); input layer 55 and 34.
 #pragma once
 #include "tc_gemm.cuh"
 
