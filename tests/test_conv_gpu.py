@@ -69,3 +69,45 @@ def test_strips_of_two_rows_and_two_tiles_match_the_oracle(nse, cuda, Nx, Ny, H)
     """Four fields whose strips of two rows fill the device twice, so that a CTA has two tiles, of one row each."""
     assert 4 * -(-Nx // 128) * -(-Ny // 2) >= 2 * 148
     test_edges_match_the_oracle(nse, cuda, Nx, Ny, H, (3, 0, 2, 1))
+
+
+@pytest.mark.parametrize("H", [16, 32, 48, 64])
+def test_sums_of_the_gradients_in_64_bits(nse, cuda, H):
+    """The sums of the input gradient and of the weight gradients alone, against 64 bits. Everything around them is
+    exact: constant activations of 20 (GELU' is 1), targets of 64 .. 127 times 2^24, beside which the output is lost in
+    rounding, output weights of a few bits and a pixel count that is a power of two, so that dZ above the sums is the
+    same to the bit and its rounding to BF16 too.
+
+    A tensor core truncates at every step of a sum, 2^-24 of the sum on average over the step, of sums that grow from
+    zero: n steps lose n 2^-26. Input gradient: 9 H / 16 steps in 1, 2, 2 or 3 accumulators, at most 14 steps each;
+    weight gradient: 6 steps. Together 20 2^-26 = 3.0e-7, and 0.5e-7 for the additions in FP32."""
+    torch = cuda
+    Nx, Ny, B = 64, 34, 2
+    rng = np.random.default_rng(H)
+    net = nse.Cnn(Nx, Ny, np.zeros(Ny), H, B)
+    net.set_scales([1.0] * 4, 1.0)
+    W = []
+    for layer in range(4):
+        ci, c_out = net.shape(layer)
+        w = rng.integers(-100, 101, (c_out, 9, ci)) / 2.0 ** 12 if layer == 3 else 0.005 * rng.standard_normal((c_out, 9, ci))
+        net.set_params(layer, w, np.full(c_out, 20.0 if layer < 3 else 0.0))
+        W.append(co.bf16(w))
+    tau = rng.integers(64, 128, (B, Ny, Nx)) * 2.0 ** 24
+    zero = torch.zeros((B, Ny, Nx), dtype=torch.float64, device="cuda")
+    net.gradients(zero, zero, zero, zero, _dev(torch, tau), idx=range(B))
+    h1 = np.full((Ny, Nx, H), 20.0)
+    z1 = np.einsum("jitc,otc->jio", co.im2col(h1), W[1]) + 20.0
+    assert z1.min() > 8.0
+    h2 = co.bf16(z1)
+    ref = {1: [0.0, 0.0], 2: [0.0, 0.0]}
+    for s in range(B):
+        d = np.zeros((Ny, Nx))
+        d[1:-1] = -2.0 * tau[s, 1:-1] / (B * Nx * (Ny - 2))
+        dz = {2: co.col2im(np.einsum("jio,otc->jitc", co.bf16(d[:, :, None]), W[3]))}
+        dz[1] = co.col2im(np.einsum("jio,otc->jitc", co.bf16(dz[2]), W[2]))
+        for layer, h in ((1, h1), (2, h2)):
+            ref[layer][0] = ref[layer][0] + np.einsum("jio,jitc->otc", dz[layer], co.im2col(h))
+            ref[layer][1] = ref[layer][1] + dz[layer].sum((0, 1))
+    for layer in (1, 2):
+        for got, want in zip(net.get_grads(layer), ref[layer]):
+            assert _rel(got, want) < 3.5e-7, (layer, _rel(got, want))
